@@ -635,6 +635,7 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
         MapArgs ma;
         ma.g = g;
         ma.layers = ti->layers.p;
+        ma.layer_elems = (long long)ti->nlayers * ti->g.N;
         ma.slots = w->slots.p;
         ma.terms = w->terms.p;
         ma.maxterms = maxterms;
@@ -1198,6 +1199,7 @@ int sim_batches(qsk_sim *s, const std::vector<Step> &steps, bool teacher) {
                 MapArgs ma;
                 ma.g = g;
                 ma.layers = s->ti->layers.p;
+                ma.layer_elems = (long long)s->ti->nlayers * s->ti->g.N;
                 ma.slots = s->d_slots.p;
                 ma.terms = s->d_terms.p;
                 ma.maxterms = s->maxterms;
@@ -1673,6 +1675,7 @@ int exact_nodes(qsk_sim *s, const int *nodes, int count, bool teacher) {
         MapArgs ma;
         ma.g = g;
         ma.layers = s->ti->layers.p;
+        ma.layer_elems = (long long)s->ti->nlayers * s->ti->g.N;
         ma.slots = s->d_slots.p;
         ma.terms = s->d_terms.p;
         ma.maxterms = s->maxterms;
@@ -2065,6 +2068,7 @@ int sim_batches_multi(qsk_sim *s, const std::vector<Step> &steps) {
             std::memset(&ma, 0, sizeof(ma));
             ma.g = T->g;
             ma.layers = T->layers.p;
+            ma.layer_elems = (long long)T->nlayers * T->g.N;
             ma.slots = s->d_slots.p;
             ma.terms = s->d_terms.p;
             ma.maxterms = s->maxterms;
@@ -3130,6 +3134,7 @@ int qsk_pattern_kbest_noalloc(const qsk_ti *ti, void *stream, int n_neighbours, 
         MapArgs ma;
         ma.g = g;
         ma.layers = ti->layers.p;
+        ma.layer_elems = (long long)ti->nlayers * ti->g.N;
         ma.slots = d_slot;
         ma.terms = d_terms;
         ma.maxterms = maxterms;

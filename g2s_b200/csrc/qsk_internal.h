@@ -133,9 +133,24 @@ struct SimPrepArgs {
     StaticTerm *sterms = nullptr;   // k_mt_prep: slots + static terms of the batch (null: none)
 };
 
+// x / d as a high product and a shift, exact for x < 2^31: mul = the ceiling
+// of 2^(31 + l) / d with l = ceil(log2 d), x / d = (x * mul) >> (31 + l)
+// (Granlund and Montgomery 1994); shift < 0: d == 1
+struct FastDiv {
+    unsigned mul;
+    int shift;
+};
+inline FastDiv make_fast_div(unsigned d) {
+    int l = 0;
+    while ((1ull << l) < d) ++l;
+    if (l == 0) return {0u, -1};
+    return {unsigned(((1ull << (31 + l)) + d - 1) / d), l - 1};
+}
+
 struct MapArgs {
     Geom g;
     const float *layers;
+    long long layer_elems;    // values of all layers
     const Slot *slots;
     const Term *terms;
     int maxterms;
@@ -148,6 +163,7 @@ struct MapArgs {
     // (xmask[b * xwords + m / 32]) forces valid position m to -inf; null: none
     const unsigned *xmask = nullptr;
     long long xwords = 0;
+    FastDiv div[QSK_MAXD];    // by g.fft (set by the launcher)
 };
 
 // Bit-plane layout: every plane is `plane_words(N)` words, of which the

@@ -646,191 +646,362 @@ __global__ void k_prep_tc_nodes(SimPrepArgs P, TcNodeArgs T, unsigned prep_block
 
 // ---------------------------------------------------------------------------
 // fused map + record filter
+//
+// A warp takes MR_SEGS consecutive 128-position segments at once, eight
+// positions per lane (base + 32 r + lane): a term's shared-memory read, its
+// address and the loop are paid once for eight gathers, which all go to one
+// pointer at immediate offsets, and the products run on packed FP32 pairs
+// (each half rounded as the scalar instruction rounds it).  In cache the
+// kernel is bound by L1 wavefronts, one per 32 gathers and one per term read:
+// eight positions a lane reach 23 position-terms per clock and SM of the 28
+// that nine wavefronts per 256 allow.  Positions outside the border are
+// gathered like the others where every address of the warp's span lies in the
+// layers (their scores are not used); at the two ends of the scan, and for
+// the rarer operations, they gather from a valid dummy address instead.
+// Spans without a valid position gather nothing.
+//
+// The filter keeps the prefix top-K of the positions the warp has seen over
+// all its spans (a CTA's warps take interleaved spans in scan order, so
+// everything a warp has seen lies before its next span): a segment, and a
+// round of 32 positions, whose maximum is below that K-th best holds no
+// record, and a few candidates are inserted one by one.
 // ---------------------------------------------------------------------------
+namespace {
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// x / d for x < 2^31
+__device__ __forceinline__ unsigned fast_div(unsigned x, FastDiv f) { return f.shift < 0 ? x : __umulhi(x, f.mul) >> f.shift; }
+
+constexpr int MR_SEGS = 2;               // segments a warp takes at once
+constexpr int MR_P = 4 * MR_SEGS;        // positions per lane
+
+// one pass over the terms at in-bounds addresses: p is the span's first
+// layer element of this lane
+template <bool ALL_SQ>
+__device__ __forceinline__ void map_terms_fast(const Term *__restrict__ sterm, int nt, const float *__restrict__ p,
+                                               float (&acc)[MR_P]) {
+    f32x2 a2[MR_P / 2];
+#pragma unroll
+    for (int i = 0; i < MR_P / 2; ++i) a2[i] = 0ull;
+#pragma unroll 2
+    for (int t = 0; t < nt; ++t) {
+        const Term tm = sterm[t];
+        const float *lp = p + tm.base;
+        float x[MR_P];
+#pragma unroll
+        for (int r = 0; r < MR_P; ++r) x[r] = __ldg(lp + 32 * r);
+        if (ALL_SQ || tm.op == OP_SQLIN) {
+            const f32x2 ta = pack2(tm.a, tm.a), tb = pack2(tm.b, tm.b);
+#pragma unroll
+            for (int i = 0; i < MR_P / 2; ++i) {
+                const f32x2 xx = pack2(x[2 * i], x[2 * i + 1]);
+                a2[i] = fma2(ta, mul2(xx, xx), a2[i]);
+                a2[i] = fma2(tb, xx, a2[i]);
+            }
+        } else if (tm.op == OP_EQ) {
+#pragma unroll
+            for (int i = 0; i < MR_P / 2; ++i) {
+                float u, v;
+                unpack2(a2[i], u, v);
+                u = (x[2 * i] == tm.b) ? __fadd_rn(u, tm.a) : u;
+                v = (x[2 * i + 1] == tm.b) ? __fadd_rn(v, tm.a) : v;
+                a2[i] = pack2(u, v);
+            }
+        } else {   // OP_LIN
+            const f32x2 ta = pack2(tm.a, tm.a);
+#pragma unroll
+            for (int i = 0; i < MR_P / 2; ++i) a2[i] = fma2(ta, pack2(x[2 * i], x[2 * i + 1]), a2[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < MR_P / 2; ++i) unpack2(a2[i], acc[2 * i], acc[2 * i + 1]);
+}
+
+// the same for every operation, with the positions outside the border (or
+// the scan) gathered at usafe
+__device__ void map_terms_any(const Term *__restrict__ sterm, int nt, const float *__restrict__ layers, unsigned base,
+                              unsigned vm, unsigned usafe, float (&acc)[MR_P], float (&crs)[MR_P]) {
+    unsigned mm[MR_P];
+#pragma unroll
+    for (int r = 0; r < MR_P; ++r) mm[r] = ((vm >> r) & 1u) ? base + 32 * r : usafe;
+    for (int t = 0; t < nt; ++t) {
+        const Term tm = sterm[t];
+        const float *lp = layers + tm.base;
+        float x[MR_P];
+#pragma unroll
+        for (int r = 0; r < MR_P; ++r) x[r] = __ldg(lp + mm[r]);
+        if (tm.op == OP_SQLIN) {
+#pragma unroll
+            for (int r = 0; r < MR_P; ++r) {
+                acc[r] = __fmaf_rn(tm.a, __fmul_rn(x[r], x[r]), acc[r]);
+                acc[r] = __fmaf_rn(tm.b, x[r], acc[r]);
+            }
+        } else if (tm.op == OP_EQ) {
+#pragma unroll
+            for (int r = 0; r < MR_P; ++r) acc[r] = (x[r] == tm.b) ? __fadd_rn(acc[r], tm.a) : acc[r];
+        } else if (tm.op == OP_LIN) {
+#pragma unroll
+            for (int r = 0; r < MR_P; ++r) acc[r] = __fmaf_rn(tm.a, x[r], acc[r]);
+        } else if (tm.op == OP_LINX) {
+#pragma unroll
+            for (int r = 0; r < MR_P; ++r) crs[r] = __fmaf_rn(tm.a, x[r], crs[r]);
+        } else if (tm.op == OP_SQLINM) {
+            const Term pl = sterm[t + 1];
+#pragma unroll
+            for (int r = 0; r < MR_P; ++r) {
+                const bool in = !isnan(x[r]);
+                const float x0 = in ? x[r] : 0.f;
+                const float mk = in ? 1.f : 0.f;
+                acc[r] = __fmaf_rn(tm.a, __fmul_rn(x0, x0), acc[r]);
+                acc[r] = __fmaf_rn(tm.b, x0, acc[r]);
+                acc[r] = __fmaf_rn(pl.a, mk, acc[r]);
+                crs[r] = __fmaf_rn(pl.b, mk, crs[r]);
+            }
+            ++t;
+        }
+    }
+}
+}  // namespace
+
 template <int KF>
-__global__ void __launch_bounds__(256) k_map_records(MapArgs A) {
+__global__ void __launch_bounds__(256, KF <= 4 ? 4 : 2) k_map_records(MapArgs A) {
     extern __shared__ Term sterm[];
     __shared__ Slot ss;
+    // smallest and largest layer offset of the terms; bit 0: a term that is not
+    // OP_SQLIN, bit 1: one that the fast loop does not know
+    __shared__ int s_lo, s_hi, s_ops;
     const int b = blockIdx.y;
-    if (threadIdx.x == 0) ss = A.slots[b];
+    const Term *src = A.terms + (long long)b * A.maxterms;
+    // a thread's first term is read beside the slot (the slot's block of terms
+    // is maxterms long; what lies beyond its own terms is not used)
+    Term first;
+    if ((int)threadIdx.x < A.maxterms) first = src[threadIdx.x];
+    if (threadIdx.x == 0) {
+        ss = A.slots[b];
+        s_lo = INT_MAX;
+        s_hi = INT_MIN;
+        s_ops = 0;
+    }
     __syncthreads();
     if (ss.flags & SLOT_SKIP) return;
     const int nt = ss.nterms;
-    const Term *src = A.terms + (long long)b * A.maxterms;
-    for (int t = threadIdx.x; t < nt; t += blockDim.x) sterm[t] = src[t];
+    {
+        int lo = INT_MAX, hi = INT_MIN, ops = 0;
+        for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+            const Term tm = t < (int)blockDim.x ? first : src[t];
+            sterm[t] = tm;
+            lo = min(lo, tm.base);
+            hi = max(hi, tm.base);
+            ops |= (tm.op == OP_SQLIN ? 0 : 1) | (tm.op == OP_SQLIN || tm.op == OP_EQ || tm.op == OP_LIN ? 0 : 2);
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        ops = (int)__reduce_or_sync(0xffffffffu, (unsigned)ops);
+        if ((threadIdx.x & 31) == 0 && lo <= hi) {
+            atomicMin(&s_lo, lo);
+            atomicMax(&s_hi, hi);
+            if (ops) atomicOr(&s_ops, ops);
+        }
+    }
     __syncthreads();
+    const bool all_sq = s_ops == 0, all_plain = s_ops < 2;
 
     const Geom &g = A.g;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const bool emit_masked = (ss.flags & SLOT_EMIT_MASKED) != 0;
-    // a valid scan position used for address-safe dummy gathers; with no valid
-    // position at all every entry is masked and no gather is issued
-    long long m_safe = 0;
+    const bool missing = (ss.flags & SLOT_MISSING) != 0;
+    // a valid scan position used for address-safe dummy gathers
+    unsigned usafe = 0;
     bool any_valid = true;
     for (int d = 0; d < g.nd; ++d) {
-        m_safe += (long long)ss.lo[d] * g.sstride[d];
+        usafe += (unsigned)(ss.lo[d] * g.sstride[d]);
         any_valid &= ss.lo[d] < g.fft[d];
     }
-    const int nt_eff = any_valid ? nt : 0;
-    if (!any_valid) m_safe = 0;
-    const unsigned usafe = (unsigned)m_safe;
     const unsigned uN = (unsigned)g.N;
 
     const int seg_begin = blockIdx.x * A.segs_per_cta;
-    int seg_end = seg_begin + A.segs_per_cta;
-    if (seg_end > g.nseg) seg_end = g.nseg;
+    const int seg_end = min(seg_begin + A.segs_per_cta, g.nseg);
     float *rv = A.rec_val + (long long)b * g.nseg * QSK_SEG;
     int *ri = A.rec_idx + (long long)b * g.nseg * QSK_SEG;
-
-    for (int sg = seg_begin + warp; sg < seg_end; sg += nwarps) {
-        const unsigned base = (unsigned)sg * QSK_SEG;
-        unsigned mm[4];
-        bool valid[4], exists[4];
-        float acc[4];
+    float carry[KF];   // prefix top-KF of what this warp has seen
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            unsigned m = base + 32 * r + lane;
-            exists[r] = m < uN;
-            bool ok = exists[r] && any_valid;
-            if (ok) {
+    for (int q = 0; q < KF; ++q) carry[q] = -CUDART_INF_F;
+
+    for (int sg0 = seg_begin + MR_SEGS * warp; sg0 < seg_end; sg0 += MR_SEGS * nwarps) {
+        const unsigned base = (unsigned)sg0 * QSK_SEG;
+        // bit r: the position base + 32 r + lane lies inside the border
+        unsigned vm = 0u;
+        if (any_valid) {
+#pragma unroll
+            for (int r = 0; r < MR_P; ++r) {
+                const unsigned m = base + 32 * r + lane;
+                bool ok = m < uN;
+                unsigned rest = m;
 #pragma unroll
                 for (int d = 0; d < QSK_MAXD; ++d)
-                    if (d < g.nd) ok &= (int)((m / (unsigned)g.sstride[d]) % (unsigned)g.fft[d]) >= ss.lo[d];
-            }
-            valid[r] = ok;
-            mm[r] = ok ? m : usafe;
-            acc[r] = 0.f;
-        }
-        float crs[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) crs[r] = 0.f;
-        for (int t = 0; t < nt_eff; ++t) {
-            const Term tm = sterm[t];
-            const float *lp = A.layers + tm.base;
-            float x[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) x[r] = __ldg(lp + mm[r]);
-            if (tm.op == OP_SQLIN) {
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    acc[r] = __fmaf_rn(tm.a, __fmul_rn(x[r], x[r]), acc[r]);
-                    acc[r] = __fmaf_rn(tm.b, x[r], acc[r]);
-                }
-            } else if (tm.op == OP_EQ) {
-#pragma unroll
-                for (int r = 0; r < 4; ++r) acc[r] = (x[r] == tm.b) ? __fadd_rn(acc[r], tm.a) : acc[r];
-            } else if (tm.op == OP_LIN) {
-#pragma unroll
-                for (int r = 0; r < 4; ++r) acc[r] = __fmaf_rn(tm.a, x[r], acc[r]);
-            } else if (tm.op == OP_LINX) {
-#pragma unroll
-                for (int r = 0; r < 4; ++r) crs[r] = __fmaf_rn(tm.a, x[r], crs[r]);
-            } else if (tm.op == OP_SQLINM) {
-                const Term pl = sterm[t + 1];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const bool in = !isnan(x[r]);
-                    const float x0 = in ? x[r] : 0.f;
-                    const float mk = in ? 1.f : 0.f;
-                    acc[r] = __fmaf_rn(tm.a, __fmul_rn(x0, x0), acc[r]);
-                    acc[r] = __fmaf_rn(tm.b, x0, acc[r]);
-                    acc[r] = __fmaf_rn(pl.a, mk, acc[r]);
-                    crs[r] = __fmaf_rn(pl.b, mk, crs[r]);
-                }
-                ++t;
+                    if (d < g.nd) {
+                        const unsigned q = fast_div(rest, A.div[d]);
+                        ok &= (int)(rest - q * (unsigned)g.fft[d]) >= ss.lo[d];
+                        rest = q;
+                    }
+                vm |= ok ? (1u << r) : 0u;
             }
         }
-        if (ss.flags & SLOT_MISSING) {
-            // overlap masked by the centre, then -|S/c^4| (-inf where c == 0);
-            // positions outside the border are NaN in the reference
-            // (quantileSamplingModule.hpp:507-516, CPUThreadDevice.cpp:501-524)
+        float acc[MR_P];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float cm = valid[r] ? __ldg(A.layers + ss.cmask_base + (long long)mm[r]) : 0.f;
-                const float c = __fmul_rn(crs[r], cm);
-                const float c4 = __fmul_rn(__fmul_rn(__fmul_rn(c, c), c), c);
-                float e = -fabsf(__fdiv_rn(acc[r], c4));
-                if (c == 0.f) e = -CUDART_INF_F;
-                acc[r] = valid[r] ? e : CUDART_NAN_F;
+        for (int r = 0; r < MR_P; ++r) acc[r] = 0.f;
+        const unsigned vany = __reduce_or_sync(0xffffffffu, vm);
+        if (vany) {
+            const bool inside = (long long)base + s_lo >= 0 && (long long)base + (32 * MR_P - 1) + s_hi < A.layer_elems;
+            if (inside && all_sq && !missing) {
+                map_terms_fast<true>(sterm, nt, A.layers + base + lane, acc);
+            } else if (inside && all_plain && !missing) {
+                map_terms_fast<false>(sterm, nt, A.layers + base + lane, acc);
+            } else {
+                float crs[MR_P];
+#pragma unroll
+                for (int r = 0; r < MR_P; ++r) crs[r] = 0.f;
+                map_terms_any(sterm, nt, A.layers, base + lane, vm, usafe, acc, crs);
+                if (missing) {
+                    // overlap masked by the centre, then -|S/c^4| (-inf where c == 0);
+                    // positions outside the border are NaN in the reference
+                    // (quantileSamplingModule.hpp:507-516, CPUThreadDevice.cpp:501-524)
+#pragma unroll
+                    for (int r = 0; r < MR_P; ++r) {
+                        const bool v = (vm >> r) & 1u;
+                        const float cm = v ? __ldg(A.layers + ss.cmask_base + (long long)(base + 32 * r + lane)) : 0.f;
+                        const float c = __fmul_rn(crs[r], cm);
+                        const float c4 = __fmul_rn(__fmul_rn(__fmul_rn(c, c), c), c);
+                        float e = -fabsf(__fdiv_rn(acc[r], c4));
+                        if (c == 0.f) e = -CUDART_INF_F;
+                        acc[r] = e;
+                    }
+                }
             }
         }
         // verbatim exclusion (one index, or the radius mask): -inf written over
         // the map after the compensation, at masked positions too, where it
         // replaces the NaN border of a missing-data map
         // (quantileSamplingModule.hpp:518-523, CPUThreadDevice.cpp:310-342)
-        bool hit[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) hit[r] = exists[r] && (int)(base + 32 * r + lane) == ss.excl;
+        unsigned hit = 0u;
+        if (ss.excl >= 0) {
+            const unsigned o = (unsigned)ss.excl - base - (unsigned)lane;   // 32 r for one lane of the span
+            if ((o & 31u) == 0u && o < 32u * MR_P) hit = 1u << (o >> 5);
+        }
         if (A.xmask) {
             const unsigned *xm = A.xmask + (long long)b * A.xwords;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const unsigned m = base + 32 * r + lane;
-                if (exists[r] && ((xm[m >> 5] >> (m & 31)) & 1u)) hit[r] = true;
-            }
+            for (int r = 0; r < MR_P; ++r)
+                if (base + 32 * r < uN) hit |= ((xm[(base >> 5) + r] >> lane) & 1u) << r;
         }
         // a masked position is an explicit record when the slot emits masked
         // entries, or when it is an excluded one of a missing-data map (-inf
         // instead of NaN); otherwise the replay counts it as an implicit -inf
-        const bool missing = (ss.flags & SLOT_MISSING) != 0;
-        // warp prefix top-KF over the segment in scan order; records are the
-        // positions not below the K-th best of everything before them in the
-        // segment (a superset of the global triggers).
-        float carry[KF];
 #pragma unroll
-        for (int q = 0; q < KF; ++q) carry[q] = -CUDART_INF_F;
-        int count = 0;
-        float segmax = -CUDART_INF_F;
+        for (int s = 0; s < MR_SEGS; ++s) {
+            const int sg = sg0 + s;
+            if (sg >= seg_end) break;
+            const unsigned sbase = base + s * QSK_SEG;
+            float xv[4];
+            float segmax = -CUDART_INF_F;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const float xval = hit[r] ? -CUDART_INF_F : valid[r] ? acc[r] : (missing ? CUDART_NAN_F : -CUDART_INF_F);
-            segmax = fmaxf(segmax, xval);
-            // a NaN score never compares true in the reservoir (fKb.hpp), so it
-            // is never a record and must not raise the prefix K-th best: it
-            // enters the scan as -inf (fminf/fmaxf would turn it into +inf)
-            float st[KF];
-            st[0] = isnan(xval) ? -CUDART_INF_F : xval;
+            for (int r = 0; r < 4; ++r) {
+                const int q = 4 * s + r;
+                xv[r] = ((hit >> q) & 1u)  ? -CUDART_INF_F
+                        : ((vm >> q) & 1u) ? acc[q]
+                                           : (missing ? CUDART_NAN_F : -CUDART_INF_F);
+                segmax = fmaxf(segmax, xv[r]);
+            }
 #pragma unroll
-            for (int q = 1; q < KF; ++q) st[q] = -CUDART_INF_F;
+            for (int off = 16; off > 0; off >>= 1) segmax = fmaxf(segmax, __shfl_xor_sync(0xffffffffu, segmax, off));
+            int count = 0;
+            if (!(segmax < carry[KF - 1])) {
+                // warp prefix top-KF in scan order: records are the positions not
+                // below the K-th best of everything before them (a superset of the
+                // global triggers)
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                float rcv[KF], mrg[KF];
+                for (int r = 0; r < 4; ++r) {
+                    const int q = 4 * s + r;
+                    const bool exists = sbase + 32 * r + lane < uN;
+                    const float xval = xv[r];
+                    const float kth0 = carry[KF - 1];
+                    unsigned bal = __ballot_sync(0xffffffffu, exists && xval >= kth0);
+                    if (bal == 0u) continue;
+                    if (kth0 != -CUDART_INF_F && __popc(bal) <= 6) {
+                        // finite candidates only, inserted in scan order
+                        unsigned cand = bal;
+                        while (cand) {
+                            const int l = __ffs(cand) - 1;
+                            cand &= cand - 1u;
+                            const float y = __shfl_sync(0xffffffffu, xval, l);
+                            if (y >= carry[KF - 1]) topk_insert<KF>(carry, y);
+                            else bal &= ~(1u << l);
+                        }
+                    } else {
+                        // a NaN score never compares true in the reservoir (fKb.hpp), so it
+                        // is never a record and must not raise the prefix K-th best: it
+                        // enters the scan as -inf (fminf/fmaxf would turn it into +inf)
+                        float st[KF];
+                        st[0] = isnan(xval) ? -CUDART_INF_F : xval;
 #pragma unroll
-                for (int q = 0; q < KF; ++q) rcv[q] = __shfl_up_sync(0xffffffffu, st[q], off);
-                if (lane >= off) {
-                    topk_merge<KF>(st, rcv, mrg);
+                        for (int k = 1; k < KF; ++k) st[k] = -CUDART_INF_F;
 #pragma unroll
-                    for (int q = 0; q < KF; ++q) st[q] = mrg[q];
+                        for (int off = 1; off < 32; off <<= 1) {
+                            float rcv[KF], mrg[KF];
+#pragma unroll
+                            for (int k = 0; k < KF; ++k) rcv[k] = __shfl_up_sync(0xffffffffu, st[k], off);
+                            if (lane >= off) {
+                                topk_merge<KF>(st, rcv, mrg);
+#pragma unroll
+                                for (int k = 0; k < KF; ++k) st[k] = mrg[k];
+                            }
+                        }
+                        float ex[KF], pre[KF];
+#pragma unroll
+                        for (int k = 0; k < KF; ++k) {
+                            const float y = __shfl_up_sync(0xffffffffu, st[k], 1);
+                            ex[k] = lane == 0 ? -CUDART_INF_F : y;
+                        }
+                        topk_merge<KF>(carry, ex, pre);
+                        const bool rec = exists && xval >= pre[KF - 1] &&
+                                         (((vm >> q) & 1u) || emit_masked || (((hit >> q) & 1u) && missing));
+                        bal = __ballot_sync(0xffffffffu, rec);
+                        float last[KF], nc[KF];
+#pragma unroll
+                        for (int k = 0; k < KF; ++k) last[k] = __shfl_sync(0xffffffffu, st[k], 31);
+                        topk_merge<KF>(carry, last, nc);
+#pragma unroll
+                        for (int k = 0; k < KF; ++k) carry[k] = nc[k];
+                    }
+                    if ((bal >> lane) & 1u) {
+                        const unsigned o = sbase + count + __popc(bal & lanemask_lt());
+                        rv[o] = xval;
+                        ri[o] = int(sbase + 32 * r + lane);
+                    }
+                    count += __popc(bal);
                 }
             }
-            float ex[KF], pre[KF];
-#pragma unroll
-            for (int q = 0; q < KF; ++q) {
-                float y = __shfl_up_sync(0xffffffffu, st[q], 1);
-                ex[q] = lane == 0 ? -CUDART_INF_F : y;
+            if (lane == 0) {
+                A.rec_cnt[(long long)b * g.nseg + sg] = count;
+                A.rec_max[(long long)b * g.nseg + sg] = segmax;
             }
-            topk_merge<KF>(carry, ex, pre);
-            const float kth = pre[KF - 1];
-            const bool rec = exists[r] && (xval >= kth) && (valid[r] || emit_masked || (hit[r] && missing));
-            const unsigned bal = __ballot_sync(0xffffffffu, rec);
-            if (rec) {
-                const int o = count + __popc(bal & lanemask_lt());
-                rv[base + o] = xval;
-                ri[base + o] = int(base + 32 * r + lane);
-            }
-            count += __popc(bal);
-            float last[KF], nc[KF];
-#pragma unroll
-            for (int q = 0; q < KF; ++q) last[q] = __shfl_sync(0xffffffffu, st[q], 31);
-            topk_merge<KF>(carry, last, nc);
-#pragma unroll
-            for (int q = 0; q < KF; ++q) carry[q] = nc[q];
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) segmax = fmaxf(segmax, __shfl_xor_sync(0xffffffffu, segmax, off));
-        if (lane == 0) {
-            A.rec_cnt[(long long)b * g.nseg + sg] = count;
-            A.rec_max[(long long)b * g.nseg + sg] = segmax;
         }
     }
 }
@@ -2822,16 +2993,20 @@ cudaError_t launch_prep_sim(const SimPrepArgs &a, cudaStream_t st) {
 }
 
 int map_segs_per_cta(const Geom &g, int nslots) {
-    // enough CTAs to fill the GPU several times over, at most 32 segments each
-    long long target = 148LL * 8;
-    long long per = ((long long)g.nseg * nslots + target - 1) / target;
-    if (per < 8) per = 8;
-    if (per > 32) per = 32;
-    return (int)per;
+    // a CTA takes 8 warps x MR_SEGS segments a turn; more turns (up to 8)
+    // tighten the filter and share the set-up while the grid still fills the
+    // GPU's 4 resident CTAs per SM three times
+    const long long turn = 8 * MR_SEGS;
+    const long long turns = (g.nseg + turn - 1) / turn * nslots;
+    long long per = turns / (148LL * 4 * 3);
+    per = per < 1 ? 1 : (per > 8 ? 8 : per);
+    return (int)(per * turn);
 }
 
-cudaError_t launch_map_records(const MapArgs &a, int nslots, int K, int maxterms_in_batch, cudaStream_t st) {
+cudaError_t launch_map_records(const MapArgs &args, int nslots, int K, int maxterms_in_batch, cudaStream_t st) {
     int threads = 256;
+    MapArgs a = args;
+    for (int d = 0; d < QSK_MAXD; ++d) a.div[d] = make_fast_div((unsigned)a.g.fft[d]);
     dim3 grid((unsigned)((a.g.nseg + a.segs_per_cta - 1) / a.segs_per_cta), (unsigned)nslots);
     size_t smem = sizeof(Term) * (size_t)(maxterms_in_batch > 0 ? maxterms_in_batch : 1);
     if (K <= 1) k_map_records<1><<<grid, threads, smem, st>>>(a);
