@@ -788,8 +788,8 @@ struct qsk_sim {
     DBuf<float> d_rec_val;
     DBuf<int> d_rec_idx, d_rec_cnt;
     DBuf<float> d_rec_max;
-    DBuf<unsigned> d_mt_state;       // [2][slot][624]: two batches
-    DBuf<Slot> d_sslots;             // bit-sliced path: [2][slot] slots written one batch ahead
+    DBuf<unsigned> d_mt_state;       // [2][slot][624]: two groups of batches
+    DBuf<Slot> d_sslots;             // bit-sliced path: [2][slot] slots written one group ahead
     DBuf<StaticTerm> d_sterms;       // and their terms without values [2][slot][maxterms]
     DBuf<int> d_mt_pre;
     DBuf<int> d_tpl_range, d_node_kernel, d_node_lim, d_node_nv;
@@ -797,9 +797,13 @@ struct qsk_sim {
     DBuf<float> d_node_k;
     int maxterms = 0;
     int max_slots = 0;
+    int rng_slots = 0;                  // nodes whose generator states one buffer holds
     bool use_bits = false;
     qsk_sim_info info;
     bool neighbours_ready = false;
+    bool tmax_ready = false;            // tmax and few follow the neighbour lists
+    std::vector<int> tmax;
+    std::vector<unsigned char> few;
     bool profiling = false;
     bool use_graph = false;             // plain path: the batch chain as one CUDA graph
     // tensor-core form (qsk_sim_set_tensor)
@@ -819,7 +823,7 @@ struct qsk_sim {
     DBuf<unsigned long long> d_tc_key, d_tc_counts;
     DBuf<Slot> d_tc_slots;
     DBuf<Term> d_tc_terms;
-    DBuf<int> d_audit_nodes;
+    DBuf<int> d_audit_nodes, d_exact_nodes;
     DBuf<float> d_audit_val;
     DBuf<unsigned> d_audit_pos, d_err_max;
     DBuf<double> d_err_sum;
@@ -1013,6 +1017,7 @@ void build_path(qsk_sim *s) {
 
 int sim_neighbours(qsk_sim *s) {
     if (s->neighbours_ready) return QSK_OK;
+    s->tmax_ready = false;
     if (s->full) {
         CK(launch_neighbours_full(s->dg, s->d_tpl.p, s->ntpl, s->d_path.p, s->begin, s->nodes, s->d_post.p, s->nvar,
                                   s->n, s->local ? s->d_node_nv.p : nullptr, s->d_nb_count.p, s->d_nb_tpl.p,
@@ -1054,6 +1059,7 @@ struct Step {
     int kb_off;         // TENSOR: this step's tile K-blocks in d_tc_kb
     int scale = 1;      // TENSOR, learned proposal: the nodes' stencil scale
     int level = -1;     // tensor-core form: the dependency level (-1: one stream for all steps)
+    bool few = true;    // HASH: a node of the step may have fewer than K positions (it takes the replay)
 };
 
 int tc_step(qsk_sim *s, const Step &st, bool teacher);
@@ -1111,32 +1117,61 @@ int sim_batches(qsk_sim *s, const std::vector<Step> &steps, bool teacher) {
         pa.nb_mask = s->full ? s->d_nb_mask.p : nullptr;
         return pa;
     };
-    // Generator states of batch j go to buffer j % 2 on st_rng, one batch
-    // ahead of the simulation on st; buffer p is rewritten only after the
-    // replay that read it (ev_used[p]).
-    const size_t mt_words = size_t(s->max_slots) * 624;
-    // bit-sliced map: slots and value-free terms also come one batch ahead
+    // Generator states go to one of two buffers on st_rng, a group of batches
+    // at a time and one group ahead of the simulation; a buffer is rewritten
+    // only after the last replay that read it (ev_used).  The states depend on
+    // the path alone, so a group may span levels: consecutive entries of one
+    // node list, up to rng_slots nodes (a single batch makes the first group,
+    // which nothing hides).
+    const size_t mt_words = size_t(s->rng_slots) * 624;
+    // bit-sliced map: slots and value-free terms also come one group ahead
     // (k_mt_prep); the map reads the neighbour values itself, so nothing
     // runs before it on st
     const bool bits = s->use_bits && g_map_mode == 0;
-    const size_t st_words = size_t(s->max_slots) * s->maxterms;
-    auto launch_rng = [&](size_t j) -> int {
-        const int p = int(j & 1);
-        CK(cudaStreamWaitEvent(s->st_rng, s->ev_used[p], 0));
+    const size_t st_words = size_t(s->rng_slots) * s->maxterms;
+    struct Group {
+        size_t first, last;   // plain steps [first, last]
+        int slots;
+    };
+    std::vector<Group> groups;
+    std::vector<int> group_of(pl.size()), slot_of(pl.size());
+    for (size_t j = 0; j < pl.size(); ++j) {
         const Step &sj = steps[pl[j]];
-        SimPrepArgs pa = prep_args(sj.nodes, sj.off, sj.B);
+        bool join = groups.size() > 1;
+        if (join) {
+            const Step &before = steps[pl[j - 1]];
+            join = before.nodes == sj.nodes && before.off + before.B == sj.off &&
+                   groups.back().slots + sj.B <= s->rng_slots;
+        }
+        if (join) {
+            slot_of[j] = groups.back().slots;
+            groups.back().last = j;
+            groups.back().slots += sj.B;
+        } else {
+            slot_of[j] = 0;
+            groups.push_back({j, j, sj.B});
+        }
+        group_of[j] = int(groups.size()) - 1;
+    }
+    auto launch_rng = [&](size_t q) -> int {
+        const int p = int(q & 1);
+        CK(cudaStreamWaitEvent(s->st_rng, s->ev_used[p], 0));
+        const Step &sj = steps[pl[groups[q].first]];
+        SimPrepArgs pa = prep_args(sj.nodes, sj.off, groups[q].slots);
         if (bits) {
-            pa.slots = s->d_sslots.p + size_t(p) * s->max_slots;
+            pa.slots = s->d_sslots.p + size_t(p) * s->rng_slots;
             pa.sterms = s->d_sterms.p + p * st_words;
         }
-        CK(launch_mt_prep(pa, s->d_mt_state.p + p * mt_words, s->d_mt_pre.p + size_t(p) * s->max_slots, s->st_rng));
+        CK(launch_mt_prep(pa, s->d_mt_state.p + p * mt_words, s->d_mt_pre.p + size_t(p) * s->rng_slots, s->st_rng));
         CK(cudaEventRecord(s->ev_ready[p], s->st_rng));
+        s->info.launches += 1;
         return QSK_OK;
     };
     CK(cudaEventRecord(s->ev_used[0], s->st));   // after everything queued so far on st
     CK(cudaEventRecord(s->ev_used[1], s->st));
     int rc = pl.empty() ? QSK_OK : launch_rng(0);
     if (rc) return rc;
+    cudaStream_t rng_waited = nullptr;   // the stream that waits for the current group's states
     size_t j = 0;   // plain / audit step counter
     // tensor-core form: the exact-map steps of a level (its nodes beyond the
     // prefix) run on st2 while its tensor steps run on st; the nodes of a
@@ -1162,18 +1197,25 @@ int sim_batches(qsk_sim *s, const std::vector<Step> &steps, bool teacher) {
             CK(cudaStreamWaitEvent(s->st2, s->ev_level, 0));
             side_level = step.level;
         }
-        const int B = step.B, p = int(j & 1);
+        const size_t grp = size_t(group_of[j]);
+        const int B = step.B, p = int(grp & 1);
+        const size_t slot0 = size_t(slot_of[j]);
         const bool audit = step.kind == STEP_AUDIT;
-        if (j + 1 < pl.size() && (rc = launch_rng(j + 1)) != QSK_OK) return rc;
+        if (groups[grp].first == j) {
+            if (grp + 1 < groups.size() && (rc = launch_rng(grp + 1)) != QSK_OK) return rc;
+            rng_waited = nullptr;
+        }
+        const bool group_end = groups[grp].last == j;
         ++j;
         {
-            Slot *slots = bits ? s->d_sslots.p + size_t(p) * s->max_slots : s->d_slots.p;
+            Slot *slots = bits ? s->d_sslots.p + size_t(p) * s->rng_slots + slot0 : s->d_slots.p;
             if (s->profiling) CK(cudaEventRecord(prof_event(s), ws));
             if (!bits) CK(launch_prep_sim(prep_args(step.nodes, step.off, B), ws));
             if (s->profiling) CK(cudaEventRecord(prof_event(s), ws));
             if (bits) {
                 // the slots and static terms of this batch come from k_mt_prep
-                CK(cudaStreamWaitEvent(ws, s->ev_ready[p], 0));
+                if (rng_waited != ws) CK(cudaStreamWaitEvent(ws, s->ev_ready[p], 0));
+                rng_waited = ws;
                 BitArgs ba;
                 ba.g = g;
                 ba.planes = s->ti->planes.p;
@@ -1182,7 +1224,7 @@ int sim_batches(qsk_sim *s, const std::vector<Step> &steps, bool teacher) {
                 ba.catv = s->ti->catv.p;
                 ba.slots = slots;
                 ba.terms = nullptr;
-                ba.sterms = s->d_sterms.p + p * st_words;
+                ba.sterms = s->d_sterms.p + p * st_words + slot0 * s->maxterms;
                 ba.state = s->d_state.p;
                 ba.init = s->d_init.p;
                 ba.id_image = s->d_id.p;
@@ -1211,7 +1253,7 @@ int sim_batches(qsk_sim *s, const std::vector<Step> &steps, bool teacher) {
                 CK(launch_map_records(ma, B, s->K, s->maxterms, ws));
             }
             if (s->profiling) CK(cudaEventRecord(prof_event(s), ws));
-            s->info.launches += bits ? 3 : 4;
+            s->info.launches += bits ? 1 : 2;
             s->info.map_launches += 1;
             s->info.map_positions += (long long)B * g.N;
             ReplayArgs ra;
@@ -1238,9 +1280,10 @@ int sim_batches(qsk_sim *s, const std::vector<Step> &steps, bool teacher) {
                 ra.out_pos = s->d_audit_pos.p + (size_t)step.off * s->K;
             }
             ra.full = s->full ? 1 : 0;
-            ra.mt_state = s->d_mt_state.p + p * mt_words;
-            ra.mt_pre = s->d_mt_pre.p + size_t(p) * s->max_slots;
-            CK(cudaStreamWaitEvent(ws, s->ev_ready[p], 0));
+            ra.mt_state = s->d_mt_state.p + p * mt_words + slot0 * 624;
+            ra.mt_pre = s->d_mt_pre.p + size_t(p) * s->rng_slots + slot0;
+            if (rng_waited != ws) CK(cudaStreamWaitEvent(ws, s->ev_ready[p], 0));
+            rng_waited = ws;
             if (step.kind == STEP_HASH) {
                 ra.drawn_score = s->d_drawn_score.p;
                 ra.drawn_scale = s->d_drawn_scale.p;
@@ -1248,8 +1291,11 @@ int sim_batches(qsk_sim *s, const std::vector<Step> &steps, bool teacher) {
                 ra.only_flagged = 1;
                 s->info.launches += 1;
             }
-            CK(launch_replay(ra, ws));
-            CK(cudaEventRecord(s->ev_used[p], ws));
+            if (step.kind != STEP_HASH || step.few) {
+                CK(launch_replay(ra, ws));
+                s->info.launches += 1;
+            }
+            if (group_end) CK(cudaEventRecord(s->ev_used[p], ws));
             if (s->profiling) CK(cudaEventRecord(prof_event(s), ws));
             if (side) {
                 CK(cudaEventRecord(s->ev_side, s->st2));
@@ -1496,14 +1542,24 @@ int tc_configure(qsk_sim *s, int T_auto) {
 // template prefix (sorted by their largest template index, so that a tile of
 // 128 nodes needs few K blocks) take the tensor-core form, the rest the plain
 // path.  Rewrites the level node list in that order.
-// largest template index of every path node (-1: no neighbour but the centre)
-int tc_tmax(qsk_sim *s, std::vector<int> &tmax) {
+// s->tmax: largest template index of every path node (-1: no neighbour but
+// the centre), s->few: its pattern lies inside the TI at fewer than K
+// positions; kept with the neighbour lists, from which they follow
+int tc_tmax(qsk_sim *s) {
+    if (s->tmax_ready) return QSK_OK;
     const long long nodes = s->nodes;
     CK(s->d_tc_tmax.ensure(size_t(std::max<long long>(nodes, 1))));
-    CK(launch_tc_tmax(nodes, s->n, s->d_nb_count.p, s->d_nb_tpl.p, s->d_tc_tmax.p, s->st));
-    tmax.resize((size_t)nodes);
-    CK(cudaMemcpyAsync(tmax.data(), s->d_tc_tmax.p, sizeof(int) * nodes, cudaMemcpyDeviceToHost, s->st));
+    CK(launch_tc_tmax(nodes, s->n, s->d_nb_count.p, s->d_nb_tpl.p, s->d_tpl.p, s->ti->g, s->K, s->d_tc_tmax.p, s->st));
+    s->tmax.resize((size_t)nodes);
+    CK(cudaMemcpyAsync(s->tmax.data(), s->d_tc_tmax.p, sizeof(int) * nodes, cudaMemcpyDeviceToHost, s->st));
     CK(cudaStreamSynchronize(s->st));
+    s->few.assign((size_t)nodes, 0);
+    for (long long i = 0; i < nodes; ++i)
+        if (s->tmax[size_t(i)] >= QSK_TMAX_FEW - 1) {
+            s->few[size_t(i)] = 1;
+            s->tmax[size_t(i)] -= QSK_TMAX_FEW;
+        }
+    s->tmax_ready = true;
     return QSK_OK;
 }
 
@@ -1526,6 +1582,9 @@ int tc_auto_prefix(const std::vector<int> &tmax) {
 int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &tmax, std::vector<Step> &steps,
             std::vector<int> &audit_nodes) {
     const long long nodes = s->nodes;
+    // the exact map's nodes of all levels, one after the other (its generator
+    // states are prepared over consecutive entries)
+    CK(s->d_exact_nodes.ensure(size_t(std::max<long long>(nodes, 1))));
     std::vector<int> order((size_t)nodes);
     CK(cudaMemcpyAsync(order.data(), s->d_level_nodes.p, sizeof(int) * nodes, cudaMemcpyDeviceToHost, s->st));
     CK(cudaStreamSynchronize(s->st));
@@ -1550,7 +1609,7 @@ int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &t
         CK(cudaMemcpyAsync(lscale.data(), s->d_lscale.p, sizeof(int) * size_t(tot), cudaMemcpyDeviceToHost, s->st));
         CK(cudaStreamSynchronize(s->st));
     }
-    std::vector<int> el, pl, esc, idx;
+    std::vector<int> el, pl, esc, idx, exact;
     for (size_t l = 0; l + 1 < start.size(); ++l) {
         el.clear();
         pl.clear();
@@ -1601,13 +1660,16 @@ int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &t
             g0 = g1;
         }
         for (int off = 0; off < int(pl.size()); off += s->max_slots) {
-            Step st{STEP_HASH, s->d_level_nodes.p, start[l] + int(el.size()) + off,
+            Step st{STEP_HASH, s->d_exact_nodes.p, int(exact.size()) + off,
                     std::min(s->max_slots, int(pl.size()) - off), 0};
             // the learned proposal's fallback uses the exact map's buffers
             // inside its tensor steps: its levels stay on one stream
             st.level = learned ? -1 : int(l);
+            st.few = false;
+            for (int q = off; q < off + st.B; ++q) st.few |= s->few[size_t(pl[size_t(q)])] != 0;
             steps.push_back(st);
         }
+        exact.insert(exact.end(), pl.begin(), pl.end());
         ntc += (long long)el.size();
         npl += (long long)pl.size();
         if (athr) {
@@ -1620,6 +1682,8 @@ int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &t
         }
     }
     CK(cudaMemcpyAsync(s->d_level_nodes.p, order.data(), sizeof(int) * nodes, cudaMemcpyHostToDevice, s->st));
+    if (!exact.empty())
+        CK(cudaMemcpyAsync(s->d_exact_nodes.p, exact.data(), sizeof(int) * exact.size(), cudaMemcpyHostToDevice, s->st));
     if (kb.empty()) kb.push_back(0);   // no tensor step: a valid (unused) upload
     CK(s->d_tc_kb.upload(kb.data(), kb.size(), s->st));
     CK(cudaStreamSynchronize(s->st));   // host vectors go out of scope
@@ -1963,9 +2027,9 @@ int sim_records(qsk_sim *s, long long slots);
 // tensor-core run: plan, steps, audit, statistics.  `start`: level bounds of
 // the level node list (one level under teacher forcing)
 int tc_run(qsk_sim *s, const std::vector<int> &start, bool teacher) {
-    std::vector<int> tmax;
-    int rc = tc_tmax(s, tmax);
+    int rc = tc_tmax(s);
     if (rc) return rc;
+    const std::vector<int> &tmax = s->tmax;
     if (s->tc_T_auto == 0) s->tc_T_auto = tc_auto_prefix(tmax);
     if ((rc = tc_configure(s, s->tc_T_auto)) != QSK_OK) return rc;
     std::vector<Step> steps;
@@ -2283,9 +2347,13 @@ int qsk_sim_create(int device, const qsk_qs_params *p, const float *di_init, qsk
     }
     if (s->full && s->ti->missing)
         return bail(fail(QSK_ERR_UNSUPPORTED, "-fs with missing training-image values is not implemented"));
-    cudaError_t e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->st_rng, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->st2, cudaStreamNonBlocking);
+    // the generator states come a group ahead: their blocks give way to the
+    // level chain's, which wait for an SM the least
+    int prio_low = 0, prio_high = 0;
+    cudaError_t e = cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->st, cudaStreamNonBlocking, prio_high);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->st_rng, cudaStreamNonBlocking, prio_low);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->st2, cudaStreamNonBlocking, prio_high);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_level, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_side, cudaEventDisableTiming);
     for (int p = 0; p < 2 && e == cudaSuccess; ++p) {
@@ -2423,11 +2491,14 @@ int qsk_sim_create(int device, const qsk_qs_params *p, const float *di_init, qsk
     ms = std::max<long long>(1, std::min<long long>(ms, std::max<long long>(s->nodes, 1)));
     ms = std::min<long long>(ms, 65535);
     s->max_slots = int(ms);
+    // a group of batches prepares up to 4,096 nodes' generator states (2.5 KB
+    // each) in one launch, or one batch where that is more
+    s->rng_slots = int(std::max<long long>(ms, std::min<long long>(4096, std::max<long long>(s->nodes, 1))));
     if ((e = s->d_slots.alloc(size_t(s->max_slots))) != cudaSuccess ||
-        (e = s->d_mt_state.alloc(size_t(2) * s->max_slots * 624)) != cudaSuccess ||
-        (e = s->d_mt_pre.alloc(size_t(2) * s->max_slots)) != cudaSuccess ||
-        (s->use_bits && ((e = s->d_sslots.alloc(size_t(2) * s->max_slots)) != cudaSuccess ||
-                         (e = s->d_sterms.alloc(size_t(2) * s->max_slots * s->maxterms)) != cudaSuccess)) ||
+        (e = s->d_mt_state.alloc(size_t(2) * s->rng_slots * 624)) != cudaSuccess ||
+        (e = s->d_mt_pre.alloc(size_t(2) * s->rng_slots)) != cudaSuccess ||
+        (s->use_bits && ((e = s->d_sslots.alloc(size_t(2) * s->rng_slots)) != cudaSuccess ||
+                         (e = s->d_sterms.alloc(size_t(2) * s->rng_slots * s->maxterms)) != cudaSuccess)) ||
         (e = s->d_terms.alloc(size_t(s->max_slots) * s->maxterms)) != cudaSuccess)
         return bail(fail(e == cudaErrorMemoryAllocation ? QSK_ERR_NOMEM : QSK_ERR_CUDA, "scratch: %s",
                          cudaGetErrorString(e)));
@@ -2717,8 +2788,8 @@ int qsk_encoder_add_pairs(qsk_encoder *e, qsk_sim *s, const float *di_completed,
     s->topt = qsk_tensor_opts{};
     int rc = QSK_OK;
     if (!s->neighbours_ready && (rc = sim_neighbours(s)) != QSK_OK) return rc;
-    std::vector<int> tmax;
-    if ((rc = tc_tmax(s, tmax)) != QSK_OK) return rc;
+    if ((rc = tc_tmax(s)) != QSK_OK) return rc;
+    const std::vector<int> &tmax = s->tmax;
     std::vector<int> nodes;
     for (int q = 0; q < count; ++q) {
         const int i = path_nodes[q];

@@ -224,8 +224,8 @@ struct ReplayArgs {
     // skipped blocks stand for; null: each slot is seeded in the replay
     const unsigned *mt_state;
     const int *mt_pre;
-    // replay only the slots flagged SLOT_SKIP / SLOT_EMIT_MASKED (the hash
-    // select takes the others)
+    // replay only the slots flagged SLOT_EMIT_MASKED (the hash select takes
+    // the others, marginal draws among them)
     int only_flagged = 0;
     // hash select: per path node, the drawn candidate's score (regret audit)
     float *drawn_score = nullptr;
@@ -316,8 +316,8 @@ cudaError_t launch_build_planes(const float *layers, const Geom &g, int nvar, co
 int map_bits_segs_per_cta(const Geom &g, int nslots);
 cudaError_t launch_map_bits(const BitArgs &a, int nslots, int K, int maxterms_in_batch, cudaStream_t st);
 cudaError_t launch_replay(const ReplayArgs &a, cudaStream_t st);
-// k best by (score, tie hash) over the records; slots with SLOT_SKIP or
-// SLOT_EMIT_MASKED are left to launch_replay with only_flagged
+// k best by (score, tie hash) over the records, and marginal draws; slots
+// with SLOT_EMIT_MASKED are left to launch_replay with only_flagged
 cudaError_t launch_hash_select(const ReplayArgs &a, cudaStream_t st);
 // exclusion masks: slot b's positions around scan index center[b] (radius[b] >= 1)
 cudaError_t launch_radius_mask(const int *center, const float *radius, int nslots, const Geom &g, unsigned *mask,
@@ -464,7 +464,9 @@ struct TcSelectArgs {
 };
 // FP8: rowmax is scratch of `rows` floats
 cudaError_t launch_tc_pattern(const TcPatternArgs &a, float *rowmax, cudaStream_t st);
-cudaError_t launch_tc_tmax(long long nodes, int n, const int *nb_count, const int *nb_tpl, int *tmax, cudaStream_t st);
+#define QSK_TMAX_FEW (1 << 30)   // a node's template maximum: fewer than K positions hold its pattern
+cudaError_t launch_tc_tmax(long long nodes, int n, const int *nb_count, const int *nb_tpl, const int *tpl, const Geom &g,
+                           int K, int *tmax, cudaStream_t st);
 cudaError_t launch_tc_nodes(const TcNodeArgs &a, cudaStream_t st);
 // k_prep_sim and k_tc_nodes of one tensor-core step in one launch (rows of A
 // written, not learned)

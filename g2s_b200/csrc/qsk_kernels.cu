@@ -1030,72 +1030,6 @@ __device__ __forceinline__ unsigned mt_mix(unsigned a, unsigned b, unsigned c) {
     return c ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
 }
 
-// warp-cooperative regeneration of the 624-word state (3 dependency phases);
-// with OUT, draw k of the new block (tempered, converted) goes to out[k].
-// Branch-free: lanes past the end of a phase compute a clamped element and
-// store it into their own dummy slots (mt[624 + lane], dummy[lane]), which
-// keeps the phases free of divergent stores (3x faster than predicated ones).
-template <bool OUT>
-__device__ __forceinline__ void mt_twist(unsigned *mt, int lane, float *out, float *dummy) {
-    unsigned nv[8];
-    int kk[8];
-    // phase A: k in [0,227): old x[k], x[k+1], x[k+397]
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int k = lane + 32 * q;
-        const int kc = k < 227 ? k : 226;
-        kk[q] = k < 227 ? k : -1;
-        nv[q] = mt_mix(mt[kc], mt[kc + 1], mt[kc + 397]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int k = kk[q];
-        mt[k >= 0 ? k : 624 + lane] = nv[q];
-        if (OUT) *(k >= 0 ? out + k : dummy + lane) = mt_unit(mt_temper(nv[q]));
-    }
-    __syncwarp();
-    // phase B: k in [227,454): old x[k], x[k+1]; new x[k-227]
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int k = 227 + lane + 32 * q;
-        const int kc = k < 454 ? k : 453;
-        kk[q] = k < 454 ? k : -1;
-        nv[q] = mt_mix(mt[kc], mt[kc + 1], mt[kc - 227]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int k = kk[q];
-        mt[k >= 0 ? k : 624 + lane] = nv[q];
-        if (OUT) *(k >= 0 ? out + k : dummy + lane) = mt_unit(mt_temper(nv[q]));
-    }
-    __syncwarp();
-    // phase C: k in [454,623): old x[k], x[k+1]; new x[k-227]
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        const int k = 454 + lane + 32 * q;
-        const int kc = k < 623 ? k : 622;
-        kk[q] = k < 623 ? k : -1;
-        nv[q] = mt_mix(mt[kc], mt[kc + 1], mt[kc - 227]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        const int k = kk[q];
-        mt[k >= 0 ? k : 624 + lane] = nv[q];
-        if (OUT) *(k >= 0 ? out + k : dummy + lane) = mt_unit(mt_temper(nv[q]));
-    }
-    __syncwarp();
-    // k = 623: old x[623], new x[0], new x[396]
-    const unsigned y = mt_mix(mt[623], mt[0], mt[396]);
-    __syncwarp();
-    if (lane == 0) {
-        mt[623] = y;
-        if (OUT) out[623] = mt_unit(mt_temper(y));
-    }
-    __syncwarp();
-}
 
 // generator.seed(seedFromUnitFloat(seed) + 0)  (quantileSamplingModule.hpp:45-49,533-534):
 // the standard mt19937 initialisation, serial, on the calling thread
@@ -1112,199 +1046,97 @@ __device__ __forceinline__ void mt_seed(unsigned *mt, float sd) {
 }
 
 // ---------------------------------------------------------------------------
-// replay of the k-biggest scan + draw + write-back; one warp per slot
+// replay of the k-biggest scan + draw + write-back; one CTA per slot
 // ---------------------------------------------------------------------------
-#define RP_WARPS 4
-#define REC_CAP 1024          // records (padded to 4 per segment) of one tie super-run
-#define TAB_CAP 128           // segments of one tie super-run
-#define RNG_BUF (2 * REC_CAP + 640)   // draws of one super-run + one block
-#define SEG_WIN 256           // record counts and maxima of SEG_WIN segments staged per warp
-#define TEAM_MAX 8            // warps of one slot's team
+#define RP_WARPS 4            // slots (warps) per CTA of k_mt_prep
+#define RP_TEAM 8             // warps of one slot's team
+#define RP_THREADS (32 * RP_TEAM)
+#define REC_CAP 2048          // records staged at once
+#define RNG_BUF (2 * REC_CAP + 640)   // two draws per staged record + one block
+#define SEG_AHEAD 4           // windows of one segment per thread read at once
 
-struct __align__(16) WarpShared {
-    float rv_s[REC_CAP];      // super-run records (values), 16-byte aligned for cp.async
+struct __align__(16) ReplayShared {
+    float rv_s[REC_CAP];      // staged records (values), in scan order
     int ri_s[REC_CAP];        // and their scan indices
-    unsigned mt[624 + 32];    // + one dummy word per lane (branch-free twist)
-    float buf[RNG_BUF];
-    float dummy[32];
-    int tseg[TAB_CAP];        // super-run segments, their first padded record, record count
-    int tpre[TAB_CAP];
-    int tcnt[TAB_CAP];
-    int wc[SEG_WIN];          // record counts and maxima of segments [wbase, wbase + SEG_WIN)
-    float wm[SEG_WIN];
-    // a team of warps on one slot (k_replay with W > 1): the command warp 0
-    // posts, and the per-warp tie counts and slot maps of a super-run
-    int cmd, cmd_off, cmd_tp, cmd_xes, cmd_k, cmd_rp;
-    unsigned cmd_cpt;
-    float cmd_v;
-    int tw_sum[TEAM_MAX];
-    int tw_map[TEAM_MAX][QSK_KMAX];
+    unsigned mt[2][624];      // generator state, the next block written beside the last
+    float buf[RNG_BUF];       // draws
+    float w_top[RP_TEAM][QSK_KMAX];   // per warp: top-K of its part
+    int w_sum[RP_TEAM];       // per warp: records to stage
+    int4 w_fun[RP_TEAM];      // per warp: cpt function and draws of its part
+    int w_map[RP_TEAM][QSK_KMAX];     // per warp: slot map of its part
+    int stop, staged;         // first thread whose segment did not fit, records staged
 };
 
-enum TeamCommand : int { CMD_EXIT = 0, CMD_TWIST = 1, CMD_TWIST_OUT = 2, CMD_SUPER = 3 };
-
-// barrier 1 over the team's threads (barrier 0 stays free for __syncthreads)
-__device__ __forceinline__ void team_bar(int nthreads) { asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory"); }
-
-// mt_twist with the elements of each dependency phase spread over the NT
-// (>= 128) threads of a team
+// The next MT19937 block by the team, written beside the last one (the
+// recurrence reaches back 624, 623 and 227 words, so 227 words are
+// independent of one another): three phases, one barrier after each; with
+// OUT, draw k of the block goes to out[k].
 template <bool OUT>
-__device__ void mt_twist_team(unsigned *mt, int tid, int NT, float *out) {
-    unsigned nv[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int k = tid + i * NT;
-        nv[i] = k < 227 ? mt_mix(mt[k], mt[k + 1], mt[k + 397]) : 0u;
-    }
-    team_bar(NT);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int k = tid + i * NT;
-        if (k < 227) {
-            mt[k] = nv[i];
-            if (OUT) out[k] = mt_unit(mt_temper(nv[i]));
-        }
-    }
-    team_bar(NT);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int k = 227 + tid + i * NT;
-        nv[i] = k < 454 ? mt_mix(mt[k], mt[k + 1], mt[k - 227]) : 0u;
-    }
-    team_bar(NT);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int k = 227 + tid + i * NT;
-        if (k < 454) {
-            mt[k] = nv[i];
-            if (OUT) out[k] = mt_unit(mt_temper(nv[i]));
-        }
-    }
-    team_bar(NT);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int k = 454 + tid + i * NT;
-        nv[i] = k < 623 ? mt_mix(mt[k], mt[k + 1], mt[k - 227]) : 0u;
-    }
-    team_bar(NT);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int k = 454 + tid + i * NT;
-        if (k < 623) {
-            mt[k] = nv[i];
-            if (OUT) out[k] = mt_unit(mt_temper(nv[i]));
-        }
-    }
-    team_bar(NT);
-    if (tid == 0) {
-        const unsigned y = mt_mix(mt[623], mt[0], mt[396]);
-        mt[623] = y;
-        if (OUT) out[623] = mt_unit(mt_temper(y));
-    }
-    team_bar(NT);
+__device__ __forceinline__ void mt_block(const unsigned *old, unsigned *nw, int tid, float *out) {
+    auto put = [&](int k, unsigned y) {
+        nw[k] = y;
+        if (OUT) out[k] = mt_unit(mt_temper(y));
+    };
+    static_assert(RP_THREADS >= 227, "one word per thread and phase");
+    if (tid < 227) put(tid, mt_mix(old[tid], old[tid + 1], old[tid + 397]));
+    __syncthreads();
+    if (tid < 227) put(227 + tid, mt_mix(old[227 + tid], old[228 + tid], nw[tid]));
+    __syncthreads();
+    if (tid < 170) put(454 + tid, mt_mix(old[454 + tid], tid < 169 ? old[455 + tid] : nw[0], nw[227 + tid]));
+    __syncthreads();
 }
 
-// Make segments [q0, q0 + 32) readable from the window (w.wc / w.wm at q - wbase).
-// The scan only moves forward, so a miss restages the window from q0 on.
-__device__ __forceinline__ void win_cover(WarpShared &w, int &wbase, int q0, int nseg, const int *rc, const float *rm,
-                                          int lane) {
-    if (q0 >= wbase && q0 + 32 <= wbase + SEG_WIN) return;
-    __syncwarp();
-    wbase = q0;
-    int c[SEG_WIN / 32];
-    float m[SEG_WIN / 32];
-#pragma unroll
-    for (int i = 0; i < SEG_WIN / 32; ++i) {
-        const int q = q0 + lane + 32 * i;
-        c[i] = q < nseg ? rc[q] : 0;
-        m[i] = q < nseg ? rm[q] : -CUDART_INF_F;
-    }
-#pragma unroll
-    for (int i = 0; i < SEG_WIN / 32; ++i) {
-        w.wc[lane + 32 * i] = c[i];
-        w.wm[lane + 32 * i] = m[i];
-    }
-    __syncwarp();
-}
-
-// One MT19937 block of the slot's stream: regenerated by warp 0 alone (W ==
-// 1), or by the whole team, which warp 0 wakes with a command (W > 1).
-template <int W, bool OUT>
-__device__ __forceinline__ void rng_block(WarpShared &w, int lane, float *out) {
-    if constexpr (W == 1) {
-        mt_twist<OUT>(w.mt, lane, out, w.dummy);
-    } else {
-        __syncwarp();
-        if (lane == 0) {
-            w.cmd = OUT ? CMD_TWIST_OUT : CMD_TWIST;
-            w.cmd_off = OUT ? int(out - w.buf) : 0;
-        }
-        team_bar(32 * W);
-        mt_twist_team<OUT>(w.mt, threadIdx.x, 32 * W, out);
-    }
-}
-
-// Draw buffer with warp-replicated read pointer: rp/len live in registers of
-// every lane (all lanes execute the same control flow).
-template <int W>
-__device__ __forceinline__ void rng_refill(WarpShared &w, int lane, int &rp, int &len) {
-    const int unread = len - rp;   // <= 2 * REC_CAP by construction
-    // move the unread draws to the front (destinations never overtake sources)
-    __syncwarp();
-    for (int q = 0; 32 * q < unread; ++q) {
-        const int i = lane + 32 * q;
-        const float v = i < unread ? w.buf[rp + i] : 0.f;
-        __syncwarp();
-        if (i < unread) w.buf[i] = v;
-        __syncwarp();
-    }
-    rng_block<W, true>(w, lane, w.buf + unread);
-    len = unread + 624;
-    rp = 0;
-}
-
-template <int W>
-__device__ __forceinline__ void rng_ensure(WarpShared &w, int lane, int &rp, int &len, int need) {
-    if (len - rp < need) rng_refill<W>(w, lane, rp, len);
-}
+// A slot's draws: buf[rp, len) unread, the state in mt[par]; every thread of
+// the team holds the same values.
+struct Rng {
+    int rp = 0, len = 0, par = 0;
+};
 
 // at least `need` (<= 2 * REC_CAP) unread draws in the buffer
-template <int W>
-__device__ void rng_ensure_many(WarpShared &w, int lane, int &rp, int &len, int need) {
-    if (len - rp >= need) return;
-    const int unread = len - rp;
-    __syncwarp();
-    for (int q = 0; 32 * q < unread; ++q) {
-        const int i = lane + 32 * q;
-        const float v = i < unread ? w.buf[rp + i] : 0.f;
-        __syncwarp();
-        if (i < unread) w.buf[i] = v;
-        __syncwarp();
+__device__ __forceinline__ void rng_need(ReplayShared &w, int tid, Rng &g, int need) {
+    if (g.len - g.rp >= need) return;
+    __syncthreads();   // every thread has read the draws it took so far
+    const int unread = g.len - g.rp;
+    // the unread ones to the front (destinations never overtake sources)
+    for (int at = 0; at < unread && g.rp > 0; at += 4 * RP_THREADS) {
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = at + q * RP_THREADS + tid;
+            v[q] = i < unread ? w.buf[g.rp + i] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = at + q * RP_THREADS + tid;
+            if (i < unread) w.buf[i] = v[q];
+        }
+        __syncthreads();
     }
-    len = unread;
-    rp = 0;
-    while (len < need) {
-        rng_block<W, true>(w, lane, w.buf + len);
-        len += 624;
+    g.rp = 0;
+    g.len = unread;
+    while (g.len < need) {
+        mt_block<true>(w.mt[g.par], w.mt[g.par ^ 1], tid, w.buf + g.len);
+        g.par ^= 1;
+        g.len += 624;
     }
 }
 
-// advance the stream by n draws; whole blocks of 624 only regenerate the state
-template <int W>
-__device__ void rng_skip(WarpShared &w, int lane, int &rp, int &len, long long n) {
-    const long long avail = len - rp;
+// advance the stream by n draws; whole blocks only regenerate the state
+__device__ __forceinline__ void rng_skip(ReplayShared &w, int tid, Rng &g, long long n) {
+    const long long avail = g.len - g.rp;
     if (n <= avail) {
-        rp += int(n);
+        g.rp += int(n);
         return;
     }
     n -= avail;
-    rp = len;
-    while (n > 624) {
-        rng_block<W, false>(w, lane, nullptr);
-        n -= 624;
+    g.rp = g.len = 0;
+    for (; n > 624; n -= 624) {
+        mt_block<false>(w.mt[g.par], w.mt[g.par ^ 1], tid, nullptr);
+        g.par ^= 1;
     }
-    rng_refill<W>(w, lane, rp, len);
-    rp += int(n);
+    rng_need(w, tid, g, 1);
+    g.rp += int(n);
 }
 
 template <int KM>
@@ -1329,789 +1161,532 @@ __device__ __forceinline__ unsigned sel_u(const unsigned (&a)[KM], int i) {
     return r;
 }
 
-// One step of the reference's k-biggest scan for up to 32 consecutive
-// candidates at once (one per lane, lanes in scan order).  The value state is
-// a prefix top-K (associative merge), the tie counter cpt a composition of
-// "add" / "reset" functions, the draws a prefix count, and the position
-// updates of each trigger (swap of the tail slot, insertion, reservoir
-// replacement) slot maps whose composition is reduced across the warp.
-// State (cv, cp, cpt, rp) is replicated in all lanes.
-template <int KM>
-__device__ __forceinline__ void replay_chunk(int K, bool valid, float v, int m, float (&cv)[KM], unsigned (&cp)[KM],
-                                             unsigned &cpt, int &rp, const float *buf, int lane) {
-    const unsigned FULL = 0xffffffffu;
-    // 1. exclusive prefix top-K of the chunk's values, merged with the state
-    float st[KM];
-    st[0] = valid ? v : -CUDART_INF_F;
-#pragma unroll
-    for (int s = 1; s < KM; ++s) st[s] = -CUDART_INF_F;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        float rcv[KM], mrg[KM];
-#pragma unroll
-        for (int s = 0; s < KM; ++s) rcv[s] = __shfl_up_sync(FULL, st[s], off);
-        if (lane >= off) {
-            topk_merge<KM>(st, rcv, mrg);
-#pragma unroll
-            for (int s = 0; s < KM; ++s) st[s] = mrg[s];
-        }
-    }
-    float ex[KM], pre[KM];
-#pragma unroll
-    for (int s = 0; s < KM; ++s) {
-        float y = __shfl_up_sync(FULL, st[s], 1);
-        ex[s] = lane == 0 ? -CUDART_INF_F : y;
-    }
-    topk_merge<KM>(cv, ex, pre);
-    const float kth = sel_f<KM>(pre, K - 1);
-    const bool trig = valid && (v >= kth);
-    const bool gt = trig && (v > kth);
+// One trigger of the reference's scan (fKb.hpp): a value v >= the K-th draws x
+// among the xes tail slots holding the K-th and swaps it with slot K-1; above
+// the K-th it is inserted after the values >= v (the last slot drops out, cpt
+// restarts at 0 when the K-th was unique and counts on otherwise); equal to
+// the K-th it replaces slot K-1 with probability xes / (xes + cpt + 1) (a
+// second draw) and cpt counts on.  `slot` are the K positions, or a map of
+// slots (T int, an index i entering as -(i + 1)); returns the draws used.
+template <int KM, class T>
+__device__ __forceinline__ int replay_trigger(int K, float v, T entry, float (&cv)[KM], T (&slot)[KM], unsigned &cpt,
+                                              const float *u) {
+    const float kth = sel_f<KM>(cv, K - 1);
+    const bool gt = v > kth;
     int xes = 0, q = 0;
 #pragma unroll
     for (int s = 0; s < KM; ++s) {
-        if (s < K && pre[s] == kth) xes++;
-        if (s < K - 1 && pre[s] >= v) q++;
+        if (s < K && cv[s] == kth) xes++;
+        if (s < K - 1 && cv[s] >= v) q++;
     }
-    // 2. cpt as functions c -> r ? a : c + a, exclusive scan in lane order
-    int fr = 0, fa = 0;
-    if (trig) {
-        if (gt && xes == 1) { fr = 1; fa = 0; }
-        else { fr = 0; fa = 1; }
+    int x = K - xes + int(floorf(__fmul_rn(u[0], (float)xes)));
+    if (x > K - 1) x = K - 1;
+    T px = slot[0], pk = slot[0];
+#pragma unroll
+    for (int s = 1; s < KM; ++s) {
+        px = s == x ? slot[s] : px;
+        pk = s == K - 1 ? slot[s] : pk;
     }
-    int er = 0, ea = 0;   // exclusive composite
-    {
-        int ir = fr, ia = fa;   // inclusive composite (scan)
+    T sw[KM];
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            int rr = __shfl_up_sync(FULL, ir, off), ra = __shfl_up_sync(FULL, ia, off);
-            if (lane >= off) {
-                // earlier (rr,ra) then later (ir,ia)
-                if (!ir) { ir = rr; ia = ra + ia; }
-            }
-        }
-        int pr = __shfl_up_sync(FULL, ir, 1), pa = __shfl_up_sync(FULL, ia, 1);
-        if (lane > 0) { er = pr; ea = pa; }
-        // total composite from lane 31 for the state update below
-        int tr = __shfl_sync(FULL, ir, 31), ta = __shfl_sync(FULL, ia, 31);
-        const unsigned before = er ? unsigned(ea) : cpt + unsigned(ea);
-        const unsigned after = fr ? 0u : before + unsigned(fa);
-        // 3. draw offsets: 1 draw per trigger, a second one per tie
-        const unsigned b1 = __ballot_sync(FULL, trig), b2 = __ballot_sync(FULL, trig && !gt);
-        const unsigned lt = lanemask_lt();
-        const int off = __popc(b1 & lt) + __popc(b2 & lt);
-        int o[KM];
+    for (int s = 0; s < KM; ++s) sw[s] = (s == x) ? pk : ((s == K - 1) ? px : slot[s]);
+    if (gt) {
 #pragma unroll
-        for (int s = 0; s < KM; ++s) o[s] = s;
-        if (trig) {
-            const float u1 = buf[rp + off];
-            int x = K - xes + int(floorf(__fmul_rn(u1, (float)xes)));
-            if (x > K - 1) x = K - 1;
-            bool write = false;
-            if (!gt) {
-                const float u2 = buf[rp + off + 1];
-                write = __fmul_rn(__uint2float_rn(unsigned(xes) + after), u2) < (float)xes;
-            }
-            int sig[KM];
-#pragma unroll
-            for (int s = 0; s < KM; ++s) sig[s] = (s == x) ? K - 1 : ((s == K - 1) ? x : s);
-            if (gt) {
-#pragma unroll
-                for (int s = 0; s < KM; ++s) {
-                    if (s < K) {
-                        int prevs = s > 0 ? sig[s > 0 ? s - 1 : 0] : 0;
-                        o[s] = s < q ? sig[s] : (s == q ? -(m + 1) : prevs);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int s = 0; s < KM; ++s)
-                    if (s < K) o[s] = (write && s == K - 1) ? -(m + 1) : sig[s];
-            }
-        }
-        // 4. compose the slot maps in lane order (tree reduction to lane 0)
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            int later[KM];
-#pragma unroll
-            for (int s = 0; s < KM; ++s) later[s] = __shfl_down_sync(FULL, o[s], d);
-            if ((lane & (2 * d - 1)) == 0 && lane + d < 32) {
-                int c[KM];
-#pragma unroll
-                for (int s = 0; s < KM; ++s) c[s] = later[s] < 0 ? later[s] : sel_i<KM>(o, later[s]);
-#pragma unroll
-                for (int s = 0; s < KM; ++s) o[s] = c[s];
-            }
-        }
-        unsigned np[KM];
-#pragma unroll
-        for (int s = 0; s < KM; ++s) {
-            int t = __shfl_sync(FULL, o[s], 0);
-            np[s] = t < 0 ? unsigned(-(t + 1)) : sel_u<KM>(cp, t);
-        }
-#pragma unroll
-        for (int s = 0; s < KM; ++s) cp[s] = np[s];
-        // 5. state values, cpt, draw pointer
-        float last[KM], nv[KM];
-#pragma unroll
-        for (int s = 0; s < KM; ++s) last[s] = __shfl_sync(FULL, st[s], 31);
-        topk_merge<KM>(cv, last, nv);
-#pragma unroll
-        for (int s = 0; s < KM; ++s) cv[s] = nv[s];
-        cpt = tr ? unsigned(ta) : cpt + unsigned(ta);
-        rp += __popc(b1) + __popc(b2);
+        for (int s = 0; s < KM; ++s)
+            if (s < K) slot[s] = s < q ? sw[s] : (s == q ? entry : sw[s > 0 ? s - 1 : 0]);
+        topk_insert<KM>(cv, v);
+        cpt = (xes == 1) ? 0u : cpt + 1u;
+        return 1;
     }
+    cpt += 1u;
+    const bool write = __fmul_rn(__uint2float_rn(unsigned(xes) + cpt), u[1]) < (float)xes;
+#pragma unroll
+    for (int s = 0; s < KM; ++s)
+        if (s < K) slot[s] = (write && s == K - 1) ? entry : sw[s];
+    return 2;
 }
 
-// Steady-state fast path: every value of the state equals the K-th (so
-// xes = K and a trigger can only tie) and no candidate of the chunk exceeds
-// it.  Each tie uses two draws and increments cpt; lane ranks give both.
+// The scan over the staged records [r, n) by the whole team, thread t taking P
+// consecutive ones.  What a record does follows from prefixes: the K-th best
+// before it (a top-K scan), its draws (a count) and cpt (a composition of
+// "add" / "reset" functions); the position updates are slot maps, composed
+// in record order.  Three walks over a thread's records, one scan over the
+// team after each of the first two, a reduction of the maps after the third.
+// The state (cv, cp, cpt) is replicated in every thread.
 template <int KM>
-__device__ __forceinline__ void replay_chunk_ties(int K, bool tie, int m, unsigned (&cp)[KM], unsigned &cpt, int &rp,
-                                                  const float *buf, int lane) {
+__device__ __forceinline__ void team_scan(ReplayShared &w, int tid, int r, int n, int K, float (&cv)[KM],
+                                          unsigned (&cp)[KM], unsigned &cpt, Rng &g) {
     const unsigned FULL = 0xffffffffu;
-    const unsigned bt = __ballot_sync(FULL, tie);
-    const int rank = __popc(bt & lanemask_lt());
-    int o[KM];
+    const int lane = tid & 31, wid = tid >> 5;
+    // P odd keeps a warp's reads on distinct banks
+    const int P = ((n - r + RP_THREADS - 1) / RP_THREADS) | 1;
+    const int j0 = min(n, r + tid * P), j1 = min(n, j0 + P);
+    // 1. the K best before this thread's records
+    float pre[KM];
+    float top = -CUDART_INF_F;
+    {
+        float st[KM];
 #pragma unroll
-    for (int s = 0; s < KM; ++s) o[s] = s;
-    if (tie) {
-        const float u1 = buf[rp + 2 * rank];
-        const float u2 = buf[rp + 2 * rank + 1];
-        int x = int(floorf(__fmul_rn(u1, (float)K)));
-        if (x > K - 1) x = K - 1;
-        const unsigned after = cpt + unsigned(rank) + 1u;
-        const bool write = __fmul_rn(__uint2float_rn(unsigned(K) + after), u2) < (float)K;
+        for (int k = 0; k < KM; ++k) st[k] = -CUDART_INF_F;
+        for (int j = j0; j < j1; ++j) topk_insert<KM>(st, w.rv_s[j]);
+        top = st[0];
 #pragma unroll
-        for (int s = 0; s < KM; ++s) {
-            if (s < K) {
-                int sig = (s == x) ? K - 1 : ((s == K - 1) ? x : s);
-                o[s] = (write && s == K - 1) ? -(m + 1) : sig;
+        for (int off = 1; off < 32; off <<= 1) {
+            float rcv[KM], mrg[KM];
+#pragma unroll
+            for (int k = 0; k < KM; ++k) rcv[k] = __shfl_up_sync(FULL, st[k], off);
+            if (lane >= off) {
+                topk_merge<KM>(st, rcv, mrg);
+#pragma unroll
+                for (int k = 0; k < KM; ++k) st[k] = mrg[k];
+            }
+        }
+        if (lane == 31) {
+#pragma unroll
+            for (int k = 0; k < KM; ++k) w.w_top[wid][k] = st[k];
+        }
+#pragma unroll
+        for (int k = 0; k < KM; ++k) {
+            const float y = __shfl_up_sync(FULL, st[k], 1);
+            pre[k] = lane == 0 ? -CUDART_INF_F : y;
+        }
+        __syncthreads();
+        float e[KM], mrg[KM];
+        topk_merge<KM>(pre, cv, mrg);
+#pragma unroll
+        for (int k = 0; k < KM; ++k) pre[k] = mrg[k];
+        for (int q = 0; q < RP_TEAM; ++q) {
+#pragma unroll
+            for (int k = 0; k < KM; ++k) e[k] = w.w_top[q][k];
+            if (q < wid) {
+                topk_merge<KM>(pre, e, mrg);
+#pragma unroll
+                for (int k = 0; k < KM; ++k) pre[k] = mrg[k];
+            }
+            topk_merge<KM>(cv, e, mrg);   // the state after the run
+#pragma unroll
+            for (int k = 0; k < KM; ++k) cv[k] = mrg[k];
+        }
+    }
+    // 2. this thread's draws and cpt function c -> fr ? fa : c + fa
+    const bool active = j0 < j1 && top >= sel_f<KM>(pre, K - 1);
+    int nd = 0, fr = 0, fa = 0;
+    if (active) {
+        float st[KM];
+#pragma unroll
+        for (int k = 0; k < KM; ++k) st[k] = pre[k];
+        for (int j = j0; j < j1; ++j) {
+            const float v = w.rv_s[j];
+            const float kth = sel_f<KM>(st, K - 1);
+            if (!(v >= kth)) continue;
+            if (v > kth) {
+                int xes = 0;
+#pragma unroll
+                for (int k = 0; k < KM; ++k) xes += (k < K && st[k] == kth) ? 1 : 0;
+                nd += 1;
+                fr = xes == 1 ? 1 : fr;
+                fa = xes == 1 ? 0 : fa + 1;
+                topk_insert<KM>(st, v);
+            } else {
+                nd += 2;
+                fa += 1;
             }
         }
     }
+    int id = nd, ir = fr, ia = fa;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int dd = __shfl_up_sync(FULL, id, off), rr = __shfl_up_sync(FULL, ir, off), ra = __shfl_up_sync(FULL, ia, off);
+        if (lane >= off) {
+            id += dd;
+            if (!ir) {   // earlier (rr, ra) then later (0, ia)
+                ir = rr;
+                ia += ra;
+            }
+        }
+    }
+    if (lane == 31) w.w_fun[wid] = make_int4(id, ir, ia, 0);
+    int ed = __shfl_up_sync(FULL, id, 1), er = __shfl_up_sync(FULL, ir, 1), ea = __shfl_up_sync(FULL, ia, 1);
+    if (lane == 0) ed = er = ea = 0;
+    __syncthreads();
+    int total = 0;
+    unsigned mycpt = cpt;   // before this thread's records
+    {
+        unsigned cur = cpt;
+#pragma unroll
+        for (int q = 0; q < RP_TEAM; ++q) {
+            const int4 f = w.w_fun[q];
+            if (q == wid) {
+                ed += total;
+                mycpt = er ? unsigned(ea) : cur + unsigned(ea);
+            }
+            cur = f.y ? unsigned(f.z) : cur + unsigned(f.z);
+            total += f.x;
+        }
+        cpt = cur;
+    }
+    if (total == 0) return;   // nothing reaches the K-th
+    rng_need(w, tid, g, total);
+    // 3. this thread's slot map
+    int o[KM];
+#pragma unroll
+    for (int k = 0; k < KM; ++k) o[k] = k;
+    if (nd > 0) {
+        const float *u = w.buf + g.rp + ed;
+        for (int j = j0; j < j1; ++j) {
+            const float v = w.rv_s[j];
+            if (!(v >= sel_f<KM>(pre, K - 1))) continue;
+            u += replay_trigger<KM, int>(K, v, -(w.ri_s[j] + 1), pre, o, mycpt, u);
+        }
+    }
+    // composed in thread order: each warp's to its lane 0, then the warps'
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         int later[KM];
 #pragma unroll
-        for (int s = 0; s < KM; ++s) later[s] = __shfl_down_sync(FULL, o[s], d);
+        for (int k = 0; k < KM; ++k) later[k] = __shfl_down_sync(FULL, o[k], d);
         if ((lane & (2 * d - 1)) == 0) {
             int c[KM];
 #pragma unroll
-            for (int s = 0; s < KM; ++s) c[s] = later[s] < 0 ? later[s] : sel_i<KM>(o, later[s]);
+            for (int k = 0; k < KM; ++k) c[k] = later[k] < 0 ? later[k] : sel_i<KM>(o, later[k]);
 #pragma unroll
-            for (int s = 0; s < KM; ++s) o[s] = c[s];
+            for (int k = 0; k < KM; ++k) o[k] = c[k];
         }
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < KM; ++k) w.w_map[wid][k] = o[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < KM; ++k) o[k] = k;
+    for (int q = 0; q < RP_TEAM; ++q) {
+        int c[KM];
+#pragma unroll
+        for (int k = 0; k < KM; ++k) {
+            const int later = w.w_map[q][k];
+            c[k] = later < 0 ? later : sel_i<KM>(o, later);
+        }
+#pragma unroll
+        for (int k = 0; k < KM; ++k) o[k] = c[k];
     }
     unsigned np[KM];
 #pragma unroll
-    for (int s = 0; s < KM; ++s) {
-        int t = __shfl_sync(FULL, o[s], 0);
-        np[s] = t < 0 ? unsigned(-(t + 1)) : sel_u<KM>(cp, t);
-    }
+    for (int k = 0; k < KM; ++k) np[k] = o[k] < 0 ? unsigned(-(o[k] + 1)) : sel_u<KM>(cp, o[k]);
 #pragma unroll
-    for (int s = 0; s < KM; ++s) cp[s] = np[s];
-    const int nt = __popc(bt);
-    cpt += unsigned(nt);
-    rp += 2 * nt;
+    for (int k = 0; k < KM; ++k) cp[k] = np[k];
+    g.rp += total;
 }
 
-// A few candidates (the lanes of cand, in scan order): the reference's scan
-// step (fKb.hpp) applied to one trigger after the other, warp-uniformly.
-// A trigger v >= K-th draws x among the xes tail slots holding the K-th and
-// swaps it with slot K-1; above the K-th it is inserted after the values
-// >= v (the last slot drops out, cpt restarts at 0 when the K-th was unique
-// and counts on otherwise); equal to the K-th it replaces slot K-1 with
-// probability xes / (xes + cpt + 1) (a second draw) and cpt counts on.
-template <int KM>
-__device__ __forceinline__ void replay_scalar(int K, unsigned cand, float v, int m, float (&cv)[KM],
-                                              unsigned (&cp)[KM], unsigned &cpt, int &rp, const float *buf) {
-    const unsigned FULL = 0xffffffffu;
-    while (cand) {
-        const int l = __ffs(cand) - 1;
-        cand &= cand - 1u;
-        const float xv = __shfl_sync(FULL, v, l);
-        const unsigned xm = (unsigned)__shfl_sync(FULL, m, l);
-        const float kth = sel_f<KM>(cv, K - 1);
-        if (!(xv >= kth)) continue;
-        const bool gt = xv > kth;
-        int xes = 0, q = 0;
-#pragma unroll
-        for (int s = 0; s < KM; ++s) {
-            if (s < K && cv[s] == kth) xes++;
-            if (s < K - 1 && cv[s] >= xv) q++;
+// the cell of a slot without neighbours (one thread)
+__device__ unsigned marginal_cell(const ReplayArgs &A, const Slot &s) {
+    // marginal draw over the TI cells (simulation.hpp:586-605; complete TI)
+    unsigned chosen_cell = unsigned(int(floor((double)__fmul_rn(s.seed, __uint2float_rn((unsigned)A.ti_cells)))));
+    // float rounding of seed*cells can reach `cells` only for grids above 2^24 cells
+    if ((long long)chosen_cell >= A.ti_cells) chosen_cell = (unsigned)(A.ti_cells - 1);
+    if (A.complete_prefix) {
+        bool hasNaN = false;
+        for (int v = 0; v < A.nvar; ++v) hasNaN |= isnan(A.ti[(long long)chosen_cell * A.nvar + v]);
+        if (hasNaN) {
+            // NaN-safe draw (simulation.hpp:616-652): the first cell whose
+            // running count of complete cells reaches floor(seed*(complete/nvar))*nvar
+            const unsigned complete = (unsigned)A.complete_prefix[A.ti_cells - 1];
+            const unsigned pos2 = unsigned(int(floor((double)__fmul_rn(
+                                      s.seed, __uint2float_rn(complete / (unsigned)A.nvar))))) *
+                                  (unsigned)A.nvar;
+            long long lo2 = 0, hi2 = A.ti_cells;   // first index with prefix >= pos2
+            while (lo2 < hi2) {
+                long long mid = (lo2 + hi2) >> 1;
+                if ((unsigned)A.complete_prefix[mid] < pos2) lo2 = mid + 1;
+                else hi2 = mid;
+            }
+            chosen_cell = (unsigned)(lo2 < A.ti_cells ? lo2 : A.ti_cells - 1);
         }
-        int x = K - xes + int(floorf(__fmul_rn(buf[rp], (float)xes)));
-        if (x > K - 1) x = K - 1;
-        const unsigned px = sel_u<KM>(cp, x), pk = sel_u<KM>(cp, K - 1);
-        unsigned sw[KM];
-#pragma unroll
-        for (int s = 0; s < KM; ++s) sw[s] = (s == x) ? pk : ((s == K - 1) ? px : cp[s]);
-        if (gt) {
-#pragma unroll
-            for (int s = 0; s < KM; ++s)
-                if (s < K) cp[s] = s < q ? sw[s] : (s == q ? xm : sw[s > 0 ? s - 1 : 0]);
-            topk_insert<KM>(cv, xv);
-            cpt = (xes == 1) ? 0u : cpt + 1u;
-            rp += 1;
-        } else {
-            const unsigned after = cpt + 1u;
-            const bool write = __fmul_rn(__uint2float_rn(unsigned(xes) + after), buf[rp + 1]) < (float)xes;
-#pragma unroll
-            for (int s = 0; s < KM; ++s) cp[s] = (write && s == K - 1) ? xm : sw[s];
-            cpt = after;
-            rp += 2;
+    }
+    return chosen_cell;
+}
+
+// write-back of a slot's draw (one thread)
+__device__ __forceinline__ void replay_write(const ReplayArgs &A, const Slot &s, unsigned chosen_cell) {
+    if (A.node_cell) A.node_cell[s.node] = chosen_cell;
+    if (A.full) {
+        // -fs: the node's variable only (simulation.hpp:1016-1024)
+        const long long val = (long long)s.cell * A.nvar + s.var;
+        if (A.state && isnan(A.state[val])) A.state[val] = A.ti[(long long)chosen_cell * A.nvar + s.var];
+        if (A.id_image) A.id_image[val] = chosen_cell * A.nti + A.ti_id;
+    } else {
+        if (A.state) {
+            for (int v = 0; v < A.nvar; ++v) {
+                float *dst = A.state + (long long)s.cell * A.nvar + v;
+                if (isnan(*dst)) *dst = A.ti[(long long)chosen_cell * A.nvar + v];
+            }
         }
+        if (A.id_image) A.id_image[s.cell] = chosen_cell * A.nti + A.ti_id;
     }
 }
 
+__device__ __forceinline__ void cp_async4(void *smem_dst, const void *gmem_src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
+}
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// One tie super-run: no record of the run exceeds the K-th value V of the
-// state, so the state's values stay as they are, every record equal to V is a
-// tie (two draws, cpt + 1, a swap inside the xes tail slots that hold V and a
-// possible replacement at K-1) and the others are no-ops.  The run's segments
-// (w.tseg/tpre/tcnt, E entries, Tp padded records) arrive in shared memory by
-// the 16-byte asynchronous copies issued while they were gathered; lane l
-// then owns a contiguous range of the run, counts its ties, composes the slot
-// maps of its ties on its own, and one warp reduction combines the 32 lane
-// maps in order.
-// A super-run on a team of W warps (W > 1): thread t of the team owns
-// records [t*P, t*P + P) of the staged run (the parameters warp 0 posted),
-// the team's tie counts are scanned through shared memory, every thread
-// composes the slot maps of its ties, and the warp maps are composed in warp
-// order.  Returns the tie count and the composed map (in every thread).
-template <int KM, int W>
-__device__ void super_team(WarpShared &w, int tid, int &total, int (&o)[KM]) {
+// The k best of one slot, one CTA: the reference's findKBiggest replayed over
+// the map's records in scan order.
+//
+// Windows of one segment per thread are filtered by the whole team: a segment
+// can hold a candidate only if its maximum reaches the K-th best of the state
+// and of the window's earlier segment maxima (a lower bound of the K-th at
+// its turn).  The records of the segments left, a few dozen on a continuous
+// map, thousands where most positions tie, go to shared memory in scan order
+// and the team scans them from there (team_scan).  What bounds a slot is the
+// chain of global reads (two or three per 1024 segments), of barriers, and
+// the draws.  Every thread runs the same control flow.  Against one warp
+// that read each candidate segment on its own and replayed 32 records a step
+// (mean of a level, launch to end): a 200x200 continuous simulation (n = 50)
+// 47 -> 14 us, categorical 101x90 (n = 20) 40 -> 25 us, 250x250 -> 500x500
+// (n = 80) 65 -> 54 us; one slot of 26,000 segments 559 -> 230 us, of which
+// the generator blocks of its first masked stretch are 210.
+template <int KM>
+__global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayArgs A) {
+    __shared__ ReplayShared w;
+    constexpr int NT = RP_THREADS;
     const unsigned FULL = 0xffffffffu;
-    constexpr int NT = 32 * W;
-    const int lane = tid & 31, wid = tid >> 5;
-    const int Tp = w.cmd_tp, xes = w.cmd_xes, K = w.cmd_k, rp = w.cmd_rp;
-    const unsigned cpt = w.cmd_cpt;
-    const float V = w.cmd_v;
-    // P odd keeps a warp's reads on distinct banks; P <= REC_CAP / NT + 1 bits
-    const int P = ((Tp + NT - 1) / NT) | 1;
-    const int j0 = min(Tp, tid * P);
-    const int j1 = min(Tp, j0 + P);
-    unsigned tm = 0u;
-    for (int j = j0; j < j1; ++j) tm |= unsigned(w.rv_s[j] == V) << (j - j0);
-    const int mine = __popc(tm);
-    int incl = mine;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int y = __shfl_up_sync(FULL, incl, off);
-        if (lane >= off) incl += y;
-    }
-    if (lane == 31) w.tw_sum[wid] = incl;
-    team_bar(NT);
-    int before = 0;
-    total = 0;
-#pragma unroll
-    for (int q = 0; q < W; ++q) {
-        const int t = w.tw_sum[q];
-        before += q < wid ? t : 0;
-        total += t;
-    }
-    int rank = before + incl - mine;
-#pragma unroll
-    for (int s2 = 0; s2 < KM; ++s2) o[s2] = s2;
-    while (tm) {
-        const int j = j0 + __ffs(tm) - 1;
-        tm &= tm - 1u;
-        const float u1 = w.buf[rp + 2 * rank];
-        const float u2 = w.buf[rp + 2 * rank + 1];
-        int x = K - xes + int(floorf(__fmul_rn(u1, (float)xes)));
-        if (x > K - 1) x = K - 1;
-        const unsigned after = cpt + unsigned(rank) + 1u;
-        const bool write = __fmul_rn(__uint2float_rn(unsigned(xes) + after), u2) < (float)xes;
-        const int ox = sel_i<KM>(o, x), ok1 = sel_i<KM>(o, K - 1);
-        const int wr = -(w.ri_s[j] + 1);
-#pragma unroll
-        for (int s2 = 0; s2 < KM; ++s2) {
-            if (s2 == x) o[s2] = ok1;
-            if (s2 == K - 1) o[s2] = write ? wr : ox;
-        }
-        ++rank;
-    }
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        int later[KM];
-#pragma unroll
-        for (int s2 = 0; s2 < KM; ++s2) later[s2] = __shfl_down_sync(FULL, o[s2], d);
-        if ((lane & (2 * d - 1)) == 0) {
-            int c[KM];
-#pragma unroll
-            for (int s2 = 0; s2 < KM; ++s2) c[s2] = later[s2] < 0 ? later[s2] : sel_i<KM>(o, later[s2]);
-#pragma unroll
-            for (int s2 = 0; s2 < KM; ++s2) o[s2] = c[s2];
-        }
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int s2 = 0; s2 < KM; ++s2) w.tw_map[wid][s2] = o[s2];
-    }
-    team_bar(NT);
-#pragma unroll
-    for (int s2 = 0; s2 < KM; ++s2) o[s2] = w.tw_map[0][s2];
-#pragma unroll
-    for (int q = 1; q < W; ++q) {
-        int c[KM];
-#pragma unroll
-        for (int s2 = 0; s2 < KM; ++s2) {
-            const int later = w.tw_map[q][s2];
-            c[s2] = later < 0 ? later : sel_i<KM>(o, later);
-        }
-#pragma unroll
-        for (int s2 = 0; s2 < KM; ++s2) o[s2] = c[s2];
-    }
-}
-
-// warps 1..W-1 of a team: run the commands warp 0 posts until it is done
-template <int KM, int W>
-__device__ void team_helper(WarpShared &w) {
-    for (;;) {
-        team_bar(32 * W);
-        const int c = w.cmd;
-        if (c == CMD_EXIT) return;
-        if (c == CMD_TWIST_OUT) {
-            mt_twist_team<true>(w.mt, threadIdx.x, 32 * W, w.buf + w.cmd_off);
-        } else if (c == CMD_TWIST) {
-            mt_twist_team<false>(w.mt, threadIdx.x, 32 * W, nullptr);
-        } else {
-            int tot, o[KM];
-            super_team<KM, W>(w, threadIdx.x, tot, o);
-        }
-    }
-}
-
-template <int KM, int W>
-__device__ void replay_super_run(int K, float V, int xes, int E, int Tp, const float *rv, const int *ri, unsigned (&cp)[KM],
-                                 unsigned &cpt, int &rp, int &len, WarpShared &w, int lane) {
-    const unsigned FULL = 0xffffffffu;
-    cp_async_wait_all();   // the copies issued while the run was gathered
-    __syncwarp();
-    for (int e = lane; e < E; e += 32) {
-        const int c = w.tcnt[e], pre = w.tpre[e];
-        for (int k = c; k < ((c + 3) & ~3); ++k) w.rv_s[pre + k] = -CUDART_INF_F;
-    }
-    __syncwarp();
-    if constexpr (W > 1) {
-        // draws for every record (at most two per tie), then the team
-        rng_ensure_many<W>(w, lane, rp, len, 2 * Tp);
-        __syncwarp();
-        if (lane == 0) {
-            w.cmd = CMD_SUPER;
-            w.cmd_tp = Tp;
-            w.cmd_v = V;
-            w.cmd_xes = xes;
-            w.cmd_k = K;
-            w.cmd_rp = rp;
-            w.cmd_cpt = cpt;
-        }
-        team_bar(32 * W);
-        int total, o[KM];
-        super_team<KM, W>(w, threadIdx.x, total, o);
-        unsigned np[KM];
-#pragma unroll
-        for (int s2 = 0; s2 < KM; ++s2) np[s2] = o[s2] < 0 ? unsigned(-(o[s2] + 1)) : sel_u<KM>(cp, o[s2]);
-#pragma unroll
-        for (int s2 = 0; s2 < KM; ++s2) cp[s2] = np[s2];
-        cpt += unsigned(total);
-        rp += 2 * total;
-        __syncwarp();
+    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    const int b = blockIdx.x;
+    const Slot &sl = A.slots[b];
+    const int flags = sl.flags;
+    // only_flagged: the slots the hash select leaves (fewer valid positions
+    // than k)
+    if (A.only_flagged && (flags & (SLOT_SKIP | SLOT_EMIT_MASKED)) != SLOT_EMIT_MASKED) return;
+    const Geom &g = A.g;
+    if (flags & SLOT_SKIP) {
+        if (tid != 0 || !(A.state || A.node_cell)) return;
+        replay_write(A, sl, marginal_cell(A, sl));
         return;
     }
-    // lane l owns records [l*P, l*P + P); P odd keeps the lanes' reads on
-    // distinct shared-memory banks (P <= 33 fits a 64-bit tie mask)
-    const int P = ((Tp + 31) >> 5) | 1;
-    const int j0 = min(Tp, lane * P);
-    const int j1 = min(Tp, j0 + P);
-    unsigned long long tmask = 0ull;
-#pragma unroll 4
-    for (int j = j0; j < j1; ++j) tmask |= (unsigned long long)(w.rv_s[j] == V) << (j - j0);
-    const int mine = __popcll(tmask);
-    int incl = mine;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int y = __shfl_up_sync(FULL, incl, off);
-        if (lane >= off) incl += y;
-    }
-    const int total = __shfl_sync(FULL, incl, 31);
-    int rank = incl - mine;
-    rng_ensure_many<W>(w, lane, rp, len, 2 * total);
-    int o[KM];
-#pragma unroll
-    for (int s2 = 0; s2 < KM; ++s2) o[s2] = s2;
-    while (tmask) {
-        const int j = j0 + __ffsll((long long)tmask) - 1;
-        tmask &= tmask - 1ull;
-        const float u1 = w.buf[rp + 2 * rank];
-        const float u2 = w.buf[rp + 2 * rank + 1];
-        int x = K - xes + int(floorf(__fmul_rn(u1, (float)xes)));
-        if (x > K - 1) x = K - 1;
-        const unsigned after = cpt + unsigned(rank) + 1u;
-        const bool write = __fmul_rn(__uint2float_rn(unsigned(xes) + after), u2) < (float)xes;
-        // op = (write at K-1) o (swap x, K-1); composed after the lane's earlier ops
-        const int ox = sel_i<KM>(o, x), ok1 = sel_i<KM>(o, K - 1);
-        const int wr = -(w.ri_s[j] + 1);
-#pragma unroll
-        for (int s2 = 0; s2 < KM; ++s2) {
-            if (s2 == x) o[s2] = ok1;
-            if (s2 == K - 1) o[s2] = write ? wr : ox;
-        }
-        ++rank;
-    }
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        int later[KM];
-#pragma unroll
-        for (int s2 = 0; s2 < KM; ++s2) later[s2] = __shfl_down_sync(FULL, o[s2], d);
-        if ((lane & (2 * d - 1)) == 0) {
-            int c[KM];
-#pragma unroll
-            for (int s2 = 0; s2 < KM; ++s2) c[s2] = later[s2] < 0 ? later[s2] : sel_i<KM>(o, later[s2]);
-#pragma unroll
-            for (int s2 = 0; s2 < KM; ++s2) o[s2] = c[s2];
-        }
-    }
-    unsigned np[KM];
-#pragma unroll
-    for (int s2 = 0; s2 < KM; ++s2) {
-        int t = __shfl_sync(FULL, o[s2], 0);
-        np[s2] = t < 0 ? unsigned(-(t + 1)) : sel_u<KM>(cp, t);
-    }
-#pragma unroll
-    for (int s2 = 0; s2 < KM; ++s2) cp[s2] = np[s2];
-    cpt += unsigned(total);
-    rp += 2 * total;
-    __syncwarp();
-}
-
-// Tie stream (the state holds K finite values, the K-th is V, xes of them
-// equal V): segments from `sg` on whose maximum is V are ties or no-ops,
-// those below V are skipped, and the first segment above V ends the stream.  Segments are gathered into super-runs of
-// at most REC_CAP padded records and TAB_CAP segments.  Returns the first
-// segment above V, or nseg.
-template <int KM, int W>
-__device__ int replay_tie_stream(int K, float V, int xes, int sg, int nseg, const float *rv, const int *ri, const int *rc,
-                                 const float *rm, int &wbase, unsigned (&cp)[KM], unsigned &cpt, int &rp, int &len,
-                                 WarpShared &w, int lane) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned lt = lanemask_lt();
-    for (;;) {
-        int E = 0, Tp = 0, stop = -1;
-        for (;;) {
-            if (sg >= nseg) {
-                stop = nseg;
-                break;
-            }
-            win_cover(w, wbase, sg, nseg, rc, rm, lane);
-            const int q = sg + lane;
-            const int c = w.wc[q - wbase];
-            const float m = w.wm[q - wbase];
-            const unsigned brk = __ballot_sync(FULL, c > 0 && m > V);
-            const unsigned lim = brk ? ((1u << (__ffs(brk) - 1)) - 1u) : FULL;
-            const bool elig = ((lim >> lane) & 1u) && c > 0 && m == V;
-            const int pc = elig ? ((c + 3) & ~3) : 0;
-            int incl = pc;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int y = __shfl_up_sync(FULL, incl, off);
-                if (lane >= off) incl += y;
-            }
-            const unsigned EL = __ballot_sync(FULL, elig);
-            const int epos = E + __popc(EL & lt);
-            // the limits are monotone in lane order: the taken lanes are a prefix of EL
-            const bool take = elig && Tp + incl <= REC_CAP && epos < TAB_CAP;
-            const unsigned TK = __ballot_sync(FULL, take);
-            if (take) {
-                // the segment's records go to the run's buffers right away, so
-                // the copies overlap the rest of the gathering
-                const int dst = Tp + incl - pc;
-                w.tseg[epos] = q;
-                w.tpre[epos] = dst;
-                w.tcnt[epos] = c;
-                const long long src = (long long)q * QSK_SEG;
-                for (int k = 0; k < pc; k += 4) {
-                    cp_async16(&w.rv_s[dst + k], rv + src + k);
-                    cp_async16(&w.ri_s[dst + k], ri + src + k);
-                }
-            }
-            const int hi = TK ? 31 - __clz(TK) : 0;
-            const int add = __shfl_sync(FULL, incl, hi);
-            if (TK) {
-                Tp += add;
-                E += __popc(TK);
-            }
-            const unsigned left = EL & ~TK;
-            if (left) {   // capacity reached: the next run starts at the first segment left out
-                sg += __ffs(left) - 1;
-                break;
-            }
-            if (brk) {
-                sg += __ffs(brk) - 1;
-                stop = sg;
-                break;
-            }
-            sg += 32;
-        }
-        __syncwarp();
-        if (E > 0) replay_super_run<KM, W>(K, V, xes, E, Tp, rv, ri, cp, cpt, rp, len, w, lane);
-        if (stop >= 0) return stop;
-    }
-}
-
-// W == 1: RP_WARPS slots per CTA, one warp each.  W > 1 (what the launcher
-// uses): one slot per CTA; warp 0 replays it and the other W-1 warps join it
-// for the MT19937 blocks and the tie super-runs.
-template <int KM, int W>
-__global__ void __launch_bounds__(W == 1 ? 32 * RP_WARPS : 32 * W) k_replay(ReplayArgs A) {
-    extern __shared__ __align__(16) unsigned char rp_smem[];
-    WarpShared *wsh = reinterpret_cast<WarpShared *>(rp_smem);
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = W == 1 ? blockIdx.x * RP_WARPS + wib : blockIdx.x;
-    if (b >= A.nslots) return;
-    // only_flagged: the slots the hash select leaves (marginal draws, fewer
-    // valid positions than k); every warp of a team leaves together
-    if (A.only_flagged && !(A.slots[b].flags & (SLOT_SKIP | SLOT_EMIT_MASKED))) return;
-    WarpShared &w = wsh[W == 1 ? wib : 0];
-    if constexpr (W > 1) {
-        if (wib > 0) {
-            team_helper<KM, W>(w);
-            return;
-        }
-    }
-    const Slot s = A.slots[b];
-    const Geom &g = A.g;
+    const Slot &s = sl;
     const int K = s.K;
-    const unsigned FULL = 0xffffffffu;
-
+    Rng rng;
+    // generator state: seeded here, or prepared by k_mt_prep together with
+    // the blocks that the first masked stretch of the scan skips
+    long long preskip = 0;
+    if (A.mt_state) {
+        // 156 16-byte copies (state rows and w.mt are 16-byte aligned), awaited
+        // with the first records
+        for (int q = tid; q < 156; q += NT) cp_async16(&w.mt[0][4 * q], A.mt_state + (long long)b * 624 + 4 * q);
+        preskip = A.mt_pre[b];
+    } else if (tid == 0) {
+        mt_seed(w.mt[0], s.seed);
+    }
     float cv[KM];
     unsigned cp[KM];
 #pragma unroll
     for (int q = 0; q < KM; ++q) { cv[q] = -CUDART_INF_F; cp[q] = 0xffffffffu; }
-    unsigned chosen_cell = 0;
-    bool have = false;
+    unsigned cpt = 0;
+    long long last = -1;
+    const bool emit_masked = (flags & (SLOT_EMIT_MASKED | SLOT_MISSING)) != 0;
+    const float *rv = A.rec_val + (long long)b * g.nseg * QSK_SEG;
+    const int *ri = A.rec_idx + (long long)b * g.nseg * QSK_SEG;
+    const int *rc = A.rec_cnt + (long long)b * g.nseg;
+    const float *rm = A.rec_max + (long long)b * g.nseg;
 
-    if (s.flags & SLOT_SKIP) {
-        if (A.state || A.node_cell) {
-            // marginal draw over the TI cells (simulation.hpp:586-605; complete TI)
-            chosen_cell = unsigned(int(floor((double)__fmul_rn(s.seed, __uint2float_rn((unsigned)A.ti_cells)))));
-            // float rounding of seed*cells can reach `cells` only for grids above 2^24 cells
-            if ((long long)chosen_cell >= A.ti_cells) chosen_cell = (unsigned)(A.ti_cells - 1);
-            if (A.complete_prefix) {
-                bool hasNaN = false;
-                for (int v = 0; v < A.nvar; ++v) hasNaN |= isnan(A.ti[(long long)chosen_cell * A.nvar + v]);
-                if (hasNaN) {
-                    // NaN-safe draw (simulation.hpp:616-652): the first cell whose
-                    // running count of complete cells reaches floor(seed*(complete/nvar))*nvar
-                    const unsigned complete = (unsigned)A.complete_prefix[A.ti_cells - 1];
-                    const unsigned pos2 = unsigned(int(floor((double)__fmul_rn(
-                                              s.seed, __uint2float_rn(complete / (unsigned)A.nvar))))) *
-                                          (unsigned)A.nvar;
-                    long long lo2 = 0, hi2 = A.ti_cells;   // first index with prefix >= pos2
-                    while (lo2 < hi2) {
-                        long long mid = (lo2 + hi2) >> 1;
-                        if ((unsigned)A.complete_prefix[mid] < pos2) lo2 = mid + 1;
-                        else hi2 = mid;
-                    }
-                    chosen_cell = (unsigned)(lo2 < A.ti_cells ? lo2 : A.ti_cells - 1);
-                }
-            }
-            have = true;
+    int sg = 0;
+    while (sg < g.nseg) {
+        int c[SEG_AHEAD];
+        float m[SEG_AHEAD];
+#pragma unroll
+        for (int i = 0; i < SEG_AHEAD; ++i) {
+            const int q = sg + i * NT + tid;
+            c[i] = q < g.nseg ? rc[q] : 0;
+            m[i] = q < g.nseg ? rm[q] : -CUDART_INF_F;
         }
-    } else {
-        // generator state: seeded here, or prepared by k_mt_prep together with
-        // the blocks that the first masked stretch of the scan skips
-        long long preskip = 0;
-        if (A.mt_state) {
-            // 156 16-byte copies (state rows and w.mt are 16-byte aligned)
-            for (int i = lane; i < 156; i += 32) cp_async16(&w.mt[4 * i], A.mt_state + (long long)b * 624 + 4 * i);
-            cp_async_wait_all();
-            preskip = A.mt_pre[b];
-        } else if (lane == 0) {
-            mt_seed(w.mt, s.seed);
-        }
-        __syncwarp();
-        int rp = 0, len = 0;
-        unsigned cpt = 0;
-        long long last = -1;
-        const bool emit_masked = (s.flags & (SLOT_EMIT_MASKED | SLOT_MISSING)) != 0;
-        const float *rv = A.rec_val + (long long)b * g.nseg * QSK_SEG;
-        const int *ri = A.rec_idx + (long long)b * g.nseg * QSK_SEG;
-        const int *rc = A.rec_cnt + (long long)b * g.nseg;
-        const float *rm = A.rec_max + (long long)b * g.nseg;
-        // general replay of one segment's records, 32 per step
-        auto general_segment = [&](int sg, int cnt, float smax) {
-            const long long base = (long long)sg * QSK_SEG;
-            int r0 = 0;
-            while (r0 < cnt) {
-                const float kth0 = sel_f<KM>(cv, K - 1);
-                if (smax < kth0) break;   // nothing left in this segment can enter
-                const bool filling = (kth0 == -CUDART_INF_F);
-                const int width = filling ? 1 : 32;
-                const int j = r0 + lane;
-                const bool valid = lane < width && j < cnt;
-                const float v = valid ? rv[base + j] : -CUDART_INF_F;
-                const int m = valid ? ri[base + j] : 0;
-                const unsigned cand = __ballot_sync(FULL, valid && v >= kth0);
-                if (cand == 0u) {
-                    r0 += width;
-                    continue;
-                }
-                if (filling && !emit_masked) {
-                    // masked positions between the previous record and this one are
-                    // -inf ties while fewer than K finite values have been seen:
-                    // two draws and one cpt increment each, no visible slot change
-                    const long long mm = __shfl_sync(FULL, (long long)m, 0);
-                    long long c = (mm - (last + 1)) - (valid_prefix(g, s.lo, mm) - valid_prefix(g, s.lo, last + 1));
-                    if (c > 0) {
-                        // the first skip covers the prepared blocks (c >= the masked
-                        // positions before the first valid one, so 2c > preskip)
-                        rng_skip<W>(w, lane, rp, len, 2 * c - preskip);
-                        preskip = 0;
-                        cpt += unsigned(c);
-                    }
-                }
-                rng_ensure<W>(w, lane, rp, len, 64);
-                // all K state values equal and nothing above them in the chunk
-                if (!filling && sel_f<KM>(cv, 0) == kth0 && __ballot_sync(FULL, valid && v > kth0) == 0) {
-                    replay_chunk_ties<KM>(K, valid && v == kth0, m, cp, cpt, rp, w.buf, lane);
-                } else if (__popc(cand) <= 4) {
-                    replay_scalar<KM>(K, cand, v, m, cv, cp, cpt, rp, w.buf);
-                } else {
-                    replay_chunk<KM>(K, valid, v, m, cv, cp, cpt, rp, w.buf, lane);
-                }
-                const unsigned vb = __ballot_sync(FULL, valid);
-                last = __shfl_sync(FULL, (long long)m, 31 - __clz(vb));
-                r0 += width;
-            }
-        };
-        int sg = 0, wbase = -SEG_WIN;
-        while (sg < g.nseg) {
-            const float kth_s = sel_f<KM>(cv, K - 1);
-            if (kth_s != -CUDART_INF_F) {
-                // K finite values: tie super-runs up to the first segment above V
-                int xes = 0;
 #pragma unroll
-                for (int q = 0; q < KM; ++q) xes += (q < K && cv[q] == kth_s) ? 1 : 0;
-                sg = replay_tie_stream<KM, W>(K, kth_s, xes, sg, g.nseg, rv, ri, rc, rm, wbase, cp, cpt, rp, len, w,
-                                              lane);
-                if (sg >= g.nseg) break;
-                win_cover(w, wbase, sg, g.nseg, rc, rm, lane);
-                general_segment(sg, w.wc[sg - wbase], w.wm[sg - wbase]);
-                ++sg;
-                continue;
-            }
-            // general replay, 32 segments at a time, until K finite values are held
-            win_cover(w, wbase, sg, g.nseg, rc, rm, lane);
-            const int myc = w.wc[sg - wbase + lane];
-            const float mym = w.wm[sg - wbase + lane];
-            unsigned nz = __ballot_sync(FULL, myc > 0 && mym >= kth_s);
-            int next = sg + 32;
-            while (nz) {
-                const int l = __ffs(nz) - 1;
-                nz &= nz - 1;
-                general_segment(sg + l, __shfl_sync(FULL, myc, l), __shfl_sync(FULL, mym, l));
-                if (sel_f<KM>(cv, K - 1) != -CUDART_INF_F) {
-                    next = sg + l + 1;
-                    break;
-                }
-            }
-            sg = next;
-        }
-        // merge loop (quantileSamplingModule.hpp:546-557): repeated first-max extraction
-        float fv[KM];
-        unsigned fp[KM];
+        for (int i = 0; i < SEG_AHEAD; ++i) {
+            const int q0 = sg + i * NT;
+            if (q0 >= g.nseg) break;
+            for (;;) {   // until the window's segments are staged and scanned
+                const float kth = sel_f<KM>(cv, K - 1);
+                if (!__syncthreads_or(c[i] > 0 && m[i] >= kth)) break;
+                bool fl = c[i] > 0 && m[i] >= kth;
+                if (__syncthreads_or(fl && (m[i] > kth || kth == -CUDART_INF_F))) {
+                    // K-th best of the state and the earlier segments of the window
+                    float st[KM], pre[KM];
+                    st[0] = c[i] > 0 ? m[i] : -CUDART_INF_F;
 #pragma unroll
-        for (int j = 0; j < KM; ++j) {
-            fv[j] = -CUDART_INF_F;
-            fp[j] = 0xffffffffu;
-            if (j < K) {
-                int best = 0;
-                float bv = cv[0];
+                    for (int k = 1; k < KM; ++k) st[k] = -CUDART_INF_F;
 #pragma unroll
-                for (int l2 = 1; l2 < KM; ++l2)
-                    if (l2 < K && cv[l2] > bv) { best = l2; bv = cv[l2]; }
-                fv[j] = bv;
-                fp[j] = sel_u<KM>(cp, best);
+                    for (int off = 1; off < 32; off <<= 1) {
+                        float rcv[KM], mrg[KM];
 #pragma unroll
-                for (int l2 = 0; l2 < KM; ++l2)
-                    if (l2 == best) cv[l2] = -CUDART_INF_F;
-            }
-        }
-        // sample(): std::sort by score — insertion sort (stable) for K <= 16
+                        for (int k = 0; k < KM; ++k) rcv[k] = __shfl_up_sync(FULL, st[k], off);
+                        if (lane >= off) {
+                            topk_merge<KM>(st, rcv, mrg);
 #pragma unroll
-        for (int a2 = 1; a2 < KM; ++a2) {
-            if (a2 < K) {
-#pragma unroll
-                for (int c = a2; c > 0; --c) {
-                    if (fv[c] > fv[c - 1]) {
-                        float tv = fv[c]; fv[c] = fv[c - 1]; fv[c - 1] = tv;
-                        unsigned tp = fp[c]; fp[c] = fp[c - 1]; fp[c - 1] = tp;
-                    }
-                }
-            }
-        }
-        if (lane == 0 && A.out_val) {
-#pragma unroll
-            for (int j = 0; j < KM; ++j)
-                if (j < K) {
-                    unsigned out = fp[j];
-                    if (A.out_cells) {
-                        // cvtIndexToPosition (CPUThreadDevice.cpp:257-268)
-                        unsigned position = 0, div = (unsigned)g.N;
-                        for (int d = g.nd - 1; d >= 0; --d) {
-                            unsigned f = (unsigned)g.fft[d], sr = (unsigned)g.src[d];
-                            div /= f;
-                            position = position * sr + ((f - (out / div) % f - (unsigned)s.mn[d] - 1u) + sr) % sr;
+                            for (int k = 0; k < KM; ++k) st[k] = mrg[k];
                         }
-                        out = position;
                     }
-                    A.out_val[(long long)b * K + j] = fv[j];
-                    A.out_pos[(long long)b * K + j] = out;
+                    if (lane == 31) {
+#pragma unroll
+                        for (int k = 0; k < KM; ++k) w.w_top[wid][k] = st[k];
+                    }
+#pragma unroll
+                    for (int k = 0; k < KM; ++k) {
+                        const float y = __shfl_up_sync(FULL, st[k], 1);
+                        pre[k] = lane == 0 ? -CUDART_INF_F : y;
+                    }
+                    __syncthreads();
+                    float mrg[KM], e[KM];
+                    topk_merge<KM>(pre, cv, mrg);
+#pragma unroll
+                    for (int k = 0; k < KM; ++k) pre[k] = mrg[k];
+                    for (int q = 0; q < wid; ++q) {
+#pragma unroll
+                        for (int k = 0; k < KM; ++k) e[k] = w.w_top[q][k];
+                        topk_merge<KM>(pre, e, mrg);
+#pragma unroll
+                        for (int k = 0; k < KM; ++k) pre[k] = mrg[k];
+                    }
+                    fl = fl && m[i] >= sel_f<KM>(pre, K - 1);
                 }
-        }
-        if (A.state || A.node_cell) {
-            // cvtIndexToPosition (CPUThreadDevice.cpp:257-268), unsigned arithmetic
-            unsigned index = sel_u<KM>(fp, s.sel);
-            unsigned position = 0;
-            unsigned div = (unsigned)g.N;
-            for (int d = g.nd - 1; d >= 0; --d) {
-                unsigned f = (unsigned)g.fft[d], sr = (unsigned)g.src[d];
-                div /= f;
-                position = position * sr + ((f - (index / div) % f - (unsigned)s.mn[d] - 1u) + sr) % sr;
+                const int cnt = fl ? c[i] : 0;
+                int incl = cnt;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const int y = __shfl_up_sync(FULL, incl, off);
+                    if (lane >= off) incl += y;
+                }
+                if (lane == 31) w.w_sum[wid] = incl;
+                if (tid == 0) w.stop = INT_MAX;
+                __syncthreads();
+                int before = 0, all = 0;
+#pragma unroll
+                for (int q = 0; q < RP_TEAM; ++q) {
+                    const int t = w.w_sum[q];
+                    before += q < wid ? t : 0;
+                    all += t;
+                }
+                const int dst = before + incl - cnt;
+                const bool take = fl && dst + cnt <= REC_CAP;
+                if (fl && !take) atomicMin(&w.stop, tid);
+                // the segments' records, one segment of the warp after the other
+                unsigned todo = __ballot_sync(FULL, take);
+                while (todo) {
+                    const int l = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                    const int n = __shfl_sync(FULL, cnt, l), d = __shfl_sync(FULL, dst, l);
+                    const long long from = (long long)(q0 + 32 * wid + l) * QSK_SEG;
+                    for (int k = lane; k < n; k += 32) {
+                        cp_async4(&w.rv_s[d + k], rv + from + k);
+                        cp_async4(&w.ri_s[d + k], ri + from + k);
+                    }
+                }
+                cp_async_wait_all();
+                __syncthreads();
+                const int stop = w.stop;
+                int n = all;
+                if (stop != INT_MAX) {
+                    if (stop == tid) w.staged = dst;
+                    __syncthreads();
+                    n = w.staged;
+                }
+                // while fewer than K finite values have been seen the masked
+                // positions between two records are -inf ties: two draws and
+                // one cpt increment each, no visible slot change
+                int r = 0;
+                while (!emit_masked && r < n && sel_f<KM>(cv, K - 1) == -CUDART_INF_F) {
+                    const float v = w.rv_s[r];
+                    const int mm = w.ri_s[r];
+                    long long gap = mm - (last + 1);
+                    if (gap > 0) gap -= valid_prefix(g, s.lo, mm) - valid_prefix(g, s.lo, last + 1);
+                    if (gap > 0) {
+                        // the first skip covers the prepared blocks (gap >= the masked
+                        // positions before the first valid one, so 2 gap > preskip)
+                        rng_skip(w, tid, rng, 2 * gap - preskip);
+                        preskip = 0;
+                        cpt += unsigned(gap);
+                    }
+                    rng_need(w, tid, rng, 2);
+                    rng.rp += replay_trigger<KM, unsigned>(K, v, unsigned(mm), cv, cp, cpt, w.buf + rng.rp);
+                    last = mm;
+                    ++r;
+                }
+                if (r < n) team_scan<KM>(w, tid, r, n, K, cv, cp, cpt, rng);
+                if (stop == INT_MAX) break;
+                if (tid < stop) c[i] = 0;   // done; the rest of the window once more
             }
-            chosen_cell = position;
-            have = true;
+        }
+        sg += SEG_AHEAD * NT;
+    }
+    cp_async_wait_all();
+    if (wid != 0) return;
+    // merge loop (quantileSamplingModule.hpp:546-557): repeated first-max extraction
+    float fv[KM];
+    unsigned fp[KM];
+#pragma unroll
+    for (int j = 0; j < KM; ++j) {
+        fv[j] = -CUDART_INF_F;
+        fp[j] = 0xffffffffu;
+        if (j < K) {
+            int best = 0;
+            float bv = cv[0];
+#pragma unroll
+            for (int l2 = 1; l2 < KM; ++l2)
+                if (l2 < K && cv[l2] > bv) { best = l2; bv = cv[l2]; }
+            fv[j] = bv;
+            fp[j] = sel_u<KM>(cp, best);
+#pragma unroll
+            for (int l2 = 0; l2 < KM; ++l2)
+                if (l2 == best) cv[l2] = -CUDART_INF_F;
         }
     }
-    if constexpr (W > 1) {
-        // the team's work is done (every path of warp 0 reaches this point once)
-        __syncwarp();
-        if (lane == 0) w.cmd = CMD_EXIT;
-        team_bar(32 * W);
-    }
-    if (lane == 0 && have) {
-        if (A.node_cell) A.node_cell[s.node] = chosen_cell;
-        if (A.full) {
-            // -fs: the node's variable only (simulation.hpp:1016-1024)
-            const long long val = (long long)s.cell * A.nvar + s.var;
-            if (A.state && isnan(A.state[val])) A.state[val] = A.ti[(long long)chosen_cell * A.nvar + s.var];
-            if (A.id_image) A.id_image[val] = chosen_cell * A.nti + A.ti_id;
-        } else {
-            if (A.state) {
-                for (int v = 0; v < A.nvar; ++v) {
-                    float *dst = A.state + (long long)s.cell * A.nvar + v;
-                    if (isnan(*dst)) *dst = A.ti[(long long)chosen_cell * A.nvar + v];
+    // sample(): std::sort by score — insertion sort (stable) for K <= 16
+#pragma unroll
+    for (int a2 = 1; a2 < KM; ++a2) {
+        if (a2 < K) {
+#pragma unroll
+            for (int c = a2; c > 0; --c) {
+                if (fv[c] > fv[c - 1]) {
+                    float tv = fv[c]; fv[c] = fv[c - 1]; fv[c - 1] = tv;
+                    unsigned tp = fp[c]; fp[c] = fp[c - 1]; fp[c - 1] = tp;
                 }
             }
-            if (A.id_image) A.id_image[s.cell] = chosen_cell * A.nti + A.ti_id;
         }
     }
+    if (lane == 0 && A.out_val) {
+#pragma unroll
+        for (int j = 0; j < KM; ++j)
+            if (j < K) {
+                unsigned out = fp[j];
+                if (A.out_cells) {
+                    // cvtIndexToPosition (CPUThreadDevice.cpp:257-268)
+                    unsigned position = 0, div = (unsigned)g.N;
+                    for (int d = g.nd - 1; d >= 0; --d) {
+                        unsigned f = (unsigned)g.fft[d], sr = (unsigned)g.src[d];
+                        div /= f;
+                        position = position * sr + ((f - (out / div) % f - (unsigned)s.mn[d] - 1u) + sr) % sr;
+                    }
+                    out = position;
+                }
+                A.out_val[(long long)b * K + j] = fv[j];
+                A.out_pos[(long long)b * K + j] = out;
+            }
+    }
+    if (!(A.state || A.node_cell)) return;
+    // cvtIndexToPosition (CPUThreadDevice.cpp:257-268), unsigned arithmetic
+    unsigned index = sel_u<KM>(fp, s.sel);
+    unsigned position = 0;
+    unsigned div = (unsigned)g.N;
+    for (int d = g.nd - 1; d >= 0; --d) {
+        unsigned f = (unsigned)g.fft[d], sr = (unsigned)g.src[d];
+        div /= f;
+        position = position * sr + ((f - (index / div) % f - (unsigned)s.mn[d] - 1u) + sr) % sr;
+    }
+    if (lane == 0) replay_write(A, s, position);
 }
 
 // ---------------------------------------------------------------------------
@@ -2119,8 +1694,8 @@ __global__ void __launch_bounds__(W == 1 ? 32 * RP_WARPS : 32 * W) k_replay(Repl
 // tensor-core form, for the nodes it leaves to the plain map).  Every position
 // scoring at least the k-th best is a record (the filter keeps ties), so the
 // k largest (score, tie hash) over the records are the k largest over the map.
-// One CTA per slot; slots with SLOT_SKIP or SLOT_EMIT_MASKED are left to the
-// replay (only_flagged).
+// One CTA per slot; slots with SLOT_EMIT_MASKED are left to the replay
+// (only_flagged).
 // ---------------------------------------------------------------------------
 namespace {
 template <int W>
@@ -2154,7 +1729,11 @@ __global__ void __launch_bounds__(HS_THREADS) k_hash_select(ReplayArgs A) {
     const int b = blockIdx.x;
     if (b >= A.nslots) return;
     const Slot s = A.slots[b];
-    if (s.flags & (SLOT_SKIP | SLOT_EMIT_MASKED)) return;
+    if (s.flags & SLOT_SKIP) {
+        if (threadIdx.x == 0 && (A.state || A.node_cell)) replay_write(A, s, marginal_cell(A, s));
+        return;
+    }
+    if (s.flags & SLOT_EMIT_MASKED) return;
     const Geom &g = A.g;
     const int K = s.K < KM ? s.K : KM;
     const unsigned seed = __float_as_uint(s.seed) ^ (unsigned(s.node) * 0x85EBCA6Bu);
@@ -2842,10 +2421,70 @@ __device__ void write_static_slot(const SimPrepArgs &A, int b, int i, unsigned p
 // the number c0 of masked positions before the first valid one, so the
 // blocks that rng_skip regenerates without output for 2*c0 draws,
 // (2*c0 - 1) / 624 of them, are the first blocks of the real skip too.
+//
+// The blocks roll through registers: a step makes the next 224 words, seven
+// consecutive ones per lane (the recurrence reaches back 227 words at the
+// least, so a step depends on earlier steps only), from the three steps
+// before it: eleven shuffles, no shared memory and no barrier.  In shared
+// memory, three phases a block, the 600 blocks of a 128^3 image's first
+// masked plane took 265 us for 102 slots, now 391 us for one of 396.
+__device__ __forceinline__ void mt_step(unsigned (&n)[7], const unsigned (&a)[7], const unsigned (&b)[7],
+                                        const unsigned (&c)[7], int lane) {
+    // word t = 7 lane + i of the step needs words t - 3 of the last step (a),
+    // t + 48 and t + 49 of the third last (c); past the step's ends the word
+    // lies in the one before (b), supplied by the lanes at that end
+    unsigned g[7], q[3];
+    const unsigned f = __shfl_sync(0xffffffffu, lane < 6 ? b[6] : c[6], (lane + 6) & 31);
+#pragma unroll
+    for (int i = 0; i < 7; ++i) g[i] = __shfl_sync(0xffffffffu, lane < 7 ? b[i] : c[i], (lane + 7) & 31);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) q[i] = __shfl_sync(0xffffffffu, lane == 31 ? b[4 + i] : a[4 + i], (lane + 31) & 31);
+#pragma unroll
+    for (int i = 0; i < 7; ++i) n[i] = mt_mix(i == 0 ? f : g[i > 0 ? i - 1 : 0], g[i], i < 3 ? q[i < 3 ? i : 0] : a[i >= 3 ? i - 3 : 0]);
+}
+
+// `blocks` > 0 blocks further from the state mt[624] (shared memory), in place
+__device__ void mt_roll(unsigned *mt, long long blocks, int lane) {
+    unsigned r0[7], r1[7], r2[7], r3[7];
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        const int t = 7 * lane + i;
+        r0[i] = mt[400 + t];
+        r1[i] = mt[176 + t];
+        r2[i] = t >= 48 ? mt[t - 48] : 0u;   // words below 48 of this step are read by none
+        r3[i] = 0u;
+    }
+    const long long steps = (624 * blocks + 223) / 224;
+    for (long long s = 0; s + 4 <= steps; s += 4) {
+        mt_step(r3, r0, r1, r2, lane);
+        mt_step(r2, r3, r0, r1, lane);
+        mt_step(r1, r2, r3, r0, lane);
+        mt_step(r0, r1, r2, r3, lane);
+    }
+    __syncwarp();
+    // word 7 lane + i of step `step` is word k of the state
+    auto put = [&](const unsigned (&r)[7], long long step) {
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            const long long k = 224 * step + 7 * lane + i - 624 * (blocks - 1);
+            if (k >= 0 && k < 624) mt[k] = r[i];
+        }
+    };
+    const int rest = int(steps & 3);
+    if (rest > 0) mt_step(r3, r0, r1, r2, lane);
+    if (rest > 1) mt_step(r2, r3, r0, r1, lane);
+    if (rest > 2) mt_step(r1, r2, r3, r0, lane);
+    // the last four steps hold the 624 words (and at most 223 beyond them)
+    put(r0, rest == 0 ? steps - 1 : steps - 1 - rest);
+    put(r1, rest == 3 ? steps - 1 : steps - 2 - rest);
+    put(r2, rest >= 2 ? steps + 1 - rest : steps - 3 - rest);
+    put(r3, rest >= 1 ? steps - rest : steps - 4);
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(32 * RP_WARPS) k_mt_prep(SimPrepArgs A, unsigned *__restrict__ state,
                                                            int *__restrict__ pre) {
-    __shared__ unsigned mt[RP_WARPS][624 + 32];
-    __shared__ float dummy[RP_WARPS][32];
+    __shared__ __align__(16) unsigned mt[RP_WARPS][624];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x * RP_WARPS + wib;
     if (b >= A.nslots) return;
@@ -2865,9 +2504,10 @@ __global__ void __launch_bounds__(32 * RP_WARPS) k_mt_prep(SimPrepArgs A, unsign
         const long long n = 2 * (m0 - valid_prefix(g, ng.lo, m0));
         if (n > 624) blocks = int((n - 1) / 624);
     }
-    for (int t = 0; t < blocks; ++t) mt_twist<false>(mt[wib], lane, nullptr, dummy[wib]);
-    __syncwarp();
-    for (int i = lane; i < 624; i += 32) state[(long long)b * 624 + i] = mt[wib][i];
+    if (blocks > 0) mt_roll(mt[wib], blocks, lane);
+    // a state row is 624 words, a multiple of 16 bytes
+    uint4 *row = reinterpret_cast<uint4 *>(state + (long long)b * 624);
+    for (int i = lane; i < 156; i += 32) row[i] = *reinterpret_cast<const uint4 *>(&mt[wib][4 * i]);
     if (lane == 0) pre[b] = 624 * blocks;
 }
 
@@ -3162,16 +2802,6 @@ cudaError_t launch_mt_prep(const SimPrepArgs &a, unsigned *state, int *pre, cuda
     return cudaGetLastError();
 }
 
-template <int T>
-static void launch_replay_team(const ReplayArgs &a, size_t smem, cudaStream_t st) {
-    const unsigned blocks = (unsigned)a.nslots;
-    if (a.K <= 1) k_replay<1, T><<<blocks, 32 * T, smem, st>>>(a);
-    else if (a.K <= 2) k_replay<2, T><<<blocks, 32 * T, smem, st>>>(a);
-    else if (a.K <= 4) k_replay<4, T><<<blocks, 32 * T, smem, st>>>(a);
-    else if (a.K <= 8) k_replay<8, T><<<blocks, 32 * T, smem, st>>>(a);
-    else k_replay<16, T><<<blocks, 32 * T, smem, st>>>(a);
-}
-
 cudaError_t launch_hash_select(const ReplayArgs &a, cudaStream_t st) {
     if (a.nslots <= 0) return cudaSuccess;
     if (a.K <= 2) k_hash_select<2><<<(unsigned)a.nslots, HS_THREADS, 0, st>>>(a);
@@ -3182,37 +2812,13 @@ cudaError_t launch_hash_select(const ReplayArgs &a, cudaStream_t st) {
 }
 
 cudaError_t launch_replay(const ReplayArgs &a, cudaStream_t st) {
-    // One CTA per slot: a team of warps (warp 0 replays, the others help
-    // with the generator blocks and the tie super-runs) around one shared
-    // state of ~25 KB.  Teams of eight while every slot of the batch gets an
-    // SM slot at once (registers allow 4 such CTAs per SM); larger batches
-    // take teams of four, 8 CTAs per SM, so that they still run in one wave
-    // up to 1184 slots.  A warp per slot with a state of its own (8 warps per
-    // SM) measured slower at every batch size of the simulations.
-    static std::atomic<int> wave8[64][5];   // per device and K class; 0 until measured (jobs may run in threads)
-    const size_t smem = sizeof(WarpShared);
     if (a.nslots <= 0) return cudaSuccess;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    const int kc = a.K <= 1 ? 0 : a.K <= 2 ? 1 : a.K <= 4 ? 2 : a.K <= 8 ? 3 : 4;
-    int wave = wave8[dev][kc].load(std::memory_order_relaxed);
-    if (wave == 0) {
-        int sms = 0, per_sm = 0;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        const void *fn = kc == 0   ? (const void *)k_replay<1, TEAM_MAX>
-                         : kc == 1 ? (const void *)k_replay<2, TEAM_MAX>
-                         : kc == 2 ? (const void *)k_replay<4, TEAM_MAX>
-                         : kc == 3 ? (const void *)k_replay<8, TEAM_MAX>
-                                   : (const void *)k_replay<16, TEAM_MAX>;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * TEAM_MAX, smem)) != cudaSuccess)
-            return e;
-        wave = sms * (per_sm > 0 ? per_sm : 1);
-        wave8[dev][kc].store(wave, std::memory_order_relaxed);
-    }
-    if (a.nslots <= wave) launch_replay_team<TEAM_MAX>(a, smem, st);
-    else launch_replay_team<TEAM_MAX / 2>(a, smem, st);
+    const unsigned blocks = (unsigned)a.nslots;
+    if (a.K <= 1) k_replay<1><<<blocks, RP_THREADS, 0, st>>>(a);
+    else if (a.K <= 2) k_replay<2><<<blocks, RP_THREADS, 0, st>>>(a);
+    else if (a.K <= 4) k_replay<4><<<blocks, RP_THREADS, 0, st>>>(a);
+    else if (a.K <= 8) k_replay<8><<<blocks, RP_THREADS, 0, st>>>(a);
+    else k_replay<16><<<blocks, RP_THREADS, 0, st>>>(a);
     return cudaGetLastError();
 }
 

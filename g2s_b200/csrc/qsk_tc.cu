@@ -845,17 +845,37 @@ __global__ void k_tc_tile_scale(long long tiles, const float *__restrict__ rowma
     scale[t] = pow2_scale(mx);
 }
 
-// largest template index among a node's neighbours; -1 for nodes without a
-// neighbour other than the centre (marginal draw: the plain path)
+// one warp per node: the largest template index among its neighbours, -1 for
+// nodes without a neighbour other than the centre (marginal draw: the plain
+// path); QSK_TMAX_FEW is added where fewer than K positions hold the whole
+// pattern
 __global__ void k_tc_tmax(long long nodes, int n, const int *__restrict__ nb_count, const int *__restrict__ nb_tpl,
-                          int *__restrict__ tmax) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+                          const int *__restrict__ tpl, Geom g, int K, int *__restrict__ tmax) {
+    const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = int(threadIdx.x & 31);
     if (i >= nodes) return;
     const int c = nb_count[i];
     int m = -1;
-    if (c >= 2)
-        for (int j = 0; j < c; ++j) m = max(m, nb_tpl[i * n + j]);
-    tmax[i] = m;
+    int mn[QSK_MAXD] = {0, 0, 0, 0}, mx[QSK_MAXD] = {0, 0, 0, 0};
+    for (int j = lane; j < c; j += 32) {
+        const int t = nb_tpl[i * n + j];
+        m = max(m, t);
+        for (int d = 0; d < g.nd; ++d) {
+            const int o = tpl[t * g.nd + d];
+            mn[d] = min(mn[d], o);
+            mx[d] = max(mx[d], o);
+        }
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    long long nvalid = 1;
+#pragma unroll
+    for (int d = 0; d < QSK_MAXD; ++d) {
+        if (d >= g.nd) break;
+        const int w = g.src[d] - (__reduce_max_sync(0xffffffffu, mx[d]) - __reduce_min_sync(0xffffffffu, mn[d]));
+        nvalid *= w < 0 ? 0 : (w > g.fft[d] ? g.fft[d] : w);
+    }
+    if (c < 2) m = -1;
+    if (lane == 0) tmax[i] = m + (nvalid < K ? QSK_TMAX_FEW : 0);
 }
 
 // one warp per tensor slot: the node's row of A (coefficients of its terms at
@@ -1294,9 +1314,10 @@ cudaError_t launch_tc_pattern(const TcPatternArgs &a, float *rowmax, cudaStream_
     return cudaGetLastError();
 }
 
-cudaError_t launch_tc_tmax(long long nodes, int n, const int *nb_count, const int *nb_tpl, int *tmax, cudaStream_t st) {
+cudaError_t launch_tc_tmax(long long nodes, int n, const int *nb_count, const int *nb_tpl, const int *tpl, const Geom &g,
+                           int K, int *tmax, cudaStream_t st) {
     if (nodes <= 0) return cudaSuccess;
-    k_tc_tmax<<<(unsigned)((nodes + 255) / 256), 256, 0, st>>>(nodes, n, nb_count, nb_tpl, tmax);
+    k_tc_tmax<<<(unsigned)((nodes * 32 + 255) / 256), 256, 0, st>>>(nodes, n, nb_count, nb_tpl, tpl, g, K, tmax);
     return cudaGetLastError();
 }
 
