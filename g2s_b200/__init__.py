@@ -13,7 +13,9 @@ the index image like the reference does.
 from __future__ import annotations
 
 import ctypes
+import itertools
 import os
+import struct
 from typing import Optional, Sequence
 
 import numpy as np
@@ -195,6 +197,21 @@ def _p(a, t):
     return None if a is None else a.ctypes.data_as(t)
 
 
+_pack_term = struct.Struct("=iiiff").pack
+
+
+def _terms(terms):
+    """QskTerm array of rows (neighbour, layer, op, a, b)."""
+    n = len(terms)
+    try:
+        raw = b"".join(itertools.starmap(_pack_term, terms))
+    except (struct.error, TypeError, OverflowError):
+        # rows of other number types, or longer ones
+        return (QskTerm * max(n, 1))(*[QskTerm(int(t[0]), int(t[1]), int(t[2]), float(t[3]), float(t[4]))
+                                       for t in terms])
+    return (QskTerm * max(n, 1)).from_buffer_copy(raw or bytes(ctypes.sizeof(QskTerm)))
+
+
 def device_count() -> int:
     c = ctypes.c_int(0)
     rc = lib().qsk_device_count(ctypes.byref(c))
@@ -310,8 +327,7 @@ class Worker:
         ``exclude_radius`` >= 1 every index the reference's radius exclusion
         marks around it.  Returns (scores[k], scan_indices[k], min_offset[ndim])."""
         offs = np.ascontiguousarray(offsets, dtype=np.int32).reshape(-1, self.ti.ndim)
-        tarr = (QskTerm * max(len(terms), 1))(*[QskTerm(int(t[0]), int(t[1]), int(t[2]), float(t[3]), float(t[4]))
-                                               for t in terms])
+        tarr = _terms(terms)
         sc = np.zeros(k, np.float32)
         ix = np.zeros(k, np.uint32)
         mn = np.zeros(self.ti.ndim, np.int32)
@@ -343,8 +359,7 @@ class Worker:
             tl.extend(terms)
             term_ptr[b + 1] = term_ptr[b] + len(terms)
         offs = np.ascontiguousarray(np.concatenate(offs) if offs else np.zeros((0, nd), np.int32), np.int32)
-        tarr = (QskTerm * max(len(tl), 1))(*[QskTerm(int(t[0]), int(t[1]), int(t[2]), float(t[3]), float(t[4]))
-                                            for t in tl])
+        tarr = _terms(tl)
         sd = np.ascontiguousarray(seeds, np.float32)
         org = np.ascontiguousarray(origins, np.uint32)
         rad = None if radii is None else np.ascontiguousarray(radii, np.float32)
