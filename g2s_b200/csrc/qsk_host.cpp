@@ -232,19 +232,22 @@ int g_map_mode = 0;   // 0: automatic, 1: always the FP32 gather kernel
 struct qsk_worker {
     qsk_ti *ti = nullptr;
     cudaStream_t st = nullptr;
-    DBuf<Slot> slots;
-    DBuf<Term> terms;
+    // a call's slots, terms and exclusion centres, built in pinned memory and
+    // sent in one copy; its results, which the replay writes to pinned memory
+    // that the device sees at the same address
+    unsigned char *h_in = nullptr, *h_out = nullptr;
+    size_t h_in_cap = 0, h_out_cap = 0;
+    DBuf<unsigned char> d_in;
     DBuf<float> rec_val;
     DBuf<int> rec_idx;
     DBuf<int> rec_cnt;
     DBuf<float> rec_max;
-    DBuf<float> out_val;
-    DBuf<unsigned> out_pos;
-    DBuf<int> xcenter;        // verbatim exclusion with a radius: scan index per pattern
-    DBuf<float> xradius;
+    DBuf<unsigned> gen;       // generator states [pattern][624], then the draws they skip
     DBuf<unsigned> xmask;     // [pattern][ceil(N/32)] excluded positions
-    std::vector<Slot> h_slots;
-    std::vector<Term> h_terms;
+    ~qsk_worker() {
+        if (h_in) cudaFreeHost(h_in);
+        if (h_out) cudaFreeHost(h_out);
+    }
 };
 
 namespace {
@@ -265,7 +268,7 @@ cudaError_t ensure_records(const Geom &g, int nslots, DBuf<float> &rv, DBuf<int>
 
 // host-side slot/terms for one explicit pattern
 int build_pattern_slot(const qsk_ti *ti, int nnb, const int *offsets, int nterms, const qsk_term *terms, unsigned K,
-                       float seed, int node, Slot &s, std::vector<Term> &out, int *out_min,
+                       float seed, int node, Slot &s, Term *out, int *out_min,
                        const qsk_pattern_opts *opts = nullptr) {
     const Geom &g = ti->g;
     const int nd = g.nd;
@@ -312,7 +315,6 @@ int build_pattern_slot(const qsk_ti *ti, int nnb, const int *offsets, int nterms
             s.cmask_base = int((long long)opts->centre_mask_layer * g.N + fmn);
         }
     }
-    out.clear();
     for (int t = 0; t < nterms; ++t) {
         const qsk_term &q = terms[t];
         if (q.neighbour < 0 || q.neighbour >= nnb || q.layer < 0 || q.layer >= ti->nlayers || q.op < 0 || q.op > 3)
@@ -324,9 +326,22 @@ int build_pattern_slot(const qsk_ti *ti, int nnb, const int *offsets, int nterms
         tm.a = q.a;
         tm.b = q.b;
         tm.op = q.op == QSK_OP_LIN_CROSS ? OP_LINX : q.op;
-        out.push_back(tm);
+        out[t] = tm;
     }
-    s.nterms = int(out.size());
+    s.nterms = nterms;
+    return QSK_OK;
+}
+
+// pinned host memory of at least `bytes`, visible to the device
+int pinned_ensure(unsigned char *&p, size_t &cap, size_t bytes) {
+    if (bytes <= cap) return QSK_OK;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    cap = 0;
+    void *q = nullptr;
+    CK(cudaHostAlloc(&q, bytes, cudaHostAllocMapped));
+    p = static_cast<unsigned char *>(q);
+    cap = bytes;
     return QSK_OK;
 }
 
@@ -552,18 +567,28 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
     DeviceGuard dgd(ti->device);
     const Geom &g = ti->g;
     const int nd = g.nd;
-    w->h_slots.resize(B);
     int maxterms = 1;
     for (int b = 0; b < B; ++b) maxterms = std::max(maxterms, term_ptr[b + 1] - term_ptr[b]);
-    w->h_terms.assign(size_t(B) * maxterms, Term{0, 0.f, 0.f, 0});
-    std::vector<Term> tmp;
+    if ((size_t)maxterms * sizeof(Term) > 200 * 1024) return fail(QSK_ERR_UNSUPPORTED, "too many terms (%d)", maxterms);
+    // one block: terms, slots, exclusion centres and radii (16-byte aligned parts)
+    const size_t at_slots = sizeof(Term) * size_t(B) * maxterms;
+    const size_t at_xc = (at_slots + sizeof(Slot) * size_t(B) + 15) / 16 * 16;
+    const size_t at_xr = (at_xc + sizeof(int) * size_t(B) + 15) / 16 * 16;
+    const size_t in_bytes = at_xr + sizeof(float) * size_t(B);
+    // grown by halves: the number of terms differs from call to call
+    if (in_bytes > w->h_in_cap)
+        if (int rc = pinned_ensure(w->h_in, w->h_in_cap, std::max<size_t>(in_bytes + in_bytes / 2, 16384))) return rc;
+    Term *h_terms = reinterpret_cast<Term *>(w->h_in);
+    Slot *h_slots = reinterpret_cast<Slot *>(w->h_in + at_slots);
+    bool all_match = true;   // unit-weight matches only
     for (int b = 0; b < B; ++b) {
         int nnb = nb_ptr[b + 1] - nb_ptr[b];
         int nt = term_ptr[b + 1] - term_ptr[b];
+        Term *tb = h_terms + size_t(b) * maxterms;
         int rc = build_pattern_slot(ti, nnb, offsets + size_t(nb_ptr[b]) * nd, nt, terms + term_ptr[b], k, seeds[b], b,
-                                    w->h_slots[b], tmp, out_min ? out_min + size_t(b) * nd : nullptr, opts);
+                                    h_slots[b], tb, out_min ? out_min + size_t(b) * nd : nullptr, opts);
         if (rc) return rc;
-        std::copy(tmp.begin(), tmp.end(), w->h_terms.begin() + size_t(b) * maxterms);
+        for (int t = 0; t < h_slots[b].nterms; ++t) all_match &= tb[t].op == OP_EQ && tb[t].a == 1.f;
     }
     // verbatim exclusion of each pattern's origin (the TI cell the pattern was
     // taken from): one scan index, or every index within the radius
@@ -574,7 +599,7 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
         xc.assign(B, -1);
         xr.assign(B, 0.f);
         for (int b = 0; b < B; ++b) {
-            if (w->h_slots[b].flags & SLOT_SKIP) continue;
+            if (h_slots[b].flags & SLOT_SKIP) continue;
             xc[b] = opts->exclude_index;
             xr[b] = opts->exclude_radius;
             any_radius = true;
@@ -583,7 +608,7 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
         xc.assign(B, -1);
         xr.assign(B, 0.f);
         for (int b = 0; b < B; ++b) {
-            Slot &sl = w->h_slots[b];
+            Slot &sl = h_slots[b];
             if (origin[b] == 0xffffffffu || (sl.flags & SLOT_SKIP)) continue;
             if ((long long)origin[b] >= ti->cells) return fail(QSK_ERR_ARG, "origin %u of pattern %d outside the TI", origin[b], b);
             const unsigned idx = qsk_position_to_index(ti, sl.mn, origin[b]);
@@ -601,20 +626,27 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
         CK(set_map_smem_limit(200 * 1024));
         smem_configured_device = ti->device;
     }
-    if ((size_t)maxterms * sizeof(Term) > 200 * 1024) return fail(QSK_ERR_UNSUPPORTED, "too many terms (%d)", maxterms);
-    CK(w->slots.upload(w->h_slots.data(), B, w->st));
-    CK(w->terms.upload(w->h_terms.data(), w->h_terms.size(), w->st));
+    if (any_radius) {
+        std::memcpy(w->h_in + at_xc, xc.data(), sizeof(int) * size_t(B));
+        std::memcpy(w->h_in + at_xr, xr.data(), sizeof(float) * size_t(B));
+    }
+    const size_t out_bytes = (sizeof(float) + sizeof(unsigned)) * size_t(B) * k;
+    if (out_bytes > w->h_out_cap)
+        if (int rc = pinned_ensure(w->h_out, w->h_out_cap, std::max<size_t>(out_bytes, 4096))) return rc;
+    float *const res_val = reinterpret_cast<float *>(w->h_out);
+    unsigned *const res_pos = reinterpret_cast<unsigned *>(w->h_out) + size_t(B) * k;
+    if (in_bytes > w->d_in.n) CK(w->d_in.alloc(w->h_in_cap));
+    CK(cudaMemcpyAsync(w->d_in.p, w->h_in, any_radius ? in_bytes : at_xc, cudaMemcpyHostToDevice, w->st));
+    const Term *const d_terms = reinterpret_cast<const Term *>(w->d_in.p);
+    const Slot *const d_slots = reinterpret_cast<const Slot *>(w->d_in.p + at_slots);
     CK(ensure_records(g, B, w->rec_val, w->rec_idx, w->rec_cnt, w->rec_max));
-    CK(w->out_val.ensure(size_t(B) * k));
-    CK(w->out_pos.ensure(size_t(B) * k));
+    CK(w->gen.ensure(size_t(B) * 625));
+    GenArgs gen;
+    gen.state = w->gen.p;
+    gen.pre = reinterpret_cast<int *>(w->gen.p + size_t(B) * 624);
     // the radius masks are applied by the FP32 kernel (the bit-sliced one gives
     // the same scores, so the choice changes no result)
-    bool bits = ti->planes_ok && g_map_mode == 0 && maxterms <= 255 && !opts && !any_radius;
-    for (size_t i = 0; i < w->h_terms.size() && bits; ++i) {
-        int b = int(i / maxterms), t = int(i % maxterms);
-        if (t >= w->h_slots[b].nterms) continue;
-        bits &= (w->h_terms[i].op == OP_EQ && w->h_terms[i].a == 1.f);
-    }
+    const bool bits = ti->planes_ok && g_map_mode == 0 && maxterms <= 255 && !opts && !any_radius && all_match;
     if (bits) {
         BitArgs ba;
         ba.g = g;
@@ -622,8 +654,9 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
         ba.pw = ti->pw;
         ba.ncat = ti->ncat.p;
         ba.catv = ti->catv.p;
-        ba.slots = w->slots.p;
-        ba.terms = w->terms.p;
+        ba.slots = d_slots;
+        ba.terms = d_terms;
+        ba.gen = gen;
         ba.maxterms = maxterms;
         ba.segs_per_cta = map_bits_segs_per_cta(g, B);
         ba.rec_val = w->rec_val.p;
@@ -636,8 +669,9 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
         ma.g = g;
         ma.layers = ti->layers.p;
         ma.layer_elems = (long long)ti->nlayers * ti->g.N;
-        ma.slots = w->slots.p;
-        ma.terms = w->terms.p;
+        ma.slots = d_slots;
+        ma.terms = d_terms;
+        ma.gen = gen;
         ma.maxterms = maxterms;
         ma.segs_per_cta = map_segs_per_cta(g, B);
         ma.rec_val = w->rec_val.p;
@@ -646,10 +680,9 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
         ma.rec_max = w->rec_max.p;
         if (any_radius) {
             const long long xwords = (g.N + 31) / 32;
-            CK(w->xcenter.upload(xc.data(), size_t(B), w->st));
-            CK(w->xradius.upload(xr.data(), size_t(B), w->st));
             CK(w->xmask.ensure(size_t(B) * size_t(xwords)));
-            CK(launch_radius_mask(w->xcenter.p, w->xradius.p, B, g, w->xmask.p, xwords, w->st));
+            CK(launch_radius_mask(reinterpret_cast<const int *>(w->d_in.p + at_xc),
+                                  reinterpret_cast<const float *>(w->d_in.p + at_xr), B, g, w->xmask.p, xwords, w->st));
             ma.xmask = w->xmask.p;
             ma.xwords = xwords;
         }
@@ -658,22 +691,24 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
     ReplayArgs ra;
     std::memset(&ra, 0, sizeof(ra));
     ra.g = g;
-    ra.slots = w->slots.p;
+    ra.slots = d_slots;
     ra.nslots = B;
     ra.K = int(k);
     ra.rec_val = w->rec_val.p;
     ra.rec_idx = w->rec_idx.p;
     ra.rec_cnt = w->rec_cnt.p;
     ra.rec_max = w->rec_max.p;
-    ra.out_val = w->out_val.p;
-    ra.out_pos = w->out_pos.p;
+    ra.out_val = res_val;
+    ra.out_pos = res_pos;
+    ra.mt_state = gen.state;
+    ra.mt_pre = gen.pre;
     CK(launch_replay(ra, w->st));
-    CK(cudaMemcpyAsync(out_score, w->out_val.p, sizeof(float) * B * k, cudaMemcpyDeviceToHost, w->st));
-    CK(cudaMemcpyAsync(out_index, w->out_pos.p, sizeof(unsigned) * B * k, cudaMemcpyDeviceToHost, w->st));
     CK(cudaStreamSynchronize(w->st));
+    std::memcpy(out_score, res_val, sizeof(float) * size_t(B) * k);
+    std::memcpy(out_index, res_pos, sizeof(unsigned) * size_t(B) * k);
     // empty patterns keep -inf scores (candidateForPattern returned false)
     for (int b = 0; b < B; ++b)
-        if (w->h_slots[b].flags & SLOT_SKIP)
+        if (h_slots[b].flags & SLOT_SKIP)
             for (unsigned j = 0; j < k; ++j) {
                 out_score[size_t(b) * k + j] = -INFINITY;
                 out_index[size_t(b) * k + j] = 0xffffffffu;

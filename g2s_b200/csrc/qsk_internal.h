@@ -147,6 +147,14 @@ inline FastDiv make_fast_div(unsigned d) {
     return {unsigned(((1ull << (31 + l)) + d - 1) / d), l - 1};
 }
 
+// Generator states of explicit patterns (state rows and skipped draws as
+// k_mt_prep writes them): one more CTA per slot of a map launch makes them
+// while the others run the map; null: none
+struct GenArgs {
+    unsigned *state = nullptr;   // [slot][624]
+    int *pre = nullptr;
+};
+
 struct MapArgs {
     Geom g;
     const float *layers;
@@ -164,6 +172,7 @@ struct MapArgs {
     const unsigned *xmask = nullptr;
     long long xwords = 0;
     FastDiv div[QSK_MAXD];    // by g.fft (set by the launcher)
+    GenArgs gen;              // pattern queries: generator states made beside the map
 };
 
 // Bit-plane layout: every plane is `plane_words(N)` words, of which the
@@ -196,6 +205,7 @@ struct BitArgs {
     const int *tpl = nullptr;           // template offsets (ntpl x nd)
     int no_verbatim = 0;
     int stage_words = 0;                // shared-memory words for staged planes (set by the launcher)
+    GenArgs gen;
 };
 
 struct ReplayArgs {

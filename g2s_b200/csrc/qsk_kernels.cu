@@ -645,6 +645,141 @@ __global__ void k_prep_tc_nodes(SimPrepArgs P, TcNodeArgs T, unsigned prep_block
 }
 
 // ---------------------------------------------------------------------------
+// mt19937 (published algorithm: Matsumoto & Nishimura 1998) with the
+// conversion of std::uniform_real_distribution<float>(0,1) in libstdc++
+// (generate_canonical<float,24>: float(u32) * 2^-32, values >= 1 clamped to
+// the largest float below 1).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned mt_temper(unsigned y) {
+    y ^= y >> 11;
+    y ^= (y << 7) & 0x9d2c5680u;
+    y ^= (y << 15) & 0xefc60000u;
+    y ^= y >> 18;
+    return y;
+}
+
+__device__ __forceinline__ float mt_unit(unsigned y) {
+    float u = __fmul_rn(__uint2float_rn(y), 2.3283064365386963e-10f);
+    return u >= 1.f ? 0x1.fffffep-1f : u;
+}
+
+__device__ __forceinline__ unsigned mt_mix(unsigned a, unsigned b, unsigned c) {
+    unsigned y = (a & 0x80000000u) | (b & 0x7fffffffu);
+    return c ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+}
+
+
+// generator.seed(seedFromUnitFloat(seed) + 0)  (quantileSamplingModule.hpp:45-49,533-534):
+// the standard mt19937 initialisation, serial, on the calling thread
+__device__ __forceinline__ void mt_seed(unsigned *mt, float sd) {
+    unsigned x;
+    if (!isfinite(sd) || sd <= 0.f) x = 0u;
+    else if (sd >= 1.f) x = 0xffffffffu;
+    else x = (unsigned)floor((double)sd * 4294967295.0);
+    mt[0] = x;
+    for (int i = 1; i < 624; ++i) {
+        x = 1812433253u * (x ^ (x >> 30)) + (unsigned)i;
+        mt[i] = x;
+    }
+}
+
+// The blocks roll through registers: a step makes the next 224 words, seven
+// consecutive ones per lane (the recurrence reaches back 227 words at the
+// least, so a step depends on earlier steps only), from the three steps
+// before it: eleven shuffles, no shared memory and no barrier.  In shared
+// memory, three phases a block, the 600 blocks of a 128^3 image's first
+// masked plane took 265 us for 102 slots, now 391 us for one of 396.
+__device__ __forceinline__ void mt_step(unsigned (&n)[7], const unsigned (&a)[7], const unsigned (&b)[7],
+                                        const unsigned (&c)[7], int lane) {
+    // word t = 7 lane + i of the step needs words t - 3 of the last step (a),
+    // t + 48 and t + 49 of the third last (c); past the step's ends the word
+    // lies in the one before (b), supplied by the lanes at that end
+    unsigned g[7], q[3];
+    const unsigned f = __shfl_sync(0xffffffffu, lane < 6 ? b[6] : c[6], (lane + 6) & 31);
+#pragma unroll
+    for (int i = 0; i < 7; ++i) g[i] = __shfl_sync(0xffffffffu, lane < 7 ? b[i] : c[i], (lane + 7) & 31);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) q[i] = __shfl_sync(0xffffffffu, lane == 31 ? b[4 + i] : a[4 + i], (lane + 31) & 31);
+#pragma unroll
+    for (int i = 0; i < 7; ++i) n[i] = mt_mix(i == 0 ? f : g[i > 0 ? i - 1 : 0], g[i], i < 3 ? q[i < 3 ? i : 0] : a[i >= 3 ? i - 3 : 0]);
+}
+
+// `blocks` > 0 blocks further from the state mt[624] (shared memory), in place
+__device__ void mt_roll(unsigned *mt, long long blocks, int lane) {
+    unsigned r0[7], r1[7], r2[7], r3[7];
+#pragma unroll
+    for (int i = 0; i < 7; ++i) {
+        const int t = 7 * lane + i;
+        r0[i] = mt[400 + t];
+        r1[i] = mt[176 + t];
+        r2[i] = t >= 48 ? mt[t - 48] : 0u;   // words below 48 of this step are read by none
+        r3[i] = 0u;
+    }
+    const long long steps = (624 * blocks + 223) / 224;
+    for (long long s = 0; s + 4 <= steps; s += 4) {
+        mt_step(r3, r0, r1, r2, lane);
+        mt_step(r2, r3, r0, r1, lane);
+        mt_step(r1, r2, r3, r0, lane);
+        mt_step(r0, r1, r2, r3, lane);
+    }
+    __syncwarp();
+    // word 7 lane + i of step `step` is word k of the state
+    auto put = [&](const unsigned (&r)[7], long long step) {
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+            const long long k = 224 * step + 7 * lane + i - 624 * (blocks - 1);
+            if (k >= 0 && k < 624) mt[k] = r[i];
+        }
+    };
+    const int rest = int(steps & 3);
+    if (rest > 0) mt_step(r3, r0, r1, r2, lane);
+    if (rest > 1) mt_step(r2, r3, r0, r1, lane);
+    if (rest > 2) mt_step(r1, r2, r3, r0, lane);
+    // the last four steps hold the 624 words (and at most 223 beyond them)
+    put(r0, rest == 0 ? steps - 1 : steps - 1 - rest);
+    put(r1, rest == 3 ? steps - 1 : steps - 2 - rest);
+    put(r2, rest >= 2 ? steps + 1 - rest : steps - 3 - rest);
+    put(r3, rest >= 1 ? steps - rest : steps - 4);
+    __syncwarp();
+}
+
+// blocks that the first skip of a slot's replay regenerates without output:
+// see k_mt_prep
+__device__ long long skipped_blocks(const Geom &g, const int *lo, long long nvalid, int K) {
+    if (nvalid < K || nvalid <= 0) return 0;
+    long long m0 = 0;
+    for (int d = 0; d < g.nd; ++d) m0 += (long long)lo[d] * g.sstride[d];
+    const long long n = 2 * (m0 - valid_prefix(g, lo, m0));
+    return n > 624 ? (n - 1) / 624 : 0;
+}
+
+// the state mt[624] (shared memory) and its skipped draws to row b, one warp
+__device__ void store_generator(const unsigned *mt, long long blocks, int b, unsigned *state, int *pre, int lane) {
+    // a state row is 624 words, a multiple of 16 bytes
+    uint4 *row = reinterpret_cast<uint4 *>(state + (long long)b * 624);
+    for (int i = lane; i < 156; i += 32) row[i] = *reinterpret_cast<const uint4 *>(&mt[4 * i]);
+    if (lane == 0) pre[b] = int(624 * blocks);
+}
+
+// GenArgs: slot b's generator state by the first warp of a CTA
+__device__ void slot_generator(const Geom &g, const Slot &sl, int b, const GenArgs &gen, unsigned *mt) {
+    if (threadIdx.x >= 32 || (sl.flags & SLOT_SKIP)) return;
+    const int lane = threadIdx.x;
+    if (lane == 0) mt_seed(mt, sl.seed);
+    __syncwarp();
+    long long blocks = 0;
+    if (!(sl.flags & (SLOT_EMIT_MASKED | SLOT_MISSING))) {
+        long long nvalid = 1;
+        int lo[QSK_MAXD];
+        for (int d = 0; d < QSK_MAXD; ++d) lo[d] = sl.lo[d];
+        for (int d = 0; d < g.nd; ++d) nvalid *= g.fft[d] - lo[d];
+        blocks = skipped_blocks(g, lo, nvalid, sl.K);
+    }
+    if (blocks > 0) mt_roll(mt, blocks, lane);
+    store_generator(mt, blocks, b, gen.state, gen.pre, lane);
+}
+
+// ---------------------------------------------------------------------------
 // fused map + record filter
 //
 // A warp takes MR_SEGS consecutive 128-position segments at once, eight
@@ -780,14 +915,19 @@ __device__ void map_terms_any(const Term *__restrict__ sterm, int nt, const floa
 }
 }  // namespace
 
-template <int KF>
+template <int KF, bool GEN>
 __global__ void __launch_bounds__(256, KF <= 4 ? 4 : 2) k_map_records(MapArgs A) {
-    extern __shared__ Term sterm[];
+    extern __shared__ __align__(16) Term sterm[];
     __shared__ Slot ss;
     // smallest and largest layer offset of the terms; bit 0: a term that is not
     // OP_SQLIN, bit 1: one that the fast loop does not know
     __shared__ int s_lo, s_hi, s_ops;
     const int b = blockIdx.y;
+    if (GEN && blockIdx.x == 0) {
+        slot_generator(A.g, A.slots[b], b, A.gen, reinterpret_cast<unsigned *>(sterm));
+        return;
+    }
+    const int part = int(blockIdx.x) - (GEN ? 1 : 0);
     const Term *src = A.terms + (long long)b * A.maxterms;
     // a thread's first term is read beside the slot (the slot's block of terms
     // is maxterms long; what lies beyond its own terms is not used)
@@ -836,7 +976,7 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 4 : 2) k_map_records(MapArgs A)
     }
     const unsigned uN = (unsigned)g.N;
 
-    const int seg_begin = blockIdx.x * A.segs_per_cta;
+    const int seg_begin = part * A.segs_per_cta;
     const int seg_end = min(seg_begin + A.segs_per_cta, g.nseg);
     float *rv = A.rec_val + (long long)b * g.nseg * QSK_SEG;
     int *ri = A.rec_idx + (long long)b * g.nseg * QSK_SEG;
@@ -1003,45 +1143,6 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 4 : 2) k_map_records(MapArgs A)
                 A.rec_max[(long long)b * g.nseg + sg] = segmax;
             }
         }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// mt19937 (published algorithm: Matsumoto & Nishimura 1998) with the
-// conversion of std::uniform_real_distribution<float>(0,1) in libstdc++
-// (generate_canonical<float,24>: float(u32) * 2^-32, values >= 1 clamped to
-// the largest float below 1).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned mt_temper(unsigned y) {
-    y ^= y >> 11;
-    y ^= (y << 7) & 0x9d2c5680u;
-    y ^= (y << 15) & 0xefc60000u;
-    y ^= y >> 18;
-    return y;
-}
-
-__device__ __forceinline__ float mt_unit(unsigned y) {
-    float u = __fmul_rn(__uint2float_rn(y), 2.3283064365386963e-10f);
-    return u >= 1.f ? 0x1.fffffep-1f : u;
-}
-
-__device__ __forceinline__ unsigned mt_mix(unsigned a, unsigned b, unsigned c) {
-    unsigned y = (a & 0x80000000u) | (b & 0x7fffffffu);
-    return c ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
-}
-
-
-// generator.seed(seedFromUnitFloat(seed) + 0)  (quantileSamplingModule.hpp:45-49,533-534):
-// the standard mt19937 initialisation, serial, on the calling thread
-__device__ __forceinline__ void mt_seed(unsigned *mt, float sd) {
-    unsigned x;
-    if (!isfinite(sd) || sd <= 0.f) x = 0u;
-    else if (sd >= 1.f) x = 0xffffffffu;
-    else x = (unsigned)floor((double)sd * 4294967295.0);
-    mt[0] = x;
-    for (int i = 1; i < 624; ++i) {
-        x = 1812433253u * (x ^ (x >> 30)) + (unsigned)i;
-        mt[i] = x;
     }
 }
 
@@ -1873,15 +1974,21 @@ __device__ __forceinline__ unsigned bits_range(int a, int b) {
 
 // K <= 4: at most 42 registers, 48 warps per SM (measured faster than 48
 // registers and 40 warps); the wider top-K states would spill under that cap
-template <int KF>
+// GEN: the first CTA of a slot makes its generator state (GenArgs)
+template <int KF, bool GEN>
 __global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
-    extern __shared__ int2 bterm[];
+    extern __shared__ __align__(16) int2 bterm[];
     __shared__ Slot ss;
     __shared__ int nbt, s_multi, s_total;
     // staged plane windows of a single-variable slot, per category: lowest and
     // highest word offset of its terms, and where its window starts
     __shared__ int s_lo[QSK_CMAX], s_hi[QSK_CMAX], s_base[QSK_CMAX];
     const int b = blockIdx.y;
+    if (GEN && blockIdx.x == 0) {   // (the staged planes leave room for a state)
+        slot_generator(A.g, A.slots[b], b, A.gen, reinterpret_cast<unsigned *>(bterm));
+        return;
+    }
+    const int part = int(blockIdx.x) - (GEN ? 1 : 0);
     if (threadIdx.x == 0) {
         ss = A.slots[b];
         nbt = 0;
@@ -1894,7 +2001,7 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
     __syncthreads();
     if (ss.flags & SLOT_SKIP) return;
     const Geom &g = A.g;
-    const int seg_begin = blockIdx.x * A.segs_per_cta;
+    const int seg_begin = part * A.segs_per_cta;
     const int nseg1k = (int)((g.N + 1023) / 1024);
     int seg_end = seg_begin + A.segs_per_cta;
     if (seg_end > nseg1k) seg_end = nseg1k;
@@ -2421,67 +2528,6 @@ __device__ void write_static_slot(const SimPrepArgs &A, int b, int i, unsigned p
 // the number c0 of masked positions before the first valid one, so the
 // blocks that rng_skip regenerates without output for 2*c0 draws,
 // (2*c0 - 1) / 624 of them, are the first blocks of the real skip too.
-//
-// The blocks roll through registers: a step makes the next 224 words, seven
-// consecutive ones per lane (the recurrence reaches back 227 words at the
-// least, so a step depends on earlier steps only), from the three steps
-// before it: eleven shuffles, no shared memory and no barrier.  In shared
-// memory, three phases a block, the 600 blocks of a 128^3 image's first
-// masked plane took 265 us for 102 slots, now 391 us for one of 396.
-__device__ __forceinline__ void mt_step(unsigned (&n)[7], const unsigned (&a)[7], const unsigned (&b)[7],
-                                        const unsigned (&c)[7], int lane) {
-    // word t = 7 lane + i of the step needs words t - 3 of the last step (a),
-    // t + 48 and t + 49 of the third last (c); past the step's ends the word
-    // lies in the one before (b), supplied by the lanes at that end
-    unsigned g[7], q[3];
-    const unsigned f = __shfl_sync(0xffffffffu, lane < 6 ? b[6] : c[6], (lane + 6) & 31);
-#pragma unroll
-    for (int i = 0; i < 7; ++i) g[i] = __shfl_sync(0xffffffffu, lane < 7 ? b[i] : c[i], (lane + 7) & 31);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) q[i] = __shfl_sync(0xffffffffu, lane == 31 ? b[4 + i] : a[4 + i], (lane + 31) & 31);
-#pragma unroll
-    for (int i = 0; i < 7; ++i) n[i] = mt_mix(i == 0 ? f : g[i > 0 ? i - 1 : 0], g[i], i < 3 ? q[i < 3 ? i : 0] : a[i >= 3 ? i - 3 : 0]);
-}
-
-// `blocks` > 0 blocks further from the state mt[624] (shared memory), in place
-__device__ void mt_roll(unsigned *mt, long long blocks, int lane) {
-    unsigned r0[7], r1[7], r2[7], r3[7];
-#pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        const int t = 7 * lane + i;
-        r0[i] = mt[400 + t];
-        r1[i] = mt[176 + t];
-        r2[i] = t >= 48 ? mt[t - 48] : 0u;   // words below 48 of this step are read by none
-        r3[i] = 0u;
-    }
-    const long long steps = (624 * blocks + 223) / 224;
-    for (long long s = 0; s + 4 <= steps; s += 4) {
-        mt_step(r3, r0, r1, r2, lane);
-        mt_step(r2, r3, r0, r1, lane);
-        mt_step(r1, r2, r3, r0, lane);
-        mt_step(r0, r1, r2, r3, lane);
-    }
-    __syncwarp();
-    // word 7 lane + i of step `step` is word k of the state
-    auto put = [&](const unsigned (&r)[7], long long step) {
-#pragma unroll
-        for (int i = 0; i < 7; ++i) {
-            const long long k = 224 * step + 7 * lane + i - 624 * (blocks - 1);
-            if (k >= 0 && k < 624) mt[k] = r[i];
-        }
-    };
-    const int rest = int(steps & 3);
-    if (rest > 0) mt_step(r3, r0, r1, r2, lane);
-    if (rest > 1) mt_step(r2, r3, r0, r1, lane);
-    if (rest > 2) mt_step(r1, r2, r3, r0, lane);
-    // the last four steps hold the 624 words (and at most 223 beyond them)
-    put(r0, rest == 0 ? steps - 1 : steps - 1 - rest);
-    put(r1, rest == 3 ? steps - 1 : steps - 2 - rest);
-    put(r2, rest >= 2 ? steps + 1 - rest : steps - 3 - rest);
-    put(r3, rest >= 1 ? steps - rest : steps - 4);
-    __syncwarp();
-}
-
 __global__ void __launch_bounds__(32 * RP_WARPS) k_mt_prep(SimPrepArgs A, unsigned *__restrict__ state,
                                                            int *__restrict__ pre) {
     __shared__ __align__(16) unsigned mt[RP_WARPS][624];
@@ -2496,19 +2542,9 @@ __global__ void __launch_bounds__(32 * RP_WARPS) k_mt_prep(SimPrepArgs A, unsign
     if (ng.skip) return;
     if (lane == 0) mt_seed(mt[wib], A.seeds[i]);
     __syncwarp();
-    int blocks = 0;
-    const Geom &g = A.g;
-    if (ng.nvalid >= ng.Ki && !A.missing && ng.nvalid > 0) {
-        long long m0 = 0;
-        for (int d = 0; d < g.nd; ++d) m0 += (long long)ng.lo[d] * g.sstride[d];
-        const long long n = 2 * (m0 - valid_prefix(g, ng.lo, m0));
-        if (n > 624) blocks = int((n - 1) / 624);
-    }
+    const long long blocks = A.missing ? 0 : skipped_blocks(A.g, ng.lo, ng.nvalid, ng.Ki);
     if (blocks > 0) mt_roll(mt[wib], blocks, lane);
-    // a state row is 624 words, a multiple of 16 bytes
-    uint4 *row = reinterpret_cast<uint4 *>(state + (long long)b * 624);
-    for (int i = lane; i < 156; i += 32) row[i] = *reinterpret_cast<const uint4 *>(&mt[wib][4 * i]);
-    if (lane == 0) pre[b] = 624 * blocks;
+    store_generator(mt[wib], blocks, b, state, pre, lane);
 }
 
 // Verbatim exclusion with a radius (CPUThreadDevice::setValueInErrorArrayWithRadius,
@@ -2643,17 +2679,23 @@ int map_segs_per_cta(const Geom &g, int nslots) {
     return (int)(per * turn);
 }
 
+template <bool GEN>
+static void launch_map_records_k(const MapArgs &a, dim3 grid, size_t smem, int K, cudaStream_t st) {
+    if (K <= 1) k_map_records<1, GEN><<<grid, 256, smem, st>>>(a);
+    else if (K <= 2) k_map_records<2, GEN><<<grid, 256, smem, st>>>(a);
+    else if (K <= 4) k_map_records<4, GEN><<<grid, 256, smem, st>>>(a);
+    else if (K <= 8) k_map_records<8, GEN><<<grid, 256, smem, st>>>(a);
+    else k_map_records<16, GEN><<<grid, 256, smem, st>>>(a);
+}
+
 cudaError_t launch_map_records(const MapArgs &args, int nslots, int K, int maxterms_in_batch, cudaStream_t st) {
-    int threads = 256;
     MapArgs a = args;
     for (int d = 0; d < QSK_MAXD; ++d) a.div[d] = make_fast_div((unsigned)a.g.fft[d]);
-    dim3 grid((unsigned)((a.g.nseg + a.segs_per_cta - 1) / a.segs_per_cta), (unsigned)nslots);
+    dim3 grid((unsigned)((a.g.nseg + a.segs_per_cta - 1) / a.segs_per_cta) + (a.gen.state ? 1u : 0u), (unsigned)nslots);
     size_t smem = sizeof(Term) * (size_t)(maxterms_in_batch > 0 ? maxterms_in_batch : 1);
-    if (K <= 1) k_map_records<1><<<grid, threads, smem, st>>>(a);
-    else if (K <= 2) k_map_records<2><<<grid, threads, smem, st>>>(a);
-    else if (K <= 4) k_map_records<4><<<grid, threads, smem, st>>>(a);
-    else if (K <= 8) k_map_records<8><<<grid, threads, smem, st>>>(a);
-    else k_map_records<16><<<grid, threads, smem, st>>>(a);
+    if (a.gen.state && smem < 624 * sizeof(unsigned)) smem = 624 * sizeof(unsigned);
+    if (a.gen.state) launch_map_records_k<true>(a, grid, smem, K, st);
+    else launch_map_records_k<false>(a, grid, smem, K, st);
     return cudaGetLastError();
 }
 
@@ -2676,33 +2718,40 @@ int map_bits_segs_per_cta(const Geom &g, int nslots) {
     return (int)per;
 }
 
+template <bool GEN>
+static void launch_map_bits_k(const BitArgs &a, dim3 grid, size_t smem, int K, cudaStream_t st) {
+    if (K <= 1) k_map_bits<1, GEN><<<grid, 256, smem, st>>>(a);
+    else if (K <= 2) k_map_bits<2, GEN><<<grid, 256, smem, st>>>(a);
+    else if (K <= 4) k_map_bits<4, GEN><<<grid, 256, smem, st>>>(a);
+    else if (K <= 8) k_map_bits<8, GEN><<<grid, 256, smem, st>>>(a);
+    else k_map_bits<16, GEN><<<grid, 256, smem, st>>>(a);
+}
+
 cudaError_t launch_map_bits(const BitArgs &args, int nslots, int K, int maxterms_in_batch, cudaStream_t st) {
-    int threads = 256;
     BitArgs a = args;
     if (a.maxterms < maxterms_in_batch) return cudaErrorInvalidValue;
     a.stage_words = MAP_BITS_STAGE_WORDS;
     long long nseg1k = (a.g.N + 1023) / 1024;
-    dim3 grid((unsigned)((nseg1k + a.segs_per_cta - 1) / a.segs_per_cta), (unsigned)nslots);
+    dim3 grid((unsigned)((nseg1k + a.segs_per_cta - 1) / a.segs_per_cta) + (a.gen.state ? 1u : 0u), (unsigned)nslots);
     size_t smem = sizeof(int2) * (size_t)(a.maxterms > 0 ? a.maxterms : 1) + sizeof(unsigned) * (size_t)a.stage_words;
-    if (K <= 1) k_map_bits<1><<<grid, threads, smem, st>>>(a);
-    else if (K <= 2) k_map_bits<2><<<grid, threads, smem, st>>>(a);
-    else if (K <= 4) k_map_bits<4><<<grid, threads, smem, st>>>(a);
-    else if (K <= 8) k_map_bits<8><<<grid, threads, smem, st>>>(a);
-    else k_map_bits<16><<<grid, threads, smem, st>>>(a);
+    if (a.gen.state) launch_map_bits_k<true>(a, grid, smem, K, st);
+    else launch_map_bits_k<false>(a, grid, smem, K, st);
     return cudaGetLastError();
 }
 
+template <int KF>
+static cudaError_t map_smem_limit(int bytes) {
+    cudaError_t e = cudaFuncSetAttribute(k_map_records<KF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_map_records<KF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 cudaError_t set_map_smem_limit(int bytes) {
-    cudaError_t e = cudaSuccess;
-    e = cudaFuncSetAttribute(k_map_records<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_map_records<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_map_records<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_map_records<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(k_map_records<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaError_t e;
+    if ((e = map_smem_limit<1>(bytes)) != cudaSuccess || (e = map_smem_limit<2>(bytes)) != cudaSuccess ||
+        (e = map_smem_limit<4>(bytes)) != cudaSuccess || (e = map_smem_limit<8>(bytes)) != cudaSuccess)
+        return e;
+    return map_smem_limit<16>(bytes);
 }
 
 cudaError_t launch_radius_mask(const int *center, const float *radius, int nslots, const Geom &g, unsigned *mask,
