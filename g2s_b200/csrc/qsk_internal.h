@@ -556,4 +556,16 @@ __host__ __device__ inline unsigned tie_hash(unsigned seed, unsigned pos) {
     return x;
 }
 
+// the position whose hash under `seed` is `hash` (every step of tie_hash is a
+// bijection; the factors are the inverses of its factors modulo 2^32)
+__host__ __device__ inline unsigned tie_position(unsigned seed, unsigned hash) {
+    unsigned x = hash;
+    x ^= x >> 16;
+    x *= 0x43021123u;
+    x ^= (x >> 15) ^ (x >> 30);
+    x *= 0x1D69E2A5u;
+    x ^= x >> 16;
+    return (x ^ seed) * 0x144CBC89u;
+}
+
 }  // namespace qsk

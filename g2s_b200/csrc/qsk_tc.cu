@@ -17,12 +17,22 @@
 //               positions x K=16/32, FP32 accumulators in TMEM, two buffers
 //               of 256 columns so that the epilogue of tile t overlaps the
 //               MMAs of tile t+1; tcgen05.commit frees stages and buffers
-//   warps 2-5   epilogue: one thread per node (TMEM lane), 32 columns per
-//               tcgen05.ld; score = acc * node_scale * pos_scale + node_bias;
-//               scores at least the heap's minimum go through the full key
-//               (ordered score, 32-bit tie hash of node seed and position),
-//               the node's validity box (the template inside the TI) and a
-//               replace-root/sift-down in shared memory
+//   the others  epilogue: groups of four warps, one thread per node (TMEM
+//               lane) and group, 32 columns per tcgen05.ld; score = acc *
+//               node_scale * pos_scale + node_bias; scores at least the
+//               W-th best so far whose position lies in the node's validity
+//               box (the template inside the TI) enter by their full key
+//               (ordered score, 32-bit tie hash of node seed and position):
+//               up to 16 keys sorted in the thread's registers, 32 as a list
+//               in shared memory that the whole warp updates.  The position
+//               is not kept beside the key: the tie hash of a seed is a
+//               bijection of positions and is inverted at the end.  The
+//               epilogue bounds the kernel wherever K is short: the 8,000-node
+//               FP8 sample of a 180x150x120 image (W = 32) went 64 -> 44 ms in
+//               this kernel with lists in place of 32-key register insertion
+//               (a chain of 31 compare-and-swaps for the whole warp), the
+//               BF16 levels of 250x250 -> 500x500 (W = 8) 171 -> 136 us with
+//               the first chunk cut to its own eight best and keys alone
 //
 // Every mbarrier wait is bounded by a clock budget; on expiry the kernel
 // records DEV_TC_WAIT, drains the copies it issued (bounded too), frees its
@@ -53,6 +63,11 @@ constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 // hide more of the insertion latency (the W = 32 registers allow two)
 __host__ __device__ constexpr int epi_groups(int W) { return W <= 16 ? 4 : 2; }
 __host__ __device__ constexpr int threads_for(int W) { return 64 + 128 * epi_groups(W); }
+// epilogue shared memory: 32 scores of each of 512 threads, or 2 x 128 lists
+// of 32 keys, a key apart (rows of 33: a lane's own list on its own banks)
+constexpr int LIST_STRIDE = 33;
+constexpr int EPI_BYTES = 2 * BM * LIST_STRIDE * 8;
+static_assert(EPI_BYTES >= 512 * 32 * 4, "scores of every epilogue thread");
 constexpr long long WAIT_CYCLES = 4000000000LL;   // about two seconds at 1.9 GHz
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -164,24 +179,69 @@ __device__ __forceinline__ float unordered(unsigned o) {
     return __uint_as_float((o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o);
 }
 
+typedef unsigned long long u64;
+
 // insert key (larger than k[0]) into the ascending register array k of W
 // keys, dropping the minimum: the new key replaces k[0] and bubbles up by
 // compare-and-swap steps (no branch, no memory)
 template <int W>
-__device__ __forceinline__ void sorted_insert(unsigned long long (&k)[W], unsigned (&p)[W], unsigned long long key,
-                                              unsigned pos) {
+__device__ __forceinline__ void sorted_insert(u64 (&k)[W], u64 key) {
     k[0] = key;
-    p[0] = pos;
 #pragma unroll
     for (int i = 0; i + 1 < W; ++i) {
         const bool sw = k[i] > k[i + 1];
-        const unsigned long long a = k[i], b = k[i + 1];
-        const unsigned pa = p[i], pb = p[i + 1];
+        const u64 a = k[i], b = k[i + 1];
         k[i] = sw ? b : a;
         k[i + 1] = sw ? a : b;
-        p[i] = sw ? pb : pa;
-        p[i + 1] = sw ? pa : pb;
     }
+}
+
+// position of a key (0xFFFFFFFF: an empty entry)
+__device__ __forceinline__ unsigned key_position(u64 key, unsigned seed) {
+    return key ? tie_position(seed, (unsigned)key) : 0xFFFFFFFFu;
+}
+
+__device__ __forceinline__ u64 shfl_u64(u64 v, int src) {
+    return (u64)__shfl_sync(0xffffffffu, (unsigned)(v >> 32), src) << 32 | __shfl_sync(0xffffffffu, (unsigned)v, src);
+}
+__device__ __forceinline__ u64 shfl_xor_u64(u64 v, int m) {
+    return (u64)__shfl_xor_sync(0xffffffffu, (unsigned)(v >> 32), m) << 32 | __shfl_xor_sync(0xffffffffu, (unsigned)v, m);
+}
+
+// one key per lane sorted over the warp: bitonic steps of sequences of `len`
+// (the first: 2), up to whole runs of 32; ascending or descending
+__device__ __forceinline__ u64 warp_sort(u64 v, int lane, int len, bool ascending) {
+    for (int k = len; k <= 32; k <<= 1)
+        for (int d = k >> 1; d > 0; d >>= 1) {
+            const u64 o = shfl_xor_u64(v, d);
+            const bool up = ((lane & k) == 0) == ascending;   // direction of this lane's sequence (k = 32: all)
+            const bool low = (lane & d) == 0;
+            v = ((v < o) == (up == low)) ? v : o;
+        }
+    return v;
+}
+
+__device__ __forceinline__ void order_desc(float &a, float &b) {
+    const float hi = fmaxf(a, b);
+    b = fminf(a, b);
+    a = hi;
+}
+// eight values in descending order (Batcher's odd-even merge sort, 19 steps)
+__device__ __forceinline__ void sort8(float (&x)[8]) {
+    constexpr int A[19] = {0, 2, 4, 6, 0, 1, 4, 5, 1, 5, 0, 1, 2, 3, 2, 3, 1, 3, 5};
+    constexpr int B[19] = {1, 3, 5, 7, 2, 3, 6, 7, 2, 6, 4, 5, 6, 7, 4, 5, 2, 4, 6};
+#pragma unroll
+    for (int i = 0; i < 19; ++i) order_desc(x[A[i]], x[B[i]]);
+}
+// a: the eight largest of a and b (both descending), descending
+__device__ __forceinline__ void merge8(float (&a)[8], const float (&b)[8]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = fmaxf(a[i], b[7 - i]);
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1)
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if ((i & d) == 0) order_desc(a[i], a[i + d]);
 }
 
 template <int KIND, int W, int STAGES>
@@ -193,11 +253,12 @@ __global__ void __launch_bounds__(threads_for(W), 1)
     uint8_t *smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     uint8_t *sA = smem;                                   // STAGES x A_BYTES
     uint8_t *sB = smem + STAGES * A_BYTES;                // STAGES x B_BYTES
-    constexpr int G = epi_groups(W), EPI_WARPS = 4 * G, THREADS = threads_for(W);
-    // the other epilogue groups' W best per node, for the final merge: [group-1][entry][row]
-    unsigned long long *hk = reinterpret_cast<unsigned long long *>(smem + STAGES * STAGE_BYTES);
-    unsigned *hp = reinterpret_cast<unsigned *>(hk + (G - 1) * W * BM);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(hp + (G - 1) * W * BM);
+    constexpr int G = epi_groups(W), EPI_WARPS = 4 * G;
+    // epilogue memory: the lists of W keys per group and node (LISTS), or the
+    // chunk's scores of every thread, later the other groups' keys
+    constexpr bool LISTS = W > 16;
+    u64 *epi = reinterpret_cast<u64 *>(smem + STAGES * STAGE_BYTES);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES + EPI_BYTES);
     uint64_t *full = bar, *empty = bar + STAGES, *tfull = bar + 2 * STAGES, *tempty = tfull + 2, *done = tempty + 2;
     __shared__ unsigned tmem_base_s;
     __shared__ volatile int abort_s;
@@ -317,9 +378,9 @@ __global__ void __launch_bounds__(threads_for(W), 1)
             mbar_wait(done, 0, nullptr);
         }
     } else {
-        // ---------------- epilogue: one thread per node and half ----------------
-        // warps 2..9: lane quarter q = warp % 4 (the TMEM lanes this warp may
-        // read), half h: the even or odd 32-column chunks of every tile
+        // ---------------- epilogue: one thread per node and group ----------------
+        // lane quarter q = warp % 4 (the TMEM lanes this warp may read), group
+        // h: every G-th 32-column chunk of every tile
         const int e = warp - 2;
         const int q = warp & 3, h = e >> 2;   // lane quarter, group
         const int row = q * 32 + lane;
@@ -335,19 +396,27 @@ __global__ void __launch_bounds__(threads_for(W), 1)
 #pragma unroll
             for (int d = 0; d < 6; ++d) box[d] = a.node_box[node * 6 + d];
         }
-        // this half's W best keys in registers, ascending (rk[0] the minimum);
-        // keys start at 0, below every real key (ordered() of a score is > 0)
-        unsigned long long rk[W];
-        unsigned rp[W];
+        // this group's W best keys, ascending (rk[0] the minimum), or in the
+        // node's list; keys start at 0, below every real key (ordered() of a
+        // score is > 0)
+        constexpr int R = LISTS ? 1 : W;
+        u64 rk[R];
 #pragma unroll
-        for (int f = 0; f < W; ++f) {
-            rk[f] = 0ull;
-            rp[f] = 0xFFFFFFFFu;
+        for (int f = 0; f < R; ++f) rk[f] = 0ull;
+        u64 *lists = epi + (size_t)(h * BM + q * 32) * LIST_STRIDE;   // LISTS: this warp's 32 nodes
+        if constexpr (LISTS) {
+            for (int l = 0; l < 32; ++l) lists[l * LIST_STRIDE + lane] = 0ull;
+            __syncwarp();
         }
-        unsigned long long root = 0ull;
+        float *scratch = reinterpret_cast<float *>(epi) + e * 32 + lane;   // !LISTS: score j at [j * 32 * EPI_WARPS]
+        u64 root = 0ull;   // the W-th best key
         float thr = -INFINITY;
         unsigned g_seen = 0u;   // largest value of the shared bound this thread has read or published
         int i = 0;
+        // TI coordinates of the tile's first position
+        int x0 = (int)((t_begin * BN) % a.X);
+        int y0 = (int)((t_begin * BN) / a.X % a.Y);
+        int z0 = (int)((t_begin * BN) / a.X / a.Y);
         for (long long t = t_begin; t < t_end; ++t, ++i) {
             const int b = i & 1;
             const unsigned tph = (unsigned)(i >> 1) & 1u;
@@ -368,26 +437,24 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                 g_seen = g > g_seen ? g : g_seen;
                 if (g) thr = fmaxf(thr, unordered(g));
             }
-            // TI coordinates of the tile's first position
-            const int x0 = pos0 % a.X, y0 = (pos0 / a.X) % a.Y, z0 = pos0 / (a.X * a.Y);
 #pragma unroll 1
             for (int c = h; c < BN / 32; c += G) {
                 float v[32];
                 tmem_ld32(tmem + ((unsigned)(q * 32) << 16) + (unsigned)(b * BN + c * 32), v);
-                // candidates of this lane (0 for a dead row, a chunk whose best
-                // score is below the threshold, or no valid position); every
-                // lane reaches the warp-wide round count below
-                unsigned cand = 0u;
-                const int pc = pos0 + c * 32;
                 // a chunk's best score is exactly fmaf(max v, s, bias): fmaf is
                 // monotone in v for s > 0
                 float m01 = fmaxf(v[0], v[1]);
 #pragma unroll
                 for (int j = 2; j < 32; ++j) m01 = fmaxf(m01, v[j]);
-                if (live && fmaf(m01, s, nbias) >= thr) {
+                const bool reach = live && fmaf(m01, s, nbias) >= thr;
+                if (!__any_sync(0xffffffffu, reach)) continue;
+                const int pc = pos0 + c * 32;
+                // candidates of this lane (0 for a dead row, a chunk whose best
+                // score is below the threshold, or no valid position)
+                unsigned vmask = 0u;
+                if (reach) {
                     // validity of the chunk's 32 positions for this node (its
                     // template inside the TI): the box cut row by row
-                    unsigned vmask = 0u;
                     int x = x0 + c * 32, y = y0, z = z0;
                     while (x >= a.X) {
                         x -= a.X;
@@ -412,40 +479,101 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                             ++z;
                         }
                     }
-                    // at least the threshold; a tie with the heap's own minimum
-                    // qualifies only with a larger tie hash
-                    const float thr_loc = root ? unordered((unsigned)(root >> 32)) : -INFINITY;
+                }
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const float sc = fmaf(v[j], s, nbias);
-                        bool cj = sc >= thr && ((vmask >> j) & 1u);
-                        if (cj && root != 0ull && sc == thr_loc) cj = tie_hash(nseed, (unsigned)(pc + j)) > (unsigned)root;
-                        cand |= cj ? (1u << j) : 0u;
+                for (int j = 0; j < 32; ++j) v[j] = fmaf(v[j], s, nbias);
+                float bound = thr;
+                if constexpr (W == 8) {
+                    // fewer than eight keys so far: no more than the chunk's own
+                    // eight best can enter (their ties too), which a sorting
+                    // network finds without one insertion
+                    if (__any_sync(0xffffffffu, root == 0ull && vmask != 0u)) {
+                        float best[8], more[8];
+#pragma unroll
+                        for (int o = 0; o < 32; o += 8) {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) more[j] = ((vmask >> (o + j)) & 1u) ? v[o + j] : -INFINITY;
+                            sort8(more);
+                            if (o == 0) {
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) best[j] = more[j];
+                            } else {
+                                merge8(best, more);
+                            }
+                        }
+                        if (root == 0ull) bound = fmaxf(bound, best[7]);
                     }
                 }
-                // insert them in rounds: every lane its next candidate
-                const int rounds = __reduce_max_sync(0xffffffffu, __popc(cand));
-                for (int r = 0; r < rounds; ++r) {
-                    if (!cand) continue;
-                    const int j = __ffs(cand) - 1;
-                    cand &= cand - 1u;
-                    // v[j] by a 5-level select tree
-                    float t16[16], t8[8], t4[4], t2[2];
+                unsigned cand = 0u;
 #pragma unroll
-                    for (int u = 0; u < 16; ++u) t16[u] = (j & 1) ? v[2 * u + 1] : v[2 * u];
+                for (int j = 0; j < 32; ++j) cand |= v[j] >= bound ? (1u << j) : 0u;
+                cand &= vmask;
+                // a tie with the W-th best qualifies only with a larger tie hash:
+                // asked here where many positions tie (categorical match counts),
+                // else by the full key below
+                const unsigned most = __reduce_max_sync(0xffffffffu, (unsigned)__popc(cand));
+                if (most == 0u) continue;
+                if (most > 4u) {
+                    const float tie = root ? unordered((unsigned)(root >> 32)) : NAN;   // (equals no score)
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) t8[u] = (j & 2) ? t16[2 * u + 1] : t16[2 * u];
+                    for (int j = 0; j < 32; ++j)
+                        if (v[j] == tie && tie_hash(nseed, (unsigned)(pc + j)) <= (unsigned)root) cand &= ~(1u << j);
+                }
+                if constexpr (!LISTS) {
+                    // inserted in rounds, every lane its next candidate
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) t4[u] = (j & 4) ? t8[2 * u + 1] : t8[2 * u];
+                    for (int j = 0; j < 32; ++j) scratch[j * 32 * EPI_WARPS] = v[j];
+                    while (__any_sync(0xffffffffu, cand != 0u)) {
+                        if (!cand) continue;
+                        const int j = __ffs(cand) - 1;
+                        cand &= cand - 1u;
+                        const u64 key = (u64)ordered(scratch[j * 32 * EPI_WARPS]) << 32 | tie_hash(nseed, (unsigned)(pc + j));
+                        if (key <= root) continue;
+                        sorted_insert<R>(rk, key);
+                        root = rk[0];
+                        thr = root ? fmaxf(thr, unordered((unsigned)(root >> 32))) : thr;
+                    }
+                } else {
+                    // the lanes' next candidates, one list after the other: the key
+                    // takes the place of the list's smallest, whose successor two
+                    // warp-wide minima find
+                    while (__any_sync(0xffffffffu, cand != 0u)) {
+                        u64 key = 0ull;
+                        if (cand) {
+                            const int j = __ffs(cand) - 1;
+                            cand &= cand - 1u;
+                            // v[j] by a 5-level select tree
+                            float t16[16], t8[8], t4[4], t2[2];
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) t2[u] = (j & 8) ? t4[2 * u + 1] : t4[2 * u];
-                    const float sc = fmaf((j & 16) ? t2[1] : t2[0], s, nbias);
-                    const int p = pc + j;
-                    const unsigned long long key = ((unsigned long long)ordered(sc) << 32) | tie_hash(nseed, (unsigned)p);
-                    if (key <= root) continue;
-                    sorted_insert<W>(rk, rp, key, (unsigned)p);
-                    root = rk[0];
-                    thr = root ? fmaxf(thr, unordered((unsigned)(root >> 32))) : thr;
+                            for (int u = 0; u < 16; ++u) t16[u] = (j & 1) ? v[2 * u + 1] : v[2 * u];
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) t8[u] = (j & 2) ? t16[2 * u + 1] : t16[2 * u];
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) t4[u] = (j & 4) ? t8[2 * u + 1] : t8[2 * u];
+#pragma unroll
+                            for (int u = 0; u < 2; ++u) t2[u] = (j & 8) ? t4[2 * u + 1] : t4[2 * u];
+                            key = (u64)ordered((j & 16) ? t2[1] : t2[0]) << 32 | tie_hash(nseed, (unsigned)(pc + j));
+                            if (key <= root) key = 0ull;
+                        }
+                        unsigned act = __ballot_sync(0xffffffffu, key != 0ull);
+                        while (act) {
+                            const int l = __ffs(act) - 1;
+                            act &= act - 1u;
+                            const u64 kl = shfl_u64(key, l), rl = shfl_u64(root, l);
+                            u64 k = lists[l * LIST_STRIDE + lane];
+                            const int slot = __ffs(__ballot_sync(0xffffffffu, k == rl)) - 1;
+                            if (lane == slot) {
+                                k = kl;
+                                lists[l * LIST_STRIDE + lane] = kl;
+                            }
+                            const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32));
+                            const unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : ~0u);
+                            if (lane == l) {
+                                root = (u64)hi << 32 | lo;
+                                thr = root ? fmaxf(thr, unordered(hi)) : thr;
+                            }
+                        }
+                    }
                 }
             }
             // publish this heap's minimum: a lower bound of the node's W-th best
@@ -460,27 +588,50 @@ __global__ void __launch_bounds__(threads_for(W), 1)
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty[b]);
-        }
-        // the other groups hand their W best to group 0, which merges and
-        // writes the node's W best of this range
-        if (h > 0) {
-#pragma unroll
-            for (int f = 0; f < W; ++f) {
-                hk[((h - 1) * W + f) * BM + row] = rk[f];
-                hp[((h - 1) * W + f) * BM + row] = rp[f];
+            x0 += BN;
+            while (x0 >= a.X) {
+                x0 -= a.X;
+                if (++y0 == a.Y) {
+                    y0 = 0;
+                    ++z0;
+                }
             }
         }
+        // the groups' W best merged, ascending, into the node's W best of this range
         asm volatile("bar.sync 1, %0;" ::"r"(EPI_WARPS * 32) : "memory");
-        if (h == 0 && live) {
-            for (int f = 0; f < (G - 1) * W; ++f) {
-                const unsigned long long key = hk[f * BM + row];
-                if (key > rk[0]) sorted_insert<W>(rk, rp, key, hp[f * BM + row]);
+        if constexpr (LISTS) {
+            static_assert(!LISTS || (W == 32 && G == 2), "two lists of one key per lane");
+            for (int r = e; r < BM; r += EPI_WARPS) {
+                const int nd = tile_m * BM + r;
+                if (nd >= a.n_nodes) break;
+                // ascending against descending: the larger of each pair are the best
+                const u64 u = warp_sort(epi[r * LIST_STRIDE + lane], lane, 2, true);
+                const u64 w = warp_sort(epi[(BM + r) * LIST_STRIDE + lane], lane, 2, false);
+                const u64 key = warp_sort(u > w ? u : w, lane, 32, true);
+                const size_t o = ((size_t)nd * a.ranges + range) * W + lane;
+                a.out_key[o] = key;
+                a.out_pos[o] = key_position(key, a.node_seed ? a.node_seed[nd] : 0u);
             }
-            const size_t o = ((size_t)node * a.ranges + range) * W;
+        } else {
+            // (every score of a chunk has been read: the scores' memory is free)
+            if (h > 0) {
 #pragma unroll
-            for (int f = 0; f < W; ++f) {
-                a.out_key[o + f] = rk[f];
-                a.out_pos[o + f] = rp[f];
+                for (int f = 0; f < R; ++f) epi[((h - 1) * W + f) * BM + row] = rk[f];
+            }
+            asm volatile("bar.sync 1, %0;" ::"r"(EPI_WARPS * 32) : "memory");
+            if (h == 0 && live) {
+                for (int o = 0; o < G - 1; ++o)
+                    for (int f = W - 1; f >= 0; --f) {   // from its best down
+                        const u64 key = epi[(o * W + f) * BM + row];
+                        if (key <= rk[0]) break;
+                        sorted_insert<R>(rk, key);
+                    }
+                const size_t o = ((size_t)node * a.ranges + range) * W;
+#pragma unroll
+                for (int f = 0; f < R; ++f) {
+                    a.out_key[o + f] = rk[f];
+                    a.out_pos[o + f] = key_position(rk[f], nseed);
+                }
             }
         }
     }
@@ -665,9 +816,9 @@ cudaError_t make_map(CUtensorMap *m, const void *base, int elem, long long k_ele
 template <int KIND, int W>
 cudaError_t launch_w(const CUtensorMap &ma, const CUtensorMap &mp, const TcArgs &a, int node_tiles,
                      cudaStream_t st) {
-    constexpr int HEAP = (tc::epi_groups(W) - 1) * W * tc::BM * 12;
+    static_assert((tc::epi_groups(W) - 1) * W * tc::BM * 8 <= tc::EPI_BYTES, "the other groups' keys");
     constexpr int STAGES = 3;
-    constexpr int SMEM = 1024 + STAGES * tc::STAGE_BYTES + HEAP + (2 * STAGES + 5) * 8;
+    constexpr int SMEM = 1024 + STAGES * tc::STAGE_BYTES + tc::EPI_BYTES + (2 * STAGES + 5) * 8;
     static_assert(SMEM <= 232448, "shared memory");
     auto kern = tc::k_tc_shortlist<KIND, W, STAGES>;
     // the shared-memory limit, once per device for this instantiation

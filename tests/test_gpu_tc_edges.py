@@ -1,0 +1,67 @@
+"""The shortlist's top-W at its edges against a full sort of the same exact
+keys: fewer valid positions than W, every score equal (the tie hash decides
+alone), scores that rise along the positions (every position enters), and the
+widths on either side of the register / list split.  Small integers are exact
+in BF16 and FP32, so keys and positions are equal, not close."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def tie_hash(seed, pos):
+    x = (np.uint64(seed) ^ ((pos.astype(np.uint64) * np.uint64(0x9E3779B9)) & np.uint64(0xFFFFFFFF)))
+    m = np.uint64(0xFFFFFFFF)
+    x ^= x >> np.uint64(16)
+    x = (x * np.uint64(0x7FEB352D)) & m
+    x ^= x >> np.uint64(15)
+    x = (x * np.uint64(0x846CA68B)) & m
+    return x ^ (x >> np.uint64(16))
+
+
+def bf16_bits(a):
+    return (np.ascontiguousarray(a, np.float32).view(np.uint32) >> 16).astype(np.uint16)
+
+
+@pytest.mark.parametrize("ranges", [1, 3])
+@pytest.mark.parametrize("W", [8, 16, 32])
+@pytest.mark.parametrize("kind", ["equal", "rising", "falling", "mixed", "narrow box"])
+def test_shortlist_edges(g2s, gpu, W, kind, ranges):
+    rng = np.random.default_rng(W + len(kind))
+    X, Y, B, K = 40, 37, 130, 64
+    N = X * Y
+    rows = np.zeros((N, K), np.float32)
+    q = np.zeros((B, K), np.float32)
+    q[:, 0] = 1.0
+    q[:, 1] = 16.0
+    p = np.arange(N)
+    if kind in ("rising", "falling"):
+        o = p if kind == "rising" else p[::-1]
+        rows[:, 0], rows[:, 1] = o % 16, o // 16   # at most 92: exact in BF16
+    elif kind != "equal":
+        rows[:, 0] = rng.integers(0, 4, N)
+        q[:, 2] = rng.integers(-2, 3, B)
+        rows[:, 2] = rng.integers(0, 3, N)
+    box = np.tile(np.array([2, X - 3, 1, Y - 2, 0, 1], np.int32), (B, 1))
+    if kind == "narrow box":
+        box[:, 0] = rng.integers(0, X, B)
+        box[:, 1] = np.minimum(box[:, 0] + rng.integers(0, 3, B), X)
+        box[:, 3] = np.minimum(box[:, 2] + rng.integers(0, 4, B), Y)
+    seeds = rng.integers(0, 2**32, B, dtype=np.uint32)
+    keys, pos = g2s.tc_topk(bf16_bits(q), bf16_bits(rows), 0, X, Y, box, W=W, ranges=ranges, q_seed=seeds)
+    score = (q @ rows.T).astype(np.float32)
+    ordered = score.view(np.uint32).astype(np.uint64)
+    ordered = np.where(score < 0, ~ordered & np.uint64(0xFFFFFFFF), ordered | np.uint64(0x80000000))
+    x, y = p % X, p // X
+    tiles = (N + 255) // 256
+    per = (tiles + ranges - 1) // ranges * 256
+    for b in range(B):
+        inside = (x >= box[b, 0]) & (x < box[b, 1]) & (y >= box[b, 2]) & (y < box[b, 3])
+        full = (ordered[b] << np.uint64(32)) | tie_hash(seeds[b], p)
+        for r in range(ranges):
+            at = p[inside & (p >= r * per) & (p < (r + 1) * per)]
+            best = at[np.argsort(full[at])][-W:]
+            want_k = np.concatenate([np.zeros(W - len(best), np.uint64), full[best]])
+            want_p = np.concatenate([np.full(W - len(best), 0xFFFFFFFF, np.uint32), best.astype(np.uint32)])
+            assert np.array_equal(keys[b, r], want_k), (b, r)
+            assert np.array_equal(pos[b, r], want_p), (b, r)
