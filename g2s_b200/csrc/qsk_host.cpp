@@ -853,7 +853,8 @@ struct qsk_sim {
     DBuf<unsigned char> d_tc_A;         // slots x tc_Kp
     DBuf<float> d_tc_nscale, d_tc_bias;
     DBuf<int> d_tc_box, d_tc_tmax, d_tc_kb, d_var_layer0, d_var_ncat;
-    DBuf<unsigned> d_tc_seed, d_tc_pos, d_tc_thr;
+    DBuf<unsigned> d_tc_seed, d_tc_pos, d_tc_cnt;
+    DBuf<unsigned long long> d_tc_thr;
     DBuf<float> d_var_catv, d_drawn_score, d_drawn_scale;
     DBuf<unsigned long long> d_tc_key, d_tc_counts;
     DBuf<Slot> d_tc_slots;
@@ -1098,6 +1099,8 @@ struct Step {
 };
 
 int tc_step(qsk_sim *s, const Step &st, bool teacher);
+constexpr int TC_LIST = 1536;   // keys a node's bounded shortlist may hold (ranges x W)
+bool tc_bounded(const qsk_sim *s) { return s->tc_S <= s->tc_W && s->topt.mode != 3; }
 
 // plain steps, one per slot budget of every level (levels in order)
 std::vector<Step> plain_steps(qsk_sim *s, const std::vector<int> &start) {
@@ -1911,6 +1914,7 @@ int tc_step(qsk_sim *s, const Step &step, bool teacher) {
     na.A = learned ? nullptr : s->d_tc_A.p;   // rows zeroed by the kernel
     na.rows = Bp;
     na.node_thr = s->d_tc_thr.p;
+    na.node_count = s->d_tc_cnt.p;
     na.node_scale = s->d_tc_nscale.p;
     na.node_bias = s->d_tc_bias.p;
     na.node_box = s->d_tc_box.p;
@@ -1920,13 +1924,14 @@ int tc_step(qsk_sim *s, const Step &step, bool teacher) {
     if (learned) CK(launch_tc_nodes(na, s->st));
     else CK(launch_prep_tc_nodes(pa, na, s->st));
     if (s->profiling) CK(cudaEventRecord(tc_event(s), s->st));
-    // GEMM shortlist: enough position ranges to fill the GPU, at most
-    // SEL_CAND / W candidates per node.  With a shortlist of at most W the
-    // shared bound makes the ranges' union hold the exact overall top W for
-    // any number of ranges: one wave of CTAs (one per SM), each scanning
-    // more position tiles, saves a second wave's set-up (TMEM allocation,
-    // pipeline fill) on the short levels.  A longer shortlist keeps two
-    // waves' worth of ranges, whose heaps it is drawn from.
+    // GEMM shortlist: enough position ranges to fill the GPU.  With a
+    // shortlist of at most W the shared bound makes the ranges' union hold the
+    // exact overall top W for any number of ranges, and the ranges leave what
+    // it lets through (TC_LIST keys at most): one wave of CTAs (one per SM),
+    // each scanning more position tiles, saves a second wave's set-up (TMEM
+    // allocation, pipeline fill) on the short levels.  A longer shortlist
+    // keeps two waves' worth of ranges, whose heaps it is drawn from, at most
+    // SEL_CAND / W.
     if (s->sm_count <= 0) {
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
@@ -1937,7 +1942,9 @@ int tc_step(qsk_sim *s, const Step &step, bool teacher) {
     const long long sms = s->sm_count;
     int ranges = int(s->tc_S <= s->tc_W ? std::max<long long>(1, sms / node_tiles)
                                         : std::max<long long>(1, (2 * sms + node_tiles - 1) / node_tiles));
-    ranges = int(std::min<long long>({(long long)ranges, ntiles, 768LL / s->tc_W}));
+    // (the learned proposal's check reads the ranges' heap minima)
+    const bool bounded = tc_bounded(s);
+    ranges = int(std::min<long long>({(long long)ranges, ntiles, (bounded ? (long long)TC_LIST : 768LL) / s->tc_W}));
     TcArgs a{};
     a.n_nodes = B;
     a.n_pos = s->ti->cells;
@@ -1956,7 +1963,9 @@ int tc_step(qsk_sim *s, const Step &step, bool teacher) {
     a.Y = g.nd > 1 ? g.src[1] : 1;
     // a shared bound across ranges keeps the overall top W in the union of the
     // ranges' heaps: enough when the shortlist takes at most W of them
-    a.node_thr = s->tc_S <= s->tc_W ? s->d_tc_thr.p : nullptr;
+    a.node_thr = bounded ? s->d_tc_thr.p : nullptr;
+    a.out_count = bounded ? s->d_tc_cnt.p : nullptr;
+    a.out_stride = TC_LIST;
     a.out_key = s->d_tc_key.p;
     a.out_pos = s->d_tc_pos.p;
     a.status = s->d_status.p;
@@ -1974,6 +1983,9 @@ int tc_step(qsk_sim *s, const Step &step, bool teacher) {
     sa.cand_key = s->d_tc_key.p;
     sa.cand_pos = s->d_tc_pos.p;
     sa.ncand = a.ranges * s->tc_W;
+    sa.cand_count = a.out_count;
+    sa.cand_stride = TC_LIST;
+    sa.node_seed = s->d_tc_seed.p;
     sa.S = s->tc_S;
     sa.fp64 = s->tc_fmt == 1 ? 1 : 0;
     sa.ti = s->ti->grid.p;
@@ -2031,8 +2043,13 @@ int tc_buffers(qsk_sim *s, size_t n_audit) {
     CK(s->d_tc_box.ensure(bp * 6));
     CK(s->d_tc_seed.ensure(bp));
     CK(s->d_tc_thr.ensure(bp));
-    CK(s->d_tc_key.ensure(slots * 768));
-    CK(s->d_tc_pos.ensure(slots * 768));
+    CK(s->d_tc_cnt.ensure(bp));
+    if (tc_bounded(s)) {
+        CK(s->d_tc_key.ensure(slots * TC_LIST));
+    } else {
+        CK(s->d_tc_key.ensure(slots * 768));
+        CK(s->d_tc_pos.ensure(slots * 768));
+    }
     CK(s->d_tc_slots.ensure(slots));
     CK(s->d_tc_terms.ensure(slots * size_t(s->maxterms)));
     CK(s->d_drawn_score.ensure(size_t(std::max<long long>(s->nodes, 1))));

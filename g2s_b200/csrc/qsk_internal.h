@@ -356,10 +356,17 @@ struct TcArgs {
     const unsigned *node_seed; // per A row tie-break seed (null: 0)
     const int *node_box;       // per A row: x0, x1, y0, y1, z0, z1 (p valid iff x0 <= x < x1, ...)
     int X, Y;                  // P row p is TI cell (x, y, z), x fastest
-    unsigned *node_thr;        // per A row, zeroed before the launch: the best heap minimum of any range
-                               // (ordered score), a lower bound of the row's W-th best (null: none)
-    unsigned long long *out_key;   // [row][range][W]: (ordered score << 32) | tie hash; 0 = empty
-    unsigned *out_pos;             // [row][range][W]
+    // null, or per A row (zeroed before the launch) the best heap minimum of
+    // any range, a lower bound of the row's W-th best key: the ranges filter
+    // against it and leave only what it lets through, as a list per row
+    unsigned long long *node_thr;
+    unsigned *out_count;           // with node_thr: per A row, zeroed before the launch, keys in its list
+    // with node_thr: [row][out_stride] the row's out_count keys, in no order;
+    // else [row][range][W] ascending, 0 = empty.  A key is
+    // (ordered score << 32) | tie hash
+    unsigned long long *out_key;
+    unsigned *out_pos;             // [row][range][W] (not written with node_thr)
+    int out_stride;                // >= ranges * W
     int *status;
 };
 int tc_supported_width(int w);
@@ -430,7 +437,8 @@ struct TcNodeArgs {
     int fmt;
     void *A;                   // rows x Kp, zeroed here (rows >= nslots: the padding rows too)
     long long rows;
-    unsigned *node_thr;        // the shortlist's per-node bound, zeroed here (may be null)
+    unsigned long long *node_thr;  // the shortlist's per-node bound and key count, zeroed here (may be null)
+    unsigned *node_count;
     float *node_scale;
     float *node_bias;          // sum of the weights of neighbours in a variable's last category
     int *node_box;
@@ -443,9 +451,14 @@ struct TcSelectArgs {
     int maxterms;
     int nslots;
     const float *layers;                 // FP32 flipped layers (exact scores)
-    const unsigned long long *cand_key;  // [slot][ncand]
+    // [slot][ncand] keys and positions, or (cand_count) cand_count[slot] keys
+    // of a row of cand_stride, their positions from the tie hash
+    const unsigned long long *cand_key;
     const unsigned *cand_pos;
     int ncand;                           // ranges x W
+    const unsigned *cand_count = nullptr;
+    int cand_stride = 0;
+    const unsigned *node_seed = nullptr; // with cand_count: the slots' tie seeds
     int S;                               // candidates scored exactly (<= 256)
     int fp64;                            // rank by the FP64 exact score
     const float *ti;

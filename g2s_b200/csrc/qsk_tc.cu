@@ -409,9 +409,10 @@ __global__ void __launch_bounds__(threads_for(W), 1)
             __syncwarp();
         }
         float *scratch = reinterpret_cast<float *>(epi) + e * 32 + lane;   // !LISTS: score j at [j * 32 * EPI_WARPS]
-        u64 root = 0ull;   // the W-th best key
-        float thr = -INFINITY;
-        unsigned g_seen = 0u;   // largest value of the shared bound this thread has read or published
+        u64 root = 0ull;    // this group's W-th best key
+        u64 kb = 0ull;      // the bound to pass: root, or the best W-th of any range seen
+        float thr = -INFINITY;   // its score
+        u64 g_seen = 0ull;  // largest value of the shared bound this thread has read or published
         int i = 0;
         // TI coordinates of the tile's first position
         int x0 = (int)((t_begin * BN) % a.X);
@@ -433,9 +434,9 @@ __global__ void __launch_bounds__(threads_for(W), 1)
             const int pos0 = (int)(t * BN);
             const float s = nscale * (a.pos_scale ? __ldg(a.pos_scale + t) : 1.f);
             if (live && a.node_thr) {
-                const unsigned g = *(volatile unsigned *)(a.node_thr + node);
-                g_seen = g > g_seen ? g : g_seen;
-                if (g) thr = fmaxf(thr, unordered(g));
+                g_seen = max(g_seen, *(volatile u64 *)(a.node_thr + node));
+                kb = max(kb, g_seen);
+                if (kb) thr = unordered((unsigned)(kb >> 32));
             }
 #pragma unroll 1
             for (int c = h; c < BN / 32; c += G) {
@@ -508,16 +509,16 @@ __global__ void __launch_bounds__(threads_for(W), 1)
 #pragma unroll
                 for (int j = 0; j < 32; ++j) cand |= v[j] >= bound ? (1u << j) : 0u;
                 cand &= vmask;
-                // a tie with the W-th best qualifies only with a larger tie hash:
-                // asked here where many positions tie (categorical match counts),
-                // else by the full key below
+                // a tie with the bound qualifies only with a larger tie hash: asked
+                // here where many positions tie (categorical match counts), else
+                // by the full key below
                 const unsigned most = __reduce_max_sync(0xffffffffu, (unsigned)__popc(cand));
                 if (most == 0u) continue;
                 if (most > 4u) {
-                    const float tie = root ? unordered((unsigned)(root >> 32)) : NAN;   // (equals no score)
+                    const float tie = kb ? thr : NAN;   // (equals no score)
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
-                        if (v[j] == tie && tie_hash(nseed, (unsigned)(pc + j)) <= (unsigned)root) cand &= ~(1u << j);
+                        if (v[j] == tie && tie_hash(nseed, (unsigned)(pc + j)) <= (unsigned)kb) cand &= ~(1u << j);
                 }
                 if constexpr (!LISTS) {
                     // inserted in rounds, every lane its next candidate
@@ -528,10 +529,11 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                         const int j = __ffs(cand) - 1;
                         cand &= cand - 1u;
                         const u64 key = (u64)ordered(scratch[j * 32 * EPI_WARPS]) << 32 | tie_hash(nseed, (unsigned)(pc + j));
-                        if (key <= root) continue;
+                        if (key <= kb) continue;
                         sorted_insert<R>(rk, key);
                         root = rk[0];
-                        thr = root ? fmaxf(thr, unordered((unsigned)(root >> 32))) : thr;
+                        kb = max(kb, root);
+                        thr = kb ? unordered((unsigned)(kb >> 32)) : thr;
                     }
                 } else {
                     // the lanes' next candidates, one list after the other: the key
@@ -553,7 +555,7 @@ __global__ void __launch_bounds__(threads_for(W), 1)
 #pragma unroll
                             for (int u = 0; u < 2; ++u) t2[u] = (j & 8) ? t4[2 * u + 1] : t4[2 * u];
                             key = (u64)ordered((j & 16) ? t2[1] : t2[0]) << 32 | tie_hash(nseed, (unsigned)(pc + j));
-                            if (key <= root) key = 0ull;
+                            if (key <= kb) key = 0ull;
                         }
                         unsigned act = __ballot_sync(0xffffffffu, key != 0ull);
                         while (act) {
@@ -570,7 +572,8 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                             const unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : ~0u);
                             if (lane == l) {
                                 root = (u64)hi << 32 | lo;
-                                thr = root ? fmaxf(thr, unordered(hi)) : thr;
+                                kb = max(kb, root);
+                                thr = kb ? unordered((unsigned)(kb >> 32)) : thr;
                             }
                         }
                     }
@@ -581,9 +584,9 @@ __global__ void __launch_bounds__(threads_for(W), 1)
             // bound only grows, so a minimum at or below the value last read
             // changes nothing: skipping it spares the bound's few cache lines,
             // which every CTA of the launch reads and updates, most updates
-            if (live && root && a.node_thr && (unsigned)(root >> 32) > g_seen) {
-                atomicMax(a.node_thr + node, (unsigned)(root >> 32));
-                g_seen = (unsigned)(root >> 32);
+            if (live && a.node_thr && root > g_seen) {
+                atomicMax(a.node_thr + node, root);
+                g_seen = root;
             }
             tc_fence_before();
             __syncwarp();
@@ -607,7 +610,18 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                 // ascending against descending: the larger of each pair are the best
                 const u64 u = warp_sort(epi[r * LIST_STRIDE + lane], lane, 2, true);
                 const u64 w = warp_sort(epi[(BM + r) * LIST_STRIDE + lane], lane, 2, false);
-                const u64 key = warp_sort(u > w ? u : w, lane, 32, true);
+                u64 key = u > w ? u : w;
+                if (a.node_thr) {
+                    const u64 bound = *(volatile u64 *)(a.node_thr + nd);
+                    const unsigned keep = __ballot_sync(0xffffffffu, key != 0ull && key >= bound);
+                    unsigned at = 0u;
+                    if (lane == 0 && keep) at = atomicAdd(a.out_count + nd, (unsigned)__popc(keep));
+                    at = __shfl_sync(0xffffffffu, at, 0);
+                    if ((keep >> lane) & 1u)
+                        a.out_key[(size_t)nd * a.out_stride + at + __popc(keep & ((1u << lane) - 1u))] = key;
+                    continue;
+                }
+                key = warp_sort(key, lane, 32, true);
                 const size_t o = ((size_t)nd * a.ranges + range) * W + lane;
                 a.out_key[o] = key;
                 a.out_pos[o] = key_position(key, a.node_seed ? a.node_seed[nd] : 0u);
@@ -626,11 +640,25 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                         if (key <= rk[0]) break;
                         sorted_insert<R>(rk, key);
                     }
-                const size_t o = ((size_t)node * a.ranges + range) * W;
+                if (a.node_thr) {
+                    // what the bound, as it stands now, lets through
+                    const u64 bound = max(*(volatile u64 *)(a.node_thr + node), 1ull);
+                    unsigned keep = 0u;
 #pragma unroll
-                for (int f = 0; f < R; ++f) {
-                    a.out_key[o + f] = rk[f];
-                    a.out_pos[o + f] = key_position(rk[f], nseed);
+                    for (int f = 0; f < R; ++f) keep += rk[f] >= bound ? 1u : 0u;
+                    if (keep) {
+                        u64 *o = a.out_key + (size_t)node * a.out_stride + atomicAdd(a.out_count + node, keep);
+#pragma unroll
+                        for (int f = 0; f < R; ++f)   // ascending: the last `keep`
+                            if (f >= R - (int)keep) o[f - (R - (int)keep)] = rk[f];
+                    }
+                } else {
+                    const size_t o = ((size_t)node * a.ranges + range) * W;
+#pragma unroll
+                    for (int f = 0; f < R; ++f) {
+                        a.out_key[o + f] = rk[f];
+                        a.out_pos[o + f] = key_position(rk[f], nseed);
+                    }
                 }
             }
         }
@@ -1037,11 +1065,18 @@ __global__ void k_tc_nodes(TcNodeArgs A) {
     tc_nodes_warp(A, int((blockIdx.x * blockDim.x + threadIdx.x) >> 5), int(threadIdx.x & 31));
 }
 
+// the part of a term's scale that no layer value enters: v^2 w of a
+// continuous neighbour (its b is 2 w v), w of a categorical one
+__device__ __forceinline__ double term_scale(const Term &T) {
+    if (T.op == OP_SQLIN) return ((double)T.b * (double)T.b) / (-4.0 * (double)T.a);
+    return T.op == OP_EQ ? (double)T.a : 0.0;
+}
+
 // exact score of one candidate from its staged layer values xs[t] (term t's
 // gathered value), in the plain map's term order (FP32, bit-identical to
-// k_map_records) and in FP64; `scale` is the term scale
-__device__ __forceinline__ void exact_score_staged(const Term *__restrict__ tm, int nt, const float *xs, float &s32,
-                                                   double &s64, double &scale) {
+// k_map_records) and in FP64; `scale` is the term scale, ts[t] = term_scale
+__device__ __forceinline__ void exact_score_staged(const Term *__restrict__ tm, int nt, const float *xs,
+                                                   const double *ts, float &s32, double &s64, double &scale) {
     float acc = 0.f;
     double a64 = 0.0, sc = 0.0;
     for (int t = 0; t < nt; ++t) {
@@ -1051,11 +1086,11 @@ __device__ __forceinline__ void exact_score_staged(const Term *__restrict__ tm, 
             acc = __fmaf_rn(T.a, __fmul_rn(x, x), acc);
             acc = __fmaf_rn(T.b, x, acc);
             a64 += (double)T.a * ((double)x * (double)x) + (double)T.b * (double)x;
-            sc += -(double)T.a * ((double)x * (double)x) + ((double)T.b * (double)T.b) / (-4.0 * (double)T.a);
+            sc += -(double)T.a * ((double)x * (double)x) + ts[t];
         } else if (T.op == OP_EQ) {
             acc = (x == T.b) ? __fadd_rn(acc, T.a) : acc;
             a64 += (x == T.b) ? (double)T.a : 0.0;
-            sc += (double)T.a;
+            sc += ts[t];
         } else if (T.op == OP_LIN) {
             acc = __fmaf_rn(T.a, x, acc);
             a64 += (double)T.a * (double)x;
@@ -1081,11 +1116,11 @@ __device__ __forceinline__ void exact_score(const Term *__restrict__ tm, int nt,
             acc = __fmaf_rn(T.a, __fmul_rn(x, x), acc);
             acc = __fmaf_rn(T.b, x, acc);
             a64 += (double)T.a * ((double)x * (double)x) + (double)T.b * (double)x;
-            sc += -(double)T.a * ((double)x * (double)x) + ((double)T.b * (double)T.b) / (-4.0 * (double)T.a);
+            sc += -(double)T.a * ((double)x * (double)x) + term_scale(T);
         } else if (T.op == OP_EQ) {
             acc = (x == T.b) ? __fadd_rn(acc, T.a) : acc;
             a64 += (x == T.b) ? (double)T.a : 0.0;
-            sc += (double)T.a;
+            sc += term_scale(T);
         } else if (T.op == OP_LIN) {
             acc = __fmaf_rn(T.a, x, acc);
             a64 += (double)T.a * (double)x;
@@ -1099,6 +1134,7 @@ __device__ __forceinline__ void exact_score(const Term *__restrict__ tm, int nt,
 
 constexpr int SEL_WARPS = 4;
 constexpr int SEL_CAND = 768;    // candidates per slot staged in shared memory
+constexpr int SEL_TERMS = 96;    // terms per slot staged there
 constexpr int SEL_CPL = 8;       // shortlist entries per lane: at most 256 re-scored
 
 // one warp per tensor slot: the S best candidates by approximate key, their
@@ -1107,28 +1143,37 @@ constexpr int SEL_CPL = 8;       // shortlist entries per lane: at most 256 re-s
 __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
     __shared__ unsigned long long skey[SEL_WARPS][SEL_CAND];
     __shared__ unsigned spos[SEL_WARPS][SEL_CAND];
-    __shared__ Term sterm[SEL_WARPS][96];
-    griddep_wait();   // launched programmatically after the shortlist
+    __shared__ Term sterm[SEL_WARPS][SEL_TERMS];
+    __shared__ double sscale[SEL_WARPS][SEL_TERMS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x * SEL_WARPS + w;
     if (b >= A.nslots) return;
+    // The slot and its terms come from the kernel before the shortlist, which
+    // had completed when the shortlist's blocks let this grid launch: they are
+    // read while the shortlist runs
     const Slot s = A.slots[b];
     const Geom &g = A.g;
     const int nt = s.nterms;
     const Term *tm = A.terms + (long long)b * A.maxterms;
-    const bool small = nt <= 96;
+    const bool small = nt <= SEL_TERMS;
     if (small)
-        for (int t = lane; t < nt; t += 32) sterm[w][t] = tm[t];
-    const int nc = A.ncand;
+        for (int t = lane; t < nt; t += 32) {
+            sterm[w][t] = tm[t];
+            sscale[w][t] = term_scale(tm[t]);
+        }
+    griddep_wait();   // launched programmatically after the shortlist
     // largest key a position outside the final shortlist can have by the
     // proposal (learned mode): the best of the ranges' heap minima (a full
     // heap's minimum bounds what that range left out)
     unsigned long long lout = 0ull;
-    for (int c = lane; c < nc; c += 32) {
-        const unsigned long long k = A.cand_key[(long long)b * nc + c];
-        skey[w][c] = k;
-        spos[w][c] = A.cand_pos[(long long)b * nc + c];
-    }
+    const int nc = A.cand_count ? (int)min(A.cand_count[b], (unsigned)A.cand_stride) : A.ncand;
+    const unsigned long long *keys = A.cand_key + (long long)b * (A.cand_count ? A.cand_stride : nc);
+    const bool staged = nc <= SEL_CAND;   // (lists are rarely longer)
+    if (staged)
+        for (int c = lane; c < nc; c += 32) {
+            skey[w][c] = keys[c];
+            if (!A.cand_count) spos[w][c] = A.cand_pos[(long long)b * nc + c];
+        }
     __syncwarp();
     if (A.fallback && A.conf_z > 0.f && A.range_w > 0) {
         for (int r = lane; r * A.range_w < nc; r += 32) {
@@ -1140,7 +1185,8 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
         for (int o = 16; o > 0; o >>= 1) lout = max(lout, __shfl_xor_sync(0xffffffffu, lout, o));
     }
     const Term *tt = small ? sterm[w] : tm;
-    // the S largest keys (S rounds of warp argmax); lane r keeps round r and r+32
+    // the S largest keys, in rounds; lane r keeps round r and r+32.  Keys are
+    // distinct (a node's tie hashes are): the next is the largest below the last
     unsigned long long mykey[SEL_CPL];
     unsigned mypos[SEL_CPL];
 #pragma unroll
@@ -1149,38 +1195,81 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
         mypos[h] = 0u;
     }
     int nsel = 0;
-    for (int r = 0; r < A.S; ++r) {
-        unsigned long long bk = 0ull;
-        int bi = -1;
-        for (int c = lane; c < nc; c += 32) {
-            const unsigned long long k = skey[w][c];
-            if (k > bk) {
-                bk = k;
-                bi = c;
+    if (nc <= 32) {
+        // one key per lane
+        unsigned long long mine = lane < nc ? skey[w][lane] : 0ull;
+        for (int r = 0; r < A.S; ++r) {
+            const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(mine >> 32));
+            if (hi == 0u) break;
+            const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(mine >> 32) == hi ? (unsigned)mine : 0u);
+            const unsigned long long bk = (unsigned long long)hi << 32 | lo;
+            const int src = __ffs(__ballot_sync(0xffffffffu, mine == bk)) - 1;
+            if (lane == r) {
+                mykey[0] = bk;
+                mypos[0] = A.cand_count ? tie_position(A.node_seed[b], lo) : spos[w][src];
             }
+            if (lane == src) mine = 0ull;
+            ++nsel;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long ok = __shfl_xor_sync(0xffffffffu, bk, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ok > bk || (ok == bk && oi > bi)) {
-                bk = ok;
-                bi = oi;
+        if (lane < nc) skey[w][lane] = mine;
+        __syncwarp();
+    } else if (A.cand_count) {
+        unsigned long long last = ~0ull;
+        for (int r = 0; r < A.S; ++r) {
+            unsigned long long bk = 0ull;
+            for (int c = lane; c < nc; c += 32) {
+                const unsigned long long k = staged ? skey[w][c] : keys[c];
+                if (k < last && k > bk) bk = k;
             }
-        }
-        if (bk == 0ull) break;
-        if (lane == (r & 31)) {
 #pragma unroll
-            for (int h = 0; h < SEL_CPL; ++h)
-                if (h == (r >> 5)) {
-                    mykey[h] = bk;
-                    mypos[h] = spos[w][bi];
+            for (int o = 16; o > 0; o >>= 1) bk = max(bk, __shfl_xor_sync(0xffffffffu, bk, o));
+            if (bk == 0ull) break;
+            last = bk;
+            if (lane == (r & 31)) {
+#pragma unroll
+                for (int h = 0; h < SEL_CPL; ++h)
+                    if (h == (r >> 5)) {
+                        mykey[h] = bk;
+                        mypos[h] = tie_position(A.node_seed[b], (unsigned)bk);
+                    }
+            }
+            ++nsel;
+        }
+        __syncwarp();
+    } else {
+        for (int r = 0; r < A.S; ++r) {
+            unsigned long long bk = 0ull;
+            int bi = -1;
+            for (int c = lane; c < nc; c += 32) {
+                const unsigned long long k = skey[w][c];
+                if (k > bk) {
+                    bk = k;
+                    bi = c;
                 }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long ok = __shfl_xor_sync(0xffffffffu, bk, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (ok > bk || (ok == bk && oi > bi)) {
+                    bk = ok;
+                    bi = oi;
+                }
+            }
+            if (bk == 0ull) break;
+            if (lane == (r & 31)) {
+#pragma unroll
+                for (int h = 0; h < SEL_CPL; ++h)
+                    if (h == (r >> 5)) {
+                        mykey[h] = bk;
+                        mypos[h] = spos[w][bi];
+                    }
+            }
+            __syncwarp();
+            if (lane == 0) skey[w][bi] = 0ull;
+            __syncwarp();
+            ++nsel;
         }
-        __syncwarp();
-        if (lane == 0) skey[w][bi] = 0ull;
-        __syncwarp();
-        ++nsel;
     }
     if (A.fallback && A.conf_z > 0.f) {
         unsigned long long nk = 0ull;
@@ -1234,7 +1323,7 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
             __syncwarp();
             for (int h = 0; h < SEL_CPL; ++h) {
                 const int r = h * 32 + lane;
-                if (r >= r0 && r < r1) exact_score_staged(tt, nt, xs + (r - r0) * nt, e32[h], e64[h], esc[h]);
+                if (r >= r0 && r < r1) exact_score_staged(tt, nt, xs + (r - r0) * nt, sscale[w], e32[h], e64[h], esc[h]);
             }
             __syncwarp();
         }
@@ -1480,7 +1569,7 @@ cudaError_t launch_tc_nodes(const TcNodeArgs &a, cudaStream_t st) {
 }
 
 cudaError_t launch_tc_select(const TcSelectArgs &a, cudaStream_t st) {
-    if (a.ncand > SEL_CAND || a.S > 32 * SEL_CPL) return cudaErrorInvalidValue;
+    if ((!a.cand_count && a.ncand > SEL_CAND) || a.S > 32 * SEL_CPL) return cudaErrorInvalidValue;
     return launch_pdl(k_tc_select, dim3((unsigned)((a.nslots + SEL_WARPS - 1) / SEL_WARPS)), dim3(32 * SEL_WARPS), 0,
                       st, a);
 }

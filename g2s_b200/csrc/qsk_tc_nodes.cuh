@@ -44,7 +44,10 @@ __device__ __forceinline__ void tc_nodes_warp(const TcNodeArgs &A, const int war
         __syncwarp();
     }
     if (warp >= A.nslots) return;
-    if (A.node_thr && lane == 0) A.node_thr[warp] = 0u;
+    if (A.node_thr && lane == 0) {
+        A.node_thr[warp] = 0ull;
+        A.node_count[warp] = 0u;
+    }
     const int i = A.nodes[warp];
     const unsigned cell = A.path[A.begin + i];
     const int cnt = A.nb_count[i];
