@@ -1098,7 +1098,7 @@ struct Step {
     bool few = true;    // HASH: a node of the step may have fewer than K positions (it takes the replay)
 };
 
-int tc_step(qsk_sim *s, const Step &st, bool teacher);
+int tc_step(qsk_sim *s, const Step &st, bool teacher, bool after_select);
 constexpr int TC_LIST = 1536;   // keys a node's bounded shortlist may hold (ranges x W)
 bool tc_bounded(const qsk_sim *s) { return s->tc_S <= s->tc_W && s->topt.mode != 3; }
 
@@ -1218,17 +1218,29 @@ int sim_batches(qsk_sim *s, const std::vector<Step> &steps, bool teacher) {
     // starts when both streams have finished the one before.
     int cur_level = -1, side_level = -1;
     bool side_pending = false;
-    for (const Step &step : steps) {
+    bool after_select = false;   // the last operation on st is a tensor step's select
+    for (size_t si = 0; si < steps.size(); ++si) {
+        const Step &step = steps[si];
         if (step.level >= 0 && step.level != cur_level) {
             if (side_pending) CK(cudaStreamWaitEvent(s->st, s->ev_side, 0));
+            if (side_pending) after_select = false;
             side_pending = false;
-            CK(cudaEventRecord(s->ev_level, s->st));
+            // a level with exact-map steps: they wait for its start
+            bool has_side = false;
+            for (size_t q = si; q < steps.size() && steps[q].level == step.level; ++q)
+                has_side |= steps[q].kind == STEP_HASH;
+            if (has_side) {
+                CK(cudaEventRecord(s->ev_level, s->st));
+                after_select = false;
+            }
             cur_level = step.level;
         }
         if (step.kind == STEP_TENSOR) {
-            if ((rc = tc_step(s, step, teacher)) != QSK_OK) return rc;
+            if ((rc = tc_step(s, step, teacher, after_select)) != QSK_OK) return rc;
+            after_select = s->topt.mode != 3;   // (the learned proposal's steps end on the host)
             continue;
         }
+        after_select = false;
         const bool side = step.kind == STEP_HASH && step.level >= 0;
         cudaStream_t ws = side ? s->st2 : s->st;
         if (side && side_level != step.level) {
@@ -1818,7 +1830,7 @@ int exact_nodes(qsk_sim *s, const int *nodes, int count, bool teacher) {
     return QSK_OK;
 }
 
-int tc_step(qsk_sim *s, const Step &step, bool teacher) {
+int tc_step(qsk_sim *s, const Step &step, bool teacher, bool after_select) {
     const Geom &g = s->ti->g;
     const int B = step.B;
     const int elem = s->tc_fmt == 0 ? 2 : 1;
@@ -1922,7 +1934,7 @@ int tc_step(qsk_sim *s, const Step &step, bool teacher) {
     // the exact terms and the node rows in one launch (learned: the rows of
     // A come from the encoder, after the terms)
     if (learned) CK(launch_tc_nodes(na, s->st));
-    else CK(launch_prep_tc_nodes(pa, na, s->st));
+    else CK(launch_prep_tc_nodes(pa, na, after_select && !s->profiling, s->st));
     if (s->profiling) CK(cudaEventRecord(tc_event(s), s->st));
     // GEMM shortlist: enough position ranges to fill the GPU.  With a
     // shortlist of at most W the shared bound makes the ranges' union hold the

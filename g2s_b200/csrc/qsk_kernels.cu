@@ -514,6 +514,9 @@ __device__ __forceinline__ void prep_sim_warp(const SimPrepArgs &A, const int wa
     const int cnt = A.nb_count[i];
     const int nd = A.g.nd;
     const NodeGeom ng = node_geometry(A, i, cell, lane);
+    // launched programmatically (k_prep_tc_nodes): what is read above follows
+    // from the path alone; simulated values, slots and terms come below
+    griddep_wait();
     Slot s;
     s.node = i;
     s.cell = cell;
@@ -2652,12 +2655,14 @@ cudaError_t launch_levels(const LevelArgs &a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_prep_tc_nodes(const SimPrepArgs &p, const TcNodeArgs &a, cudaStream_t st) {
+cudaError_t launch_prep_tc_nodes(const SimPrepArgs &p, const TcNodeArgs &a, bool after_select, cudaStream_t st) {
     if (!a.A || a.nslots != p.nslots || a.rows < a.nslots || (a.Kp * (a.fmt == 1 ? 1 : 2)) % 16 != 0)
         return cudaErrorInvalidValue;
     const long long prep_blocks = ((long long)p.nslots * 32 + 255) / 256;
     const long long node_blocks = (a.rows * 32 + 255) / 256;
-    k_prep_tc_nodes<<<(unsigned)(prep_blocks + node_blocks), 256, 0, st>>>(p, a, (unsigned)prep_blocks);
+    const dim3 grid((unsigned)(prep_blocks + node_blocks));
+    if (after_select) return launch_pdl(k_prep_tc_nodes, grid, dim3(256), 0, st, p, a, (unsigned)prep_blocks);
+    k_prep_tc_nodes<<<grid, 256, 0, st>>>(p, a, (unsigned)prep_blocks);
     return cudaGetLastError();
 }
 

@@ -1135,11 +1135,13 @@ __device__ __forceinline__ void exact_score(const Term *__restrict__ tm, int nt,
 constexpr int SEL_WARPS = 4;
 constexpr int SEL_CAND = 768;    // candidates per slot staged in shared memory
 constexpr int SEL_TERMS = 96;    // terms per slot staged there
-constexpr int SEL_CPL = 8;       // shortlist entries per lane: at most 256 re-scored
+constexpr int SEL_CPL = 8;       // shortlist entries per lane at most: 256 re-scored
 
 // one warp per tensor slot: the S best candidates by approximate key, their
 // exact scores, the node's k best by exact score (ties by the key's hash),
 // the draw and the write-back
+// CPL: shortlist entries per lane (S <= 32 CPL)
+template <int CPL>
 __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
     __shared__ unsigned long long skey[SEL_WARPS][SEL_CAND];
     __shared__ unsigned spos[SEL_WARPS][SEL_CAND];
@@ -1147,7 +1149,10 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
     __shared__ double sscale[SEL_WARPS][SEL_TERMS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x * SEL_WARPS + w;
-    if (b >= A.nslots) return;
+    if (b >= A.nslots) {
+        griddep_wait();   // (a block counts as having let the next grid launch once its warps have left)
+        return;
+    }
     // The slot and its terms come from the kernel before the shortlist, which
     // had completed when the shortlist's blocks let this grid launch: they are
     // read while the shortlist runs
@@ -1162,6 +1167,7 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
             sscale[w][t] = term_scale(tm[t]);
         }
     griddep_wait();   // launched programmatically after the shortlist
+    griddep_launch(); // ... and the next level's rows of A may be cleared: the shortlist has completed
     // largest key a position outside the final shortlist can have by the
     // proposal (learned mode): the best of the ranges' heap minima (a full
     // heap's minimum bounds what that range left out)
@@ -1187,10 +1193,10 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
     const Term *tt = small ? sterm[w] : tm;
     // the S largest keys, in rounds; lane r keeps round r and r+32.  Keys are
     // distinct (a node's tie hashes are): the next is the largest below the last
-    unsigned long long mykey[SEL_CPL];
-    unsigned mypos[SEL_CPL];
+    unsigned long long mykey[CPL];
+    unsigned mypos[CPL];
 #pragma unroll
-    for (int h = 0; h < SEL_CPL; ++h) {
+    for (int h = 0; h < CPL; ++h) {
         mykey[h] = 0ull;
         mypos[h] = 0u;
     }
@@ -1227,7 +1233,7 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
             last = bk;
             if (lane == (r & 31)) {
 #pragma unroll
-                for (int h = 0; h < SEL_CPL; ++h)
+                for (int h = 0; h < CPL; ++h)
                     if (h == (r >> 5)) {
                         mykey[h] = bk;
                         mypos[h] = tie_position(A.node_seed[b], (unsigned)bk);
@@ -1259,7 +1265,7 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
             if (bk == 0ull) break;
             if (lane == (r & 31)) {
 #pragma unroll
-                for (int h = 0; h < SEL_CPL; ++h)
+                for (int h = 0; h < CPL; ++h)
                     if (h == (r >> 5)) {
                         mykey[h] = bk;
                         mypos[h] = spos[w][bi];
@@ -1281,12 +1287,12 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
     // exact scores of the shortlist: the scan index of every candidate, then
     // all (candidate, term) layer values gathered by the whole warp at once
     // into shared memory, then each candidate's term chain from there
-    float e32[SEL_CPL];
-    double e64[SEL_CPL], esc[SEL_CPL];
-    unsigned hsh[SEL_CPL];
-    bool live[SEL_CPL];
+    float e32[CPL];
+    double e64[CPL], esc[CPL];
+    unsigned hsh[CPL];
+    bool live[CPL];
 #pragma unroll
-    for (int h = 0; h < SEL_CPL; ++h) {
+    for (int h = 0; h < CPL; ++h) {
         e32[h] = -INFINITY;
         e64[h] = -INFINITY;
         esc[h] = 0.0;
@@ -1297,7 +1303,8 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
     double errsum = 0.0;
     int errn = 0;
     int *msc = reinterpret_cast<int *>(&spos[w][0]);   // candidate list no longer needed
-    for (int h = 0; h < SEL_CPL; ++h) {
+#pragma unroll
+    for (int h = 0; h < CPL; ++h) {
         const int r = h * 32 + lane;
         if (r >= nsel) continue;
         // natural cell -> scan index of the reference's flipped space (cvtPositionToIndex)
@@ -1316,24 +1323,41 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
     if (per > 0) {
         for (int r0 = 0; r0 < nsel; r0 += per) {
             const int r1 = min(nsel, r0 + per);
-            for (int r = r0; r < r1; ++r) {
-                const long long m = msc[r];
-                for (int t = lane; t < nt; t += 32) xs[(r - r0) * nt + t] = __ldg(A.layers + tt[t].base + m);
+            // all (candidate, term) pairs over the lanes, four loads in flight each
+            int r = r0 + lane / nt, t = lane % nt;
+            const int total = (r1 - r0) * nt;
+            for (int i = lane; i < total; i += 128) {
+                float x[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    x[q] = i + 32 * q < total ? __ldg(A.layers + tt[t].base + msc[r]) : 0.f;
+                    t += 32;
+                    while (t >= nt && r < r1) {
+                        t -= nt;
+                        ++r;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (i + 32 * q < total) xs[i + 32 * q] = x[q];
             }
             __syncwarp();
-            for (int h = 0; h < SEL_CPL; ++h) {
+#pragma unroll
+            for (int h = 0; h < CPL; ++h) {
                 const int r = h * 32 + lane;
                 if (r >= r0 && r < r1) exact_score_staged(tt, nt, xs + (r - r0) * nt, sscale[w], e32[h], e64[h], esc[h]);
             }
             __syncwarp();
         }
     } else {
-        for (int h = 0; h < SEL_CPL; ++h) {
+#pragma unroll
+        for (int h = 0; h < CPL; ++h) {
             const int r = h * 32 + lane;
             if (r < nsel) exact_score(tt, nt, A.layers, (long long)msc[r], e32[h], e64[h], esc[h]);
         }
     }
-    for (int h = 0; h < SEL_CPL; ++h) {
+#pragma unroll
+    for (int h = 0; h < CPL; ++h) {
         const int r = h * 32 + lane;
         if (r >= nsel) continue;
         const float approx = tc::unordered((unsigned)(mykey[h] >> 32));
@@ -1355,18 +1379,17 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
     double kth_score = -INFINITY;   // the K-th best exact score (ranking precision)
     for (int k = 0; k < K && k < nsel; ++k) {
         int bh = -1;
-        for (int h = 0; h < SEL_CPL; ++h) {
-            if (!live[h]) continue;
-            if (bh < 0) {
+        double bv = -INFINITY;
+        unsigned bhs = 0u;
+#pragma unroll
+        for (int h = 0; h < CPL; ++h) {
+            const double v = f64 ? e64[h] : (double)e32[h];
+            if (live[h] && (bh < 0 || v > bv || (v == bv && hsh[h] > bhs))) {
                 bh = h;
-                continue;
+                bv = v;
+                bhs = hsh[h];
             }
-            const bool better = f64 ? (e64[h] > e64[bh] || (e64[h] == e64[bh] && hsh[h] > hsh[bh]))
-                                    : (e32[h] > e32[bh] || (e32[h] == e32[bh] && hsh[h] > hsh[bh]));
-            if (better) bh = h;
         }
-        double bv = bh >= 0 ? (f64 ? e64[bh] : (double)e32[bh]) : -INFINITY;
-        unsigned bhs = bh >= 0 ? hsh[bh] : 0u;
         int bl = bh >= 0 ? lane : -1;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -1385,7 +1408,7 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
         float w320 = 0.f;
         double wsc0 = 0.0;
 #pragma unroll
-        for (int h = 0; h < SEL_CPL; ++h)
+        for (int h = 0; h < CPL; ++h)
             if (h == wh) {
                 wp0 = mypos[h];
                 w320 = e32[h];
@@ -1417,7 +1440,7 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
         int br = 0x7FFFFFFF;
         double bv2 = -INFINITY;
         unsigned bh2 = 0u;
-        for (int h = 0; h < SEL_CPL; ++h) {
+        for (int h = 0; h < CPL; ++h) {
             const int r = h * 32 + lane;
             if (r >= nsel) continue;
             const double v2 = f64 ? e64[h] : (double)e32[h];
@@ -1445,7 +1468,7 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
             // score is below a L_out + b + z sd with high probability; the
             // node is confident when its k-th best exact score clears that
             double n = 0, sl = 0, ss = 0, sll = 0, sls = 0;
-            for (int h = 0; h < SEL_CPL; ++h) {
+            for (int h = 0; h < CPL; ++h) {
                 const int r = h * 32 + lane;
                 if (r >= nsel) continue;
                 const double L = (double)tc::unordered((unsigned)(mykey[h] >> 32));
@@ -1468,7 +1491,7 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
             const double aa = den > 0 ? (n * sls - sl * ss) / den : 0.0;
             const double bb = n > 0 ? (ss - aa * sl) / n : 0.0;
             double r2 = 0;
-            for (int h = 0; h < SEL_CPL; ++h) {
+            for (int h = 0; h < CPL; ++h) {
                 const int r = h * 32 + lane;
                 if (r >= nsel) continue;
                 const double L = (double)tc::unordered((unsigned)(mykey[h] >> 32));
@@ -1483,7 +1506,7 @@ __global__ void __launch_bounds__(32 * SEL_WARPS) k_tc_select(TcSelectArgs A) {
             // the fraction conf_r2 of it for its extrapolation to be trusted
             const double var = n > 1 ? 1.0 : 0.0;
             double tv = 0;
-            for (int h = 0; h < SEL_CPL; ++h) {
+            for (int h = 0; h < CPL; ++h) {
                 const int r = h * 32 + lane;
                 if (r >= nsel) continue;
                 const double v2 = (f64 ? e64[h] : (double)e32[h]) - (n > 0 ? ss / n : 0.0);
@@ -1570,8 +1593,10 @@ cudaError_t launch_tc_nodes(const TcNodeArgs &a, cudaStream_t st) {
 
 cudaError_t launch_tc_select(const TcSelectArgs &a, cudaStream_t st) {
     if ((!a.cand_count && a.ncand > SEL_CAND) || a.S > 32 * SEL_CPL) return cudaErrorInvalidValue;
-    return launch_pdl(k_tc_select, dim3((unsigned)((a.nslots + SEL_WARPS - 1) / SEL_WARPS)), dim3(32 * SEL_WARPS), 0,
-                      st, a);
+    const dim3 grid((unsigned)((a.nslots + SEL_WARPS - 1) / SEL_WARPS)), block(32 * SEL_WARPS);
+    if (a.S <= 32) return launch_pdl(k_tc_select<1>, grid, block, 0, st, a);
+    if (a.S <= 128) return launch_pdl(k_tc_select<4>, grid, block, 0, st, a);
+    return launch_pdl(k_tc_select<SEL_CPL>, grid, block, 0, st, a);
 }
 
 cudaError_t launch_tc_audit(int n, const int *nodes, int K, const float *plain_val, const float *drawn_score,

@@ -9,6 +9,7 @@
 #include <cuda_fp8.h>
 
 #include "qsk_internal.h"
+#include "qsk_pdl.cuh"
 
 namespace qsk {
 namespace {
@@ -44,24 +45,31 @@ __device__ __forceinline__ void tc_nodes_warp(const TcNodeArgs &A, const int war
         __syncwarp();
     }
     if (warp >= A.nslots) return;
-    if (A.node_thr && lane == 0) {
-        A.node_thr[warp] = 0ull;
-        A.node_count[warp] = 0u;
-    }
     const int i = A.nodes[warp];
     const unsigned cell = A.path[A.begin + i];
     const int cnt = A.nb_count[i];
     const int nd = A.nd;
     int mn[QSK_MAXD] = {0, 0, 0, 0}, mx[QSK_MAXD] = {0, 0, 0, 0};
-    float amax = 0.f;
     for (int j = lane; j < cnt; j += 32) {
         const int t = A.nb_tpl[(long long)i * A.n + j];
-        const unsigned nc = A.nb_cell[(long long)i * A.n + j];
         for (int d = 0; d < nd; ++d) {
             const int o = A.tpl[t * nd + d];
             mn[d] = min(mn[d], o);
             mx[d] = max(mx[d], o);
         }
+    }
+    // launched programmatically behind the previous level's select: its row of
+    // A is free then (the shortlist that read it has completed), and what is
+    // read above follows from the path alone; simulated values come below
+    griddep_wait();
+    if (A.node_thr && lane == 0) {
+        A.node_thr[warp] = 0ull;
+        A.node_count[warp] = 0u;
+    }
+    float amax = 0.f;
+    for (int j = lane; j < cnt; j += 32) {
+        const int t = A.nb_tpl[(long long)i * A.n + j];
+        const unsigned nc = A.nb_cell[(long long)i * A.n + j];
         for (int v = 0; v < A.nvar; ++v) {
             const float val = nc == cell ? A.init[(long long)nc * A.nvar + v] : A.state[(long long)nc * A.nvar + v];
             const float w = A.wtab[t * A.nvar + v];
