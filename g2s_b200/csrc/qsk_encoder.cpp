@@ -70,12 +70,11 @@ int enc_gemm(qsk_encoder *e, int M, int N, int K, const float *A, int lda, int t
     if (M <= 0 || N <= 0) return QSK_OK;
     const int kpad = (K + 63) / 64 * 64;
     const long long ar = (M + 127LL) / 128 * 128;
-    const int bn = tc_gemm_bn(N);
+    const int bn = tc_gemm_bn(M, N);
     const long long br = (N + bn - 1LL) / bn * bn;
     QSK_CK(e->pa.ensure(size_t(ar) * kpad));
     QSK_CK(e->pb.ensure(size_t(br) * kpad));
-    QSK_CK(launch_pack_bf16(M, K, A, lda, ta, ar, kpad, e->pa.p, st));
-    QSK_CK(launch_pack_bf16(N, K, B, ldb, tb ? 0 : 1, br, kpad, e->pb.p, st));
+    QSK_CK(launch_pack_bf16({M, K, A, lda, ta, ar, kpad, e->pa.p}, {N, K, B, ldb, tb ? 0 : 1, br, kpad, e->pb.p}, st));
     TcGemmArgs g;
     g.M = M;
     g.N = N;
@@ -179,7 +178,6 @@ int enc_loss_grad(qsk_encoder *e, int B, float tau) {
     // would swamp; these B x B x 64 products are a small part of a step
     // S = Q P^T
     QSK_CK(launch_sgemm(B, B, ENC_E, Q, ENC_E, 0, P, ENC_E, 1, e->S.p, B, 1.f, 0.f, nullptr, st));
-    QSK_CK(cudaMemsetAsync(e->dS.p, 0, sizeof(float) * size_t(B) * B, st));
     QSK_CK(cudaMemsetAsync(e->loss.p, 0, sizeof(float), st));
     QSK_CK(launch_infonce(B, tau, e->S.p, e->dS.p, e->loss.p, st));
     // dQ = dS P, dP = dS^T Q
@@ -262,7 +260,7 @@ int qsk_gemm_bf16(int device, int M, int N, int K, const float *A, const float *
         cudaStream_t s;
         ~StreamGuard() { cudaStreamDestroy(s); }
     } sg{st};
-    const int kpad = (K + 63) / 64 * 64, bn = tc_gemm_bn(N);
+    const int kpad = (K + 63) / 64 * 64, bn = tc_gemm_bn(M, N);
     const long long ar = (M + 127LL) / 128 * 128, br = (N + bn - 1LL) / bn * bn;
     DBuf<float> a, b, bi, c;
     DBuf<unsigned short> pa, pb;
@@ -275,8 +273,7 @@ int qsk_gemm_bf16(int device, int M, int N, int K, const float *A, const float *
     QSK_CK(pb.alloc(size_t(br) * kpad));
     QSK_CK(status.alloc(1));
     QSK_CK(cudaMemsetAsync(status.p, 0, sizeof(int), st));
-    QSK_CK(launch_pack_bf16(M, K, a.p, K, 0, ar, kpad, pa.p, st));
-    QSK_CK(launch_pack_bf16(N, K, b.p, K, 0, br, kpad, pb.p, st));
+    QSK_CK(launch_pack_bf16({M, K, a.p, K, 0, ar, kpad, pa.p}, {N, K, b.p, K, 0, br, kpad, pb.p}, st));
     TcGemmArgs g;
     g.M = M;
     g.N = N;

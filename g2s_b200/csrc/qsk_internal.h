@@ -374,7 +374,7 @@ int tc_supported_width(int w);
 // p_rows % 256 == 0, k_elems * element size % 128 == 0
 // C[M x N] = A * B^T (+ bias) on the tensor cores: A (a_rows x kpad) and B
 // (b_rows x kpad) BF16 K-major, a_rows a multiple of 128, b_rows of the N
-// tile (tc_gemm_bn(N)), kpad of 64, padding zero; C FP32 row-major (ldc)
+// tile (tc_gemm_bn(M, N)), kpad of 64, padding zero; C FP32 row-major (ldc)
 struct TcGemmArgs {
     int M = 0, N = 0, kpad = 0;
     float *C = nullptr;
@@ -382,7 +382,7 @@ struct TcGemmArgs {
     const float *bias = nullptr;
     int *status = nullptr;   // DEV_TC_WAIT when a wait ran out
 };
-int tc_gemm_bn(int N);
+int tc_gemm_bn(int M, int N);
 cudaError_t launch_tc_gemm(const void *a_bf16, long long a_rows, const void *b_bf16, long long b_rows,
                            const TcGemmArgs &g, cudaStream_t st);
 cudaError_t launch_tc_shortlist(int kind, int W, const void *a_mat, long long a_rows, const void *p_mat,
@@ -551,8 +551,18 @@ cudaError_t launch_adam(long long n, float *w, const float *g, float *m, float *
 cudaError_t launch_feat_nodes(const FeatArgs &a, cudaStream_t st);
 // rows_pad x kpad BF16 copy of a rows x cols FP32 matrix (tr: of its
 // transpose, src then cols x rows), zero-padded; both pads multiples of 32
-cudaError_t launch_pack_bf16(int rows, int cols, const float *src, long long ld, int tr, long long rows_pad, int kpad,
-                             void *dst, cudaStream_t st);
+struct PackArgs {
+    int rows = 0, cols = 0;
+    const float *src = nullptr;
+    long long ld = 0;
+    int tr = 0;
+    long long rows_pad = 0;
+    int kpad = 0;
+    void *dst = nullptr;
+};
+// the two operands of a launch_tc_gemm, which may follow as a programmatic
+// dependent
+cudaError_t launch_pack_bf16(const PackArgs &a, const PackArgs &b, cudaStream_t st);
 cudaError_t launch_feat_cells(const FeatArgs &a, cudaStream_t st);
 cudaError_t launch_to_bf16(long long n, const float *x, uint16_t *y, cudaStream_t st);
 cudaError_t launch_gather_rows(int n, int cols, const int *idx, const float *src, float *dst, cudaStream_t st);

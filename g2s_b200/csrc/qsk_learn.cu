@@ -23,60 +23,95 @@
 #include <cstdint>
 
 #include "qsk_internal.h"
+#include "qsk_pdl.cuh"
 
 namespace qsk {
 namespace {
 
-constexpr int GT = 64;       // GEMM tile (rows and columns)
-constexpr int GK = 16;       // GEMM K step
-constexpr int GTHREADS = 256;
-
 // C[M x N] = alpha * op(A)[M x K] * op(B)[K x N] + beta * C (+ bias[n]),
-// op(X) = X or X^T; row-major with leading dimensions.  64 x 64 tiles, each
-// thread 4 x 4 outputs.
-__global__ void __launch_bounds__(GTHREADS) k_sgemm(int M, int N, int K, const float *__restrict__ A, int lda, int ta,
-                                                    const float *__restrict__ B, int ldb, int tb, float *__restrict__ C,
-                                                    int ldc, float alpha, float beta, const float *__restrict__ bias) {
-    __shared__ float As[GK][GT + 1];
-    __shared__ float Bs[GK][GT + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int row0 = blockIdx.y * GT, col0 = blockIdx.x * GT;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += GK) {
-        for (int i = threadIdx.x; i < GK * GT; i += GTHREADS) {
-            const int kk = i / GT, mm = i % GT;
+// op(X) = X or X^T; row-major with leading dimensions.  TM x TN tiles, K in
+// steps of TK whose next one is read into registers while the last is
+// multiplied, each thread RM x RN outputs of one ascending chain over K (the
+// tile does not enter the result).  64 x 64 tiles where they fill the GPU;
+// 32 x 16 where N is one tile wide: dS P of 1,024 pairs (N = 64, K = 1,024)
+// is 128 CTAs instead of 16; the two such products and S of a gradient took
+// 287 us, now 50.
+template <int TM, int TN, int TK, int RM, int RN>
+__global__ void __launch_bounds__((TM / RM) * (TN / RN))
+    k_sgemm(int M, int N, int K, const float *__restrict__ A, int lda, int ta, const float *__restrict__ B, int ldb,
+            int tb, float *__restrict__ C, int ldc, float alpha, float beta, const float *__restrict__ bias) {
+    constexpr int NT = (TM / RM) * (TN / RN);
+    constexpr int LA = TM * TK / NT, LB = TN * TK / NT;   // elements a thread stages
+    static_assert(TM * TK % NT == 0 && TN * TK % NT == 0, "whole tiles per thread");
+    __shared__ float As[TK][TM + 1];
+    __shared__ float Bs[TK][TN + 1];
+    const int tid = threadIdx.x;
+    const int tx = tid % (TN / RN), ty = tid / (TN / RN);
+    const int row0 = blockIdx.y * TM, col0 = blockIdx.x * TN;
+    // a thread's elements run along the operand's contiguous dimension
+    auto a_at = [&](int i, int &kk, int &mm) {
+        kk = ta ? i / TM : i % TK;
+        mm = ta ? i % TM : i / TK;
+    };
+    auto b_at = [&](int i, int &kk, int &mm) {
+        kk = tb ? i % TK : i / TN;
+        mm = tb ? i / TK : i % TN;
+    };
+    float ra[LA], rb[LB];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < LA; ++q) {
+            int kk, mm;
+            a_at(tid + q * NT, kk, mm);
             const int r = row0 + mm, k = k0 + kk;
-            float av = 0.f;
-            if (r < M && k < K) av = ta ? A[(long long)k * lda + r] : A[(long long)r * lda + k];
-            As[kk][mm] = av;
-            const int c = col0 + mm;
-            float bv = 0.f;
-            if (c < N && k < K) bv = tb ? B[(long long)c * ldb + k] : B[(long long)k * ldb + c];
-            Bs[kk][mm] = bv;
+            ra[q] = (r < M && k < K) ? (ta ? A[(long long)k * lda + r] : A[(long long)r * lda + k]) : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < LB; ++q) {
+            int kk, mm;
+            b_at(tid + q * NT, kk, mm);
+            const int c = col0 + mm, k = k0 + kk;
+            rb[q] = (c < N && k < K) ? (tb ? B[(long long)c * ldb + k] : B[(long long)k * ldb + c]) : 0.f;
+        }
+    };
+    float acc[RM][RN] = {};
+    fetch(0);
+    for (int k0 = 0; k0 < K; k0 += TK) {
+#pragma unroll
+        for (int q = 0; q < LA; ++q) {
+            int kk, mm;
+            a_at(tid + q * NT, kk, mm);
+            As[kk][mm] = ra[q];
+        }
+#pragma unroll
+        for (int q = 0; q < LB; ++q) {
+            int kk, mm;
+            b_at(tid + q * NT, kk, mm);
+            Bs[kk][mm] = rb[q];
         }
         __syncthreads();
+        if (k0 + TK < K) fetch(k0 + TK);
 #pragma unroll
-        for (int kk = 0; kk < GK; ++kk) {
-            float a[4], b[4];
+        for (int kk = 0; kk < TK; ++kk) {
+            float a[RM], b[RN];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                a[u] = As[kk][ty * 4 + u];
-                b[u] = Bs[kk][tx * 4 + u];
-            }
+            for (int u = 0; u < RM; ++u) a[u] = As[kk][ty * RM + u];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int v = 0; v < RN; ++v) b[v] = Bs[kk][tx * RN + v];
 #pragma unroll
-                for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
+            for (int u = 0; u < RM; ++u)
+#pragma unroll
+                for (int v = 0; v < RN; ++v) acc[u][v] = fmaf(a[u], b[v], acc[u][v]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int r = row0 + ty * 4 + u;
+    for (int u = 0; u < RM; ++u) {
+        const int r = row0 + ty * RM + u;
         if (r >= M) continue;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int c = col0 + tx * 4 + v;
+        for (int v = 0; v < RN; ++v) {
+            const int c = col0 + tx * RN + v;
             if (c >= N) continue;
             float x = alpha * acc[u][v];
             if (beta != 0.f) x += beta * C[(long long)r * ldc + c];
@@ -106,41 +141,93 @@ __global__ void k_gelu_back(long long n, const float *__restrict__ pre, float *_
     if (i < n) d[i] *= gelu_grad(pre[i]);
 }
 
-// column sums (bias gradients): out[c] (+)= sum_r d[r][c]
-__global__ void k_colsum(int rows, int cols, const float *__restrict__ d, float *__restrict__ out, int accumulate) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
+// column sums (bias gradients): out[c] (+)= sum_r d[r][c]; a CTA of 32 x 32
+// threads takes 32 columns, thread row y the rows y, y + 32, ..., whose 32
+// sums are added in order (one thread per column over every row: 43 us for
+// 2,048 x 256, the latency of its chain of reads)
+__global__ void __launch_bounds__(1024) k_colsum(int rows, int cols, const float *__restrict__ d,
+                                                 float *__restrict__ out, int accumulate) {
+    __shared__ float part[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int c = blockIdx.x * 32 + tx;
     float s = 0.f;
-    for (int r = 0; r < rows; ++r) s += d[(long long)r * cols + c];
+    if (c < cols) {
+#pragma unroll 8
+        for (int r = ty; r < rows; r += 32) s += d[(long long)r * cols + c];
+    }
+    part[ty][tx] = s;
+    __syncthreads();
+    if (ty != 0 || c >= cols) return;
+    s = part[0][tx];
+    for (int y = 1; y < 32; ++y) s += part[y][tx];
     out[c] = accumulate ? out[c] + s : s;
 }
 
 // symmetric InfoNCE on logits L = S / tau (B x B, positives on the diagonal):
-// loss = (mean_i CE(row i) + mean_j CE(column j)) / 2; writes dS (the
-// gradient with respect to S) and adds the loss to *loss
-__global__ void k_infonce(int B, float tau, const float *__restrict__ S, float *__restrict__ dS, float *loss) {
-    // one warp per row for the row softmax, then one warp per column
-    const int w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+// loss = (mean_i CE(row i) + mean_j CE(column j)) / 2; dS is the gradient
+// with respect to S, written by the rows and added to by the columns
+// (k_infonce_cols, the launch after); the loss is added to *loss
+__global__ void k_infonce_rows(int B, float tau, const float *__restrict__ S, float *__restrict__ dS, float *loss) {
+    // one warp per row
+    const int i = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
-    if (w >= 2 * B) return;
-    const bool col = w >= B;
-    const int i = col ? w - B : w;
-    auto at = [&](int j) { return col ? S[(long long)j * B + i] : S[(long long)i * B + j]; };
+    if (i >= B) return;
+    const float *row = S + (long long)i * B;
     float mx = -INFINITY;
-    for (int j = lane; j < B; j += 32) mx = fmaxf(mx, at(j) / tau);
+    for (int j = lane; j < B; j += 32) mx = fmaxf(mx, row[j] / tau);
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     float se = 0.f;
-    for (int j = lane; j < B; j += 32) se += expf(at(j) / tau - mx);
+    for (int j = lane; j < B; j += 32) se += expf(row[j] / tau - mx);
     for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
     const float lse = mx + logf(se);
     const float scale = 0.5f / (float)B / tau;
     for (int j = lane; j < B; j += 32) {
-        const float p = expf(at(j) / tau - lse);
-        const float g = (p - (j == i ? 1.f : 0.f)) * scale;
-        const long long idx = col ? (long long)j * B + i : (long long)i * B + j;
-        atomicAdd(&dS[idx], g);
+        const float p = expf(row[j] / tau - lse);
+        dS[(long long)i * B + j] = (p - (j == i ? 1.f : 0.f)) * scale;
     }
-    if (lane == 0) atomicAdd(loss, 0.5f * (lse - at(i) / tau) / (float)B);
+    if (lane == 0) atomicAdd(loss, 0.5f * (lse - row[i] / tau) / (float)B);
+}
+// 32 columns per CTA: thread (x, y) takes rows y, y + 32, ... of column x, so
+// that reads run along the rows; the 32 partial results of a column are
+// combined in the order of a warp's xor reduction
+__global__ void __launch_bounds__(1024) k_infonce_cols(int B, float tau, const float *__restrict__ S,
+                                                       float *__restrict__ dS, float *loss) {
+    __shared__ float part[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + tx;
+    const bool in = i < B;
+    float v = -INFINITY;
+    if (in)
+        for (int j = ty; j < B; j += 32) v = fmaxf(v, S[(long long)j * B + i] / tau);
+    part[ty][tx] = v;
+    for (int o = 16; o > 0; o >>= 1) {
+        __syncthreads();
+        const float u = part[ty ^ o][tx];
+        __syncthreads();
+        part[ty][tx] = v = fmaxf(v, u);
+    }
+    const float mx = v;
+    __syncthreads();
+    v = 0.f;
+    if (in)
+        for (int j = ty; j < B; j += 32) v += expf(S[(long long)j * B + i] / tau - mx);
+    part[ty][tx] = v;
+    for (int o = 16; o > 0; o >>= 1) {
+        __syncthreads();
+        const float u = part[ty ^ o][tx];
+        __syncthreads();
+        part[ty][tx] = v = v + u;
+    }
+    if (!in) return;
+    const float lse = mx + logf(v);
+    const float scale = 0.5f / (float)B / tau;
+    for (int j = ty; j < B; j += 32) {
+        const float p = expf(S[(long long)j * B + i] / tau - lse);
+        // the row's part plus the column's, each rounded (no fused product)
+        float *d = dS + (long long)j * B + i;
+        *d = __fadd_rn(*d, __fmul_rn(p - (j == i ? 1.f : 0.f), scale));
+    }
+    if (ty == 0) atomicAdd(loss, 0.5f * (lse - S[(long long)i * B + i] / tau) / (float)B);
 }
 
 __global__ void k_adam(long long n, float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
@@ -331,26 +418,37 @@ __global__ void k_gather_rows(int n, int cols, const int *__restrict__ idx, cons
     for (int c = threadIdx.x; c < cols; c += blockDim.x) d[c] = s[c];
 }
 
-// BF16 operand of the tensor-core GEMM: dst (rows_pad x kpad) element
-// (r, c) = src[r * ld + c] (tr 0) or src[c * ld + r] (tr 1) for r < rows and
-// c < cols, zero elsewhere; 32 x 32 tiles through shared memory, so that
-// reads and writes are coalesced either way
-__global__ void k_pack_bf16(int rows, int cols, const float *__restrict__ src, long long ld, int tr, int kpad,
-                            __nv_bfloat16 *__restrict__ dst) {
+// BF16 operands of a tensor-core GEMM, both in one launch (blocks
+// [0, first) the first): dst (rows_pad x kpad) element (r, c) =
+// src[r * ld + c] (tr 0) or src[c * ld + r] (tr 1) for r < rows and c < cols,
+// zero elsewhere; 32 x 32 tiles through shared memory, so that reads and
+// writes are coalesced either way
+__global__ void k_pack_bf16(PackArgs a, PackArgs b, unsigned first) {
+    griddep_launch();   // the GEMM (a programmatic successor) may begin launching
     __shared__ float t[32][33];
-    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+    const bool second = blockIdx.x >= first;
+    const int rows = second ? b.rows : a.rows, cols = second ? b.cols : a.cols, kpad = second ? b.kpad : a.kpad;
+    const int tr = second ? b.tr : a.tr;
+    const long long ld = second ? b.ld : a.ld;
+    const float *__restrict__ src = second ? b.src : a.src;
+    __nv_bfloat16 *__restrict__ dst = reinterpret_cast<__nv_bfloat16 *>(second ? b.dst : a.dst);
+    const int block = int(second ? blockIdx.x - first : blockIdx.x), across = kpad / 32;
+    const long long r0 = (long long)(block / across) * 32;
+    const int c0 = block % across * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
     for (int i = ty; i < 32; i += 8) {
         if (!tr) {
-            const int r = r0 + i, c = c0 + tx;
-            t[i][tx] = (r < rows && c < cols) ? src[(long long)r * ld + c] : 0.f;
+            const long long r = r0 + i;
+            const int c = c0 + tx;
+            t[i][tx] = (r < rows && c < cols) ? src[r * ld + c] : 0.f;
         } else {
-            const int c = c0 + i, r = r0 + tx;
+            const int c = c0 + i;
+            const long long r = r0 + tx;
             t[tx][i] = (r < rows && c < cols) ? src[(long long)c * ld + r] : 0.f;
         }
     }
     __syncthreads();
-    for (int i = ty; i < 32; i += 8) dst[(long long)(r0 + i) * kpad + c0 + tx] = __float2bfloat16_rn(t[i][tx]);
+    for (int i = ty; i < 32; i += 8) dst[(r0 + i) * kpad + c0 + tx] = __float2bfloat16_rn(t[i][tx]);
 }
 
 unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -360,8 +458,13 @@ unsigned blocks_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 cudaError_t launch_sgemm(int M, int N, int K, const float *A, int lda, int ta, const float *B, int ldb, int tb, float *C,
                          int ldc, float alpha, float beta, const float *bias, cudaStream_t st) {
     if (M <= 0 || N <= 0) return cudaSuccess;
-    dim3 grid((unsigned)((N + GT - 1) / GT), (unsigned)((M + GT - 1) / GT));
-    k_sgemm<<<grid, GTHREADS, 0, st>>>(M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta, bias);
+    auto tiles = [&](int tm, int tn) { return dim3((unsigned)((N + tn - 1) / tn), (unsigned)((M + tm - 1) / tm)); };
+    const dim3 big = tiles(64, 64);
+    if ((long long)big.x * big.y >= 148)
+        k_sgemm<64, 64, 16, 4, 4><<<big, 256, 0, st>>>(M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta, bias);
+    else
+        k_sgemm<32, 16, 32, 2, 2><<<tiles(32, 16), 128, 0, st>>>(M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta,
+                                                                bias);
     return cudaGetLastError();
 }
 cudaError_t launch_gelu(long long n, const float *pre, float *out, cudaStream_t st) {
@@ -373,11 +476,12 @@ cudaError_t launch_gelu_back(long long n, const float *pre, float *d, cudaStream
     return cudaGetLastError();
 }
 cudaError_t launch_colsum(int rows, int cols, const float *d, float *out, int accumulate, cudaStream_t st) {
-    k_colsum<<<blocks_for(cols, 128), 128, 0, st>>>(rows, cols, d, out, accumulate);
+    k_colsum<<<blocks_for(cols, 32), 1024, 0, st>>>(rows, cols, d, out, accumulate);
     return cudaGetLastError();
 }
 cudaError_t launch_infonce(int B, float tau, const float *S, float *dS, float *loss, cudaStream_t st) {
-    k_infonce<<<blocks_for((long long)2 * B * 32, 256), 256, 0, st>>>(B, tau, S, dS, loss);
+    k_infonce_rows<<<blocks_for((long long)B * 32, 256), 256, 0, st>>>(B, tau, S, dS, loss);
+    k_infonce_cols<<<blocks_for(B, 32), 1024, 0, st>>>(B, tau, S, dS, loss);
     return cudaGetLastError();
 }
 cudaError_t launch_adam(long long n, float *w, const float *g, float *m, float *v, float lr, int t, cudaStream_t st) {
@@ -386,12 +490,18 @@ cudaError_t launch_adam(long long n, float *w, const float *g, float *m, float *
     k_adam<<<blocks_for(n, 256), 256, 0, st>>>(n, w, g, m, v, lr, b1, b2, 1e-8f, c1, c2);
     return cudaGetLastError();
 }
-cudaError_t launch_pack_bf16(int rows, int cols, const float *src, long long ld, int tr, long long rows_pad, int kpad,
-                             void *dst, cudaStream_t st) {
-    if (rows_pad <= 0 || kpad <= 0) return cudaSuccess;
-    if (rows_pad % 32 || kpad % 32 || rows > rows_pad || cols > kpad) return cudaErrorInvalidValue;
-    dim3 grid((unsigned)(kpad / 32), (unsigned)(rows_pad / 32));
-    k_pack_bf16<<<grid, dim3(32, 8), 0, st>>>(rows, cols, src, ld, tr, kpad, reinterpret_cast<__nv_bfloat16 *>(dst));
+cudaError_t launch_pack_bf16(const PackArgs &a, const PackArgs &b, cudaStream_t st) {
+    long long blocks[2] = {0, 0};
+    const PackArgs *p[2] = {&a, &b};
+    for (int q = 0; q < 2; ++q) {
+        if (p[q]->rows_pad <= 0 || p[q]->kpad <= 0) continue;
+        if (p[q]->rows_pad % 32 || p[q]->kpad % 32 || p[q]->rows > p[q]->rows_pad || p[q]->cols > p[q]->kpad)
+            return cudaErrorInvalidValue;
+        blocks[q] = p[q]->rows_pad / 32 * (p[q]->kpad / 32);
+    }
+    if (blocks[0] + blocks[1] == 0) return cudaSuccess;
+    if (blocks[0] + blocks[1] >= (1LL << 31)) return cudaErrorInvalidValue;
+    k_pack_bf16<<<(unsigned)(blocks[0] + blocks[1]), dim3(32, 8), 0, st>>>(a, b, (unsigned)blocks[0]);
     return cudaGetLastError();
 }
 cudaError_t launch_feat_nodes(const FeatArgs &a, cudaStream_t st) {

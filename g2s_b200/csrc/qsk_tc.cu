@@ -675,14 +675,16 @@ __global__ void __launch_bounds__(threads_for(W), 1)
 // C[M x N] = A[M x K] * B[N x K]^T (+ bias[n]), A and B BF16 K-major with
 // rows padded to the tile and K to 64 elements (zeros), C FP32 row-major.
 // One 128 x BNG output tile per CTA: warp 0 streams the K blocks of A and B
-// through a 4-stage ring with TMA, warp 1 allocates BNG TMEM columns and
+// through a ring of gemm_stages(BNG) stages with TMA, warp 1 allocates BNG TMEM columns and
 // issues the MMAs (kind::f16, BF16 in, FP32 accumulate), warps 2-5 read the
 // accumulator (one row per thread) and store the rows inside M x N.  Waits
 // are bounded as in k_tc_shortlist.
+// (about 192 KB in flight whatever the tile)
+__host__ __device__ constexpr int gemm_stages(int bng) { return bng == 64 ? 8 : bng == 128 ? 6 : 4; }
 template <int BNG>
 __global__ void __launch_bounds__(192, 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcGemmArgs g) {
-    constexpr int STAGES = 4;
+    constexpr int STAGES = gemm_stages(BNG);
     constexpr int AB = BM * BKB, BB = BNG * BKB;
     extern __shared__ uint8_t smem_raw[];
     const unsigned raw = smem_u32(smem_raw);
@@ -715,6 +717,7 @@ __global__ void __launch_bounds__(192, 1)
     __syncthreads();
     tc_fence_after();
     const unsigned tmem = tmem_base_s;
+    griddep_wait();   // launched programmatically behind the packing of its operands
     if (warp == 0) {
         if (lane == 0) {
             int s = 0;
@@ -898,8 +901,9 @@ cudaError_t launch_tc_shortlist(int kind, int W, const void *a_mat, long long a_
 namespace {
 template <int BNG>
 cudaError_t launch_gemm_bn(const CUtensorMap &ma, const CUtensorMap &mb, const TcGemmArgs &g, cudaStream_t st) {
-    // alignment slack, the 4-stage ring, 10 mbarriers
-    constexpr int SMEM = 1024 + 4 * (tc::BM + BNG) * tc::BKB + 10 * 8;
+    // alignment slack, the ring of stages, two mbarriers each and two more
+    constexpr int STAGES = tc::gemm_stages(BNG);
+    constexpr int SMEM = 1024 + STAGES * (tc::BM + BNG) * tc::BKB + (2 * STAGES + 2) * 8;
     static_assert(SMEM <= 232448, "shared memory");
     auto kern = tc::k_tc_gemm<BNG>;
     static std::mutex mu;
@@ -916,17 +920,26 @@ cudaError_t launch_gemm_bn(const CUtensorMap &ma, const CUtensorMap &mb, const T
         }
     }
     dim3 grid((unsigned)((g.M + tc::BM - 1) / tc::BM), (unsigned)((g.N + BNG - 1) / BNG));
-    kern<<<grid, 192, SMEM, st>>>(ma, mb, g);
-    return cudaGetLastError();
+    return launch_pdl(kern, grid, dim3(192), SMEM, st, ma, mb, g);
 }
 }  // namespace
 
-int tc_gemm_bn(int N) { return N <= 64 ? 64 : N <= 128 ? 128 : 256; }
+// Columns of an output tile: the widest whose tiles fill the SMs, else 64 (a
+// product of few tiles is bound by the latency of its chain of K blocks, and
+// a narrow tile's are shorter: the 14 products of a 1,024-pair gradient took
+// 368 us in tiles of 256, 171 in tiles of 64).  The products of an element run
+// in the same order in every tile.
+int tc_gemm_bn(int M, int N) {
+    const long long tm = (M + tc::BM - 1) / tc::BM;
+    if (N > 128 && tm * ((N + 255) / 256) >= 148) return 256;
+    if (N > 64 && tm * ((N + 127) / 128) >= 148) return 128;
+    return 64;
+}
 
 cudaError_t launch_tc_gemm(const void *a_bf16, long long a_rows, const void *b_bf16, long long b_rows,
                            const TcGemmArgs &g, cudaStream_t st) {
     if (g.M <= 0 || g.N <= 0) return cudaSuccess;
-    const int BNG = tc_gemm_bn(g.N);
+    const int BNG = tc_gemm_bn(g.M, g.N);
     // operands are padded: rows to the tile, K to whole 64-element blocks
     if (g.kpad <= 0 || g.kpad % 64 || a_rows % tc::BM || b_rows % BNG || a_rows < g.M || b_rows < g.N)
         return cudaErrorInvalidValue;
