@@ -317,18 +317,22 @@ struct LevelArgs {
     long long hold = -1;       // node whose level is never published (failure-path test), -1 none
 };
 cudaError_t launch_levels(const LevelArgs &a, cudaStream_t st);
-cudaError_t launch_prep_sim(const SimPrepArgs &a, cudaStream_t st);
+// chained (here and below): the stream's last operation is the kernel before
+// this one in its level's chain (replay or select -> preparation -> map ->
+// replay or hash select), behind which it may begin launching
+cudaError_t launch_prep_sim(const SimPrepArgs &a, bool chained, cudaStream_t st);
 int map_segs_per_cta(const Geom &g, int nslots);
-cudaError_t launch_map_records(const MapArgs &a, int nslots, int K, int maxterms_in_batch, cudaStream_t st);
+cudaError_t launch_map_records(const MapArgs &a, int nslots, int K, int maxterms_in_batch, bool chained,
+                               cudaStream_t st);
 cudaError_t set_map_smem_limit(int bytes);
 cudaError_t launch_build_planes(const float *layers, const Geom &g, int nvar, const int *ncat, const float *catv,
                                 int pw, unsigned *planes, cudaStream_t st);
 int map_bits_segs_per_cta(const Geom &g, int nslots);
-cudaError_t launch_map_bits(const BitArgs &a, int nslots, int K, int maxterms_in_batch, cudaStream_t st);
-cudaError_t launch_replay(const ReplayArgs &a, cudaStream_t st);
+cudaError_t launch_map_bits(const BitArgs &a, int nslots, int K, int maxterms_in_batch, bool chained, cudaStream_t st);
+cudaError_t launch_replay(const ReplayArgs &a, bool chained, cudaStream_t st);
 // k best by (score, tie hash) over the records, and marginal draws; slots
 // with SLOT_EMIT_MASKED are left to launch_replay with only_flagged
-cudaError_t launch_hash_select(const ReplayArgs &a, cudaStream_t st);
+cudaError_t launch_hash_select(const ReplayArgs &a, bool chained, cudaStream_t st);
 // exclusion masks: slot b's positions around scan index center[b] (radius[b] >= 1)
 cudaError_t launch_radius_mask(const int *center, const float *radius, int nslots, const Geom &g, unsigned *mask,
                                long long xwords, cudaStream_t st);

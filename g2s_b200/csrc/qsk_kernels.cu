@@ -514,9 +514,10 @@ __device__ __forceinline__ void prep_sim_warp(const SimPrepArgs &A, const int wa
     const int cnt = A.nb_count[i];
     const int nd = A.g.nd;
     const NodeGeom ng = node_geometry(A, i, cell, lane);
-    // launched programmatically (k_prep_tc_nodes): what is read above follows
-    // from the path alone; simulated values, slots and terms come below
+    // launched programmatically: what is read above follows from the path
+    // alone; simulated values, slots and terms come below
     griddep_wait();
+    griddep_launch();   // (no later grid reads or writes anything before this one has completed)
     Slot s;
     s.node = i;
     s.cell = cell;
@@ -632,7 +633,6 @@ __device__ __forceinline__ void prep_sim_warp(const SimPrepArgs &A, const int wa
 }
 
 __global__ void k_prep_sim(SimPrepArgs A) {
-    griddep_launch();   // a programmatic successor (k_tc_nodes) may begin launching
     prep_sim_warp(A, int((blockIdx.x * blockDim.x + threadIdx.x) >> 5), int(threadIdx.x & 31));
 }
 
@@ -931,6 +931,8 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 4 : 2) k_map_records(MapArgs A)
         return;
     }
     const int part = int(blockIdx.x) - (GEN ? 1 : 0);
+    griddep_wait();
+    griddep_launch();
     const Term *src = A.terms + (long long)b * A.maxterms;
     // a thread's first term is read beside the slot (the slot's block of terms
     // is maxterms long; what lies beyond its own terms is not used)
@@ -1562,6 +1564,8 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayAr
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
     const int b = blockIdx.x;
+    // the slot and its generator state come from kernels that had completed
+    // when the map let this grid launch; everything else is read below
     const Slot &sl = A.slots[b];
     const int flags = sl.flags;
     // only_flagged: the slots the hash select leaves (fewer valid positions
@@ -1569,6 +1573,7 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayAr
     if (A.only_flagged && (flags & (SLOT_SKIP | SLOT_EMIT_MASKED)) != SLOT_EMIT_MASKED) return;
     const Geom &g = A.g;
     if (flags & SLOT_SKIP) {
+        griddep_wait();
         if (tid != 0 || !(A.state || A.node_cell)) return;
         replay_write(A, sl, marginal_cell(A, sl));
         return;
@@ -1593,6 +1598,8 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayAr
     for (int q = 0; q < KM; ++q) { cv[q] = -CUDART_INF_F; cp[q] = 0xffffffffu; }
     unsigned cpt = 0;
     long long last = -1;
+    griddep_wait();
+    griddep_launch();
     const bool emit_masked = (flags & (SLOT_EMIT_MASKED | SLOT_MISSING)) != 0;
     const float *rv = A.rec_val + (long long)b * g.nseg * QSK_SEG;
     const int *ri = A.rec_idx + (long long)b * g.nseg * QSK_SEG;
@@ -1832,7 +1839,9 @@ __global__ void __launch_bounds__(HS_THREADS) k_hash_select(ReplayArgs A) {
     __shared__ unsigned sp[HS_THREADS * KM];
     const int b = blockIdx.x;
     if (b >= A.nslots) return;
-    const Slot s = A.slots[b];
+    const Slot s = A.slots[b];   // (complete when the map let this grid launch)
+    griddep_wait();
+    griddep_launch();
     if (s.flags & SLOT_SKIP) {
         if (threadIdx.x == 0 && (A.state || A.node_cell)) replay_write(A, s, marginal_cell(A, s));
         return;
@@ -1992,6 +2001,9 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
         return;
     }
     const int part = int(blockIdx.x) - (GEN ? 1 : 0);
+    // static slots and terms (k_mt_prep, a group of levels ahead) are read
+    // before the previous level has completed, the values below
+    if (!A.sterms) griddep_wait();
     if (threadIdx.x == 0) {
         ss = A.slots[b];
         nbt = 0;
@@ -2002,6 +2014,8 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
         s_hi[threadIdx.x] = INT_MIN;
     }
     __syncthreads();
+    griddep_wait();
+    griddep_launch();
     if (ss.flags & SLOT_SKIP) return;
     const Geom &g = A.g;
     const int seg_begin = part * A.segs_per_cta;
@@ -2666,11 +2680,10 @@ cudaError_t launch_prep_tc_nodes(const SimPrepArgs &p, const TcNodeArgs &a, bool
     return cudaGetLastError();
 }
 
-cudaError_t launch_prep_sim(const SimPrepArgs &a, cudaStream_t st) {
+cudaError_t launch_prep_sim(const SimPrepArgs &a, bool chained, cudaStream_t st) {
     int threads = 256;
     long long blocks = ((long long)a.nslots * 32 + threads - 1) / threads;
-    k_prep_sim<<<(unsigned)blocks, threads, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_chain(chained, k_prep_sim, dim3((unsigned)blocks), dim3(threads), 0, st, a);
 }
 
 int map_segs_per_cta(const Geom &g, int nslots) {
@@ -2685,23 +2698,24 @@ int map_segs_per_cta(const Geom &g, int nslots) {
 }
 
 template <bool GEN>
-static void launch_map_records_k(const MapArgs &a, dim3 grid, size_t smem, int K, cudaStream_t st) {
-    if (K <= 1) k_map_records<1, GEN><<<grid, 256, smem, st>>>(a);
-    else if (K <= 2) k_map_records<2, GEN><<<grid, 256, smem, st>>>(a);
-    else if (K <= 4) k_map_records<4, GEN><<<grid, 256, smem, st>>>(a);
-    else if (K <= 8) k_map_records<8, GEN><<<grid, 256, smem, st>>>(a);
-    else k_map_records<16, GEN><<<grid, 256, smem, st>>>(a);
+static cudaError_t launch_map_records_k(const MapArgs &a, dim3 grid, size_t smem, int K, bool chained, cudaStream_t st) {
+    const dim3 block(256);
+    if (K <= 1) return launch_chain(chained, k_map_records<1, GEN>, grid, block, smem, st, a);
+    if (K <= 2) return launch_chain(chained, k_map_records<2, GEN>, grid, block, smem, st, a);
+    if (K <= 4) return launch_chain(chained, k_map_records<4, GEN>, grid, block, smem, st, a);
+    if (K <= 8) return launch_chain(chained, k_map_records<8, GEN>, grid, block, smem, st, a);
+    return launch_chain(chained, k_map_records<16, GEN>, grid, block, smem, st, a);
 }
 
-cudaError_t launch_map_records(const MapArgs &args, int nslots, int K, int maxterms_in_batch, cudaStream_t st) {
+cudaError_t launch_map_records(const MapArgs &args, int nslots, int K, int maxterms_in_batch, bool chained,
+                               cudaStream_t st) {
     MapArgs a = args;
     for (int d = 0; d < QSK_MAXD; ++d) a.div[d] = make_fast_div((unsigned)a.g.fft[d]);
     dim3 grid((unsigned)((a.g.nseg + a.segs_per_cta - 1) / a.segs_per_cta) + (a.gen.state ? 1u : 0u), (unsigned)nslots);
     size_t smem = sizeof(Term) * (size_t)(maxterms_in_batch > 0 ? maxterms_in_batch : 1);
     if (a.gen.state && smem < 624 * sizeof(unsigned)) smem = 624 * sizeof(unsigned);
-    if (a.gen.state) launch_map_records_k<true>(a, grid, smem, K, st);
-    else launch_map_records_k<false>(a, grid, smem, K, st);
-    return cudaGetLastError();
+    return a.gen.state ? launch_map_records_k<true>(a, grid, smem, K, chained, st)
+                       : launch_map_records_k<false>(a, grid, smem, K, chained, st);
 }
 
 cudaError_t launch_build_planes(const float *layers, const Geom &g, int nvar, const int *ncat, const float *catv,
@@ -2724,24 +2738,25 @@ int map_bits_segs_per_cta(const Geom &g, int nslots) {
 }
 
 template <bool GEN>
-static void launch_map_bits_k(const BitArgs &a, dim3 grid, size_t smem, int K, cudaStream_t st) {
-    if (K <= 1) k_map_bits<1, GEN><<<grid, 256, smem, st>>>(a);
-    else if (K <= 2) k_map_bits<2, GEN><<<grid, 256, smem, st>>>(a);
-    else if (K <= 4) k_map_bits<4, GEN><<<grid, 256, smem, st>>>(a);
-    else if (K <= 8) k_map_bits<8, GEN><<<grid, 256, smem, st>>>(a);
-    else k_map_bits<16, GEN><<<grid, 256, smem, st>>>(a);
+static cudaError_t launch_map_bits_k(const BitArgs &a, dim3 grid, size_t smem, int K, bool chained, cudaStream_t st) {
+    const dim3 block(256);
+    if (K <= 1) return launch_chain(chained, k_map_bits<1, GEN>, grid, block, smem, st, a);
+    if (K <= 2) return launch_chain(chained, k_map_bits<2, GEN>, grid, block, smem, st, a);
+    if (K <= 4) return launch_chain(chained, k_map_bits<4, GEN>, grid, block, smem, st, a);
+    if (K <= 8) return launch_chain(chained, k_map_bits<8, GEN>, grid, block, smem, st, a);
+    return launch_chain(chained, k_map_bits<16, GEN>, grid, block, smem, st, a);
 }
 
-cudaError_t launch_map_bits(const BitArgs &args, int nslots, int K, int maxterms_in_batch, cudaStream_t st) {
+cudaError_t launch_map_bits(const BitArgs &args, int nslots, int K, int maxterms_in_batch, bool chained,
+                            cudaStream_t st) {
     BitArgs a = args;
     if (a.maxterms < maxterms_in_batch) return cudaErrorInvalidValue;
     a.stage_words = MAP_BITS_STAGE_WORDS;
     long long nseg1k = (a.g.N + 1023) / 1024;
     dim3 grid((unsigned)((nseg1k + a.segs_per_cta - 1) / a.segs_per_cta) + (a.gen.state ? 1u : 0u), (unsigned)nslots);
     size_t smem = sizeof(int2) * (size_t)(a.maxterms > 0 ? a.maxterms : 1) + sizeof(unsigned) * (size_t)a.stage_words;
-    if (a.gen.state) launch_map_bits_k<true>(a, grid, smem, K, st);
-    else launch_map_bits_k<false>(a, grid, smem, K, st);
-    return cudaGetLastError();
+    return a.gen.state ? launch_map_bits_k<true>(a, grid, smem, K, chained, st)
+                       : launch_map_bits_k<false>(a, grid, smem, K, chained, st);
 }
 
 template <int KF>
@@ -2856,24 +2871,23 @@ cudaError_t launch_mt_prep(const SimPrepArgs &a, unsigned *state, int *pre, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_hash_select(const ReplayArgs &a, cudaStream_t st) {
+cudaError_t launch_hash_select(const ReplayArgs &a, bool chained, cudaStream_t st) {
     if (a.nslots <= 0) return cudaSuccess;
-    if (a.K <= 2) k_hash_select<2><<<(unsigned)a.nslots, HS_THREADS, 0, st>>>(a);
-    else if (a.K <= 4) k_hash_select<4><<<(unsigned)a.nslots, HS_THREADS, 0, st>>>(a);
-    else if (a.K <= 8) k_hash_select<8><<<(unsigned)a.nslots, HS_THREADS, 0, st>>>(a);
-    else k_hash_select<16><<<(unsigned)a.nslots, HS_THREADS, 0, st>>>(a);
-    return cudaGetLastError();
+    const dim3 grid((unsigned)a.nslots), block(HS_THREADS);
+    if (a.K <= 2) return launch_chain(chained, k_hash_select<2>, grid, block, 0, st, a);
+    if (a.K <= 4) return launch_chain(chained, k_hash_select<4>, grid, block, 0, st, a);
+    if (a.K <= 8) return launch_chain(chained, k_hash_select<8>, grid, block, 0, st, a);
+    return launch_chain(chained, k_hash_select<16>, grid, block, 0, st, a);
 }
 
-cudaError_t launch_replay(const ReplayArgs &a, cudaStream_t st) {
+cudaError_t launch_replay(const ReplayArgs &a, bool chained, cudaStream_t st) {
     if (a.nslots <= 0) return cudaSuccess;
-    const unsigned blocks = (unsigned)a.nslots;
-    if (a.K <= 1) k_replay<1><<<blocks, RP_THREADS, 0, st>>>(a);
-    else if (a.K <= 2) k_replay<2><<<blocks, RP_THREADS, 0, st>>>(a);
-    else if (a.K <= 4) k_replay<4><<<blocks, RP_THREADS, 0, st>>>(a);
-    else if (a.K <= 8) k_replay<8><<<blocks, RP_THREADS, 0, st>>>(a);
-    else k_replay<16><<<blocks, RP_THREADS, 0, st>>>(a);
-    return cudaGetLastError();
+    const dim3 grid((unsigned)a.nslots), block(RP_THREADS);
+    if (a.K <= 1) return launch_chain(chained, k_replay<1>, grid, block, 0, st, a);
+    if (a.K <= 2) return launch_chain(chained, k_replay<2>, grid, block, 0, st, a);
+    if (a.K <= 4) return launch_chain(chained, k_replay<4>, grid, block, 0, st, a);
+    if (a.K <= 8) return launch_chain(chained, k_replay<8>, grid, block, 0, st, a);
+    return launch_chain(chained, k_replay<16>, grid, block, 0, st, a);
 }
 
 }  // namespace qsk

@@ -32,4 +32,13 @@ cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, c
     return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 
+// the same with a normal launch when `pdl` is false
+template <typename... P, typename... A>
+cudaError_t launch_chain(bool pdl, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                         A &&...args) {
+    if (pdl) return launch_pdl(kern, grid, block, smem, st, std::forward<A>(args)...);
+    kern<<<grid, block, smem, st>>>(std::forward<A>(args)...);
+    return cudaGetLastError();
+}
+
 }  // namespace qsk
