@@ -1984,11 +1984,15 @@ __device__ __forceinline__ unsigned bits_range(int a, int b) {
     return hi & ~((1u << a) - 1u);
 }
 
-// K <= 4: at most 42 registers, 48 warps per SM (measured faster than 48
-// registers and 40 warps); the wider top-K states would spill under that cap
+// K <= 4: 64 registers, 32 warps per SM.  A warp's later segments are cheap
+// once its carried K-th best is near the map's (no scan, no records), so fewer
+// CTAs with more segments each do less work than 48 warps of one or two
+// segments: 250x250 -> 500x500 (n = 80, plain) 110.5 ms with 40 registers and
+// one or two segments a warp, 103.5 with more segments, 95.8 with 64 registers
+// (no spills) as well.
 // GEN: the first CTA of a slot makes its generator state (GenArgs)
 template <int KF, bool GEN>
-__global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
+__global__ void __launch_bounds__(256, KF <= 4 ? 4 : 1) k_map_bits(BitArgs A) {
     extern __shared__ __align__(16) int2 bterm[];
     __shared__ Slot ss;
     __shared__ int nbt, s_multi, s_total;
@@ -2110,6 +2114,11 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
     float *rv = A.rec_val + (long long)b * g.nseg * QSK_SEG;
     int *ri = A.rec_idx + (long long)b * g.nseg * QSK_SEG;
 
+    // prefix top-KF of what this warp has seen: a CTA's warps take interleaved
+    // segments in scan order, so all of it lies before the next segment
+    float carry[KF];
+#pragma unroll
+    for (int q = 0; q < KF; ++q) carry[q] = -CUDART_INF_F;
     for (int sg = seg_begin + warp; sg < seg_end; sg += nwarps) {
         const long long m0 = (long long)sg * 1024 + 32 * lane;
         // validity of the lane's 32 positions
@@ -2286,7 +2295,24 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
                 rest &= ~cand;
             }
         }
+        // largest score of each 128-position sub-segment (4 lanes) and of all
+        const long long sub = (long long)sg * 8 + (lane >> 2);
+        float gmax = lmax;
+        gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 1));
+        gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 2));
+        float smax = gmax;
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) smax = fmaxf(smax, __shfl_xor_sync(0xffffffffu, smax, off));
+        if (smax < carry[KF - 1]) {
+            // nothing reaches the K-th best before the segment: no record
+            if (sub < g.nseg && (lane & 3) == 0) {
+                A.rec_cnt[(long long)b * g.nseg + sub] = 0;
+                A.rec_max[(long long)b * g.nseg + sub] = gmax;
+            }
+            continue;
+        }
         // exclusive prefix of the lane states across the 1024-position segment
+        // and all before it
         float inc[KF];
 #pragma unroll
         for (int q = 0; q < KF; ++q) inc[q] = lst[q];
@@ -2301,19 +2327,21 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
                 for (int q = 0; q < KF; ++q) inc[q] = mrg[q];
             }
         }
-        float st[KF];
+        float st[KF], before[KF];
 #pragma unroll
         for (int q = 0; q < KF; ++q) {
-            float y = __shfl_up_sync(0xffffffffu, inc[q], 1);
-            st[q] = lane == 0 ? -CUDART_INF_F : y;
+            const float y = __shfl_up_sync(0xffffffffu, inc[q], 1);
+            before[q] = lane == 0 ? -CUDART_INF_F : y;
         }
-        // Lane 0 has no earlier lane, so its running K-th starts from nothing
-        // and most of its positions would be visited one by one below.  The
-        // warp decides them instead: position p of lane 0 on lane p, and an
-        // exclusive prefix top-K over the lanes gives the K-th before each.
-        float x0v;
-        unsigned rmask0;
-        {
+        topk_merge<KF>(carry, before, st);
+        // Before the warp has seen K values, lane 0's running K-th starts from
+        // (almost) nothing and most of its positions would be visited one by one
+        // below.  The warp decides them instead: position p of lane 0 on lane p,
+        // and an exclusive prefix top-K over the lanes gives the K-th before each.
+        const bool special = carry[KF - 1] == -CUDART_INF_F;
+        float x0v = 0.f;
+        unsigned rmask0 = 0u;
+        if (special) {
             const unsigned vm0 = __shfl_sync(0xffffffffu, vm, 0);
             const unsigned recok0 = __shfl_sync(0xffffffffu, emit_masked ? emask : (emask & vmask), 0);
             const unsigned cnt = ((__shfl_sync(0xffffffffu, c0, 0) >> lane) & 1u) |
@@ -2341,22 +2369,37 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
                     for (int q = 0; q < KF; ++q) in0[q] = mrg[q];
                 }
             }
-            const float y = __shfl_up_sync(0xffffffffu, in0[KF - 1], 1);
-            const float kth = lane == 0 ? -CUDART_INF_F : y;
+            float ex0[KF], pre0[KF];
+#pragma unroll
+            for (int q = 0; q < KF; ++q) {
+                const float y = __shfl_up_sync(0xffffffffu, in0[q], 1);
+                ex0[q] = lane == 0 ? -CUDART_INF_F : y;
+            }
+            topk_merge<KF>(carry, ex0, pre0);
+            const float kth = pre0[KF - 1];
             // before K finite values every position that can be a candidate is
             // a record; afterwards the valid ones not below the K-th
             const bool rec = kth == -CUDART_INF_F ? ((recok0 >> lane) & 1u) != 0u : (val && x0v >= kth);
             rmask0 = __ballot_sync(0xffffffffu, rec);
         }
+        {
+            float all[KF], nc[KF];
+#pragma unroll
+            for (int q = 0; q < KF; ++q) all[q] = __shfl_sync(0xffffffffu, inc[q], 31);
+            topk_merge<KF>(carry, all, nc);
+#pragma unroll
+            for (int q = 0; q < KF; ++q) carry[q] = nc[q];
+        }
+        const bool decided = special && lane == 0;   // by the warp, above
         // record flags: value not below the K-th best of everything before it
         // (earlier lanes, then earlier positions of this lane)
-        unsigned rmask = lane == 0 ? rmask0 : 0u;
+        unsigned rmask = decided ? rmask0 : 0u;
         const float T0s = st[KF - 1];
         unsigned eqm = 0u;       // records whose value is tval (no count extraction)
         float tval = 0.f;
-        unsigned from = lane == 0 ? 0u : 0xffffffffu;   // positions decided by the threshold path below
+        unsigned from = decided ? 0u : 0xffffffffu;   // positions decided by the threshold path below
         float T0 = T0s;
-        if (lane != 0 && T0 == -CUDART_INF_F) {
+        if (!decided && T0 == -CUDART_INF_F) {
             // Fewer than K finite values before this lane: every position is a
             // record until K finite values are held (masked ones only when they
             // can be candidates).  Only the valid positions up to that point are
@@ -2425,31 +2468,55 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 6 : 1) k_map_bits(BitArgs A) {
         if ((lane & 3) >= 2) pre += y2;
         const int excl = pre - rc;
         const int tot = __shfl_sync(0xffffffffu, pre, (lane | 3));
-        float gmax = lmax;
-        gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 1));
-        gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 2));
-        const long long sub = (long long)sg * 8 + (lane >> 2);
         // lane 0's records, one per lane (the first ones of its sub-segment)
         if ((rmask0 >> lane) & 1u) {
             const long long r0 = (long long)sg * 8 * QSK_SEG + __popc(rmask0 & lanemask_lt());
             rv[r0] = x0v;
             ri[r0] = int((long long)sg * 1024 + lane);
         }
-        if (sub < g.nseg) {
-            const long long rb = sub * QSK_SEG + excl;
-            int o = 0;
-            unsigned rm = lane == 0 ? 0u : rmask;
+        const int rb = int(sub * QSK_SEG) + excl;   // (scan positions are below 2^31)
+        unsigned rm = decided || sub >= g.nseg ? 0u : rmask;
+        if (__reduce_max_sync(0xffffffffu, (unsigned)__popc(rm)) > 6u) {
+            // many records in a lane (ties): one lane's positions after the
+            // other, position p on lane p, in coalesced stores
+            unsigned todo = __ballot_sync(0xffffffffu, rm != 0u);
+            while (todo) {
+                const int l = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const unsigned mask = __shfl_sync(0xffffffffu, rm, l), eq = __shfl_sync(0xffffffffu, eqm, l);
+                const unsigned in = __shfl_sync(0xffffffffu, vm, l);
+                const int at = __shfl_sync(0xffffffffu, rb, l);
+                float x = __shfl_sync(0xffffffffu, tval, l);
+                if (mask & ~eq) {
+                    const unsigned cnt = ((__shfl_sync(0xffffffffu, c0, l) >> lane) & 1u) |
+                                         (((__shfl_sync(0xffffffffu, c1, l) >> lane) & 1u) << 1) |
+                                         (((__shfl_sync(0xffffffffu, c2, l) >> lane) & 1u) << 2) |
+                                         (((__shfl_sync(0xffffffffu, c3, l) >> lane) & 1u) << 3) |
+                                         (((__shfl_sync(0xffffffffu, c4, l) >> lane) & 1u) << 4) |
+                                         (((__shfl_sync(0xffffffffu, c5, l) >> lane) & 1u) << 5) |
+                                         (((__shfl_sync(0xffffffffu, c6, l) >> lane) & 1u) << 6) |
+                                         (((__shfl_sync(0xffffffffu, c7, l) >> lane) & 1u) << 7);
+                    if (!((eq >> lane) & 1u)) x = ((in >> lane) & 1u) ? (float)cnt : -CUDART_INF_F;
+                }
+                if ((mask >> lane) & 1u) {
+                    const int o = at + __popc(mask & lanemask_lt());
+                    rv[o] = x;
+                    ri[o] = int((long long)sg * 1024 + 32 * l + lane);
+                }
+            }
+        } else {
+            int o = rb;
             while (rm) {
                 const int bit = __ffs(rm) - 1;
                 rm &= rm - 1u;
-                rv[rb + o] = ((eqm >> bit) & 1u) ? tval : (((vm >> bit) & 1u) ? (float)count_at(bit) : -CUDART_INF_F);
-                ri[rb + o] = int(m0 + bit);
+                rv[o] = ((eqm >> bit) & 1u) ? tval : (((vm >> bit) & 1u) ? (float)count_at(bit) : -CUDART_INF_F);
+                ri[o] = int(m0 + bit);
                 o++;
             }
-            if ((lane & 3) == 0) {
-                A.rec_cnt[(long long)b * g.nseg + sub] = tot;
-                A.rec_max[(long long)b * g.nseg + sub] = gmax;
-            }
+        }
+        if (sub < g.nseg && (lane & 3) == 0) {
+            A.rec_cnt[(long long)b * g.nseg + sub] = tot;
+            A.rec_max[(long long)b * g.nseg + sub] = gmax;
         }
     }
 }
@@ -2725,16 +2792,18 @@ cudaError_t launch_build_planes(const float *layers, const Geom &g, int nvar, co
     return cudaGetLastError();
 }
 
-// shared-memory words for the staged plane windows of k_map_bits (24 KB)
-#define MAP_BITS_STAGE_WORDS 6144
+// shared-memory words for the staged plane windows of k_map_bits (30 KB)
+#define MAP_BITS_STAGE_WORDS 7680
 
 int map_bits_segs_per_cta(const Geom &g, int nslots) {
-    long long nseg1k = (g.N + 1023) / 1024;
-    long long target = 148LL * 8;
-    long long per = (nseg1k * nslots + target - 1) / target;
-    if (per < 8) per = 8;
-    if (per > 16) per = 16;
-    return (int)per;
+    // a CTA takes 8 segments of 1024 positions a turn; more turns (up to 8, in
+    // equal shares) tighten the filter of its later segments, whose records
+    // and threshold work are most of the kernel, while three CTAs per SM stay
+    const long long per_slot = (g.N + 8191) / 8192;
+    long long turns = per_slot * nslots / (148LL * 3);
+    turns = turns < 1 ? 1 : (turns > 8 ? 8 : turns);
+    const long long ctas = (per_slot + turns - 1) / turns;
+    return (int)((per_slot + ctas - 1) / ctas * 8);
 }
 
 template <bool GEN>
