@@ -1162,12 +1162,14 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 4 : 2) k_map_records(MapArgs A)
 #define SEG_AHEAD 4           // windows of one segment per thread read at once
 
 struct __align__(16) ReplayShared {
-    float rv_s[REC_CAP];      // staged records (values), in scan order
-    int ri_s[REC_CAP];        // and their scan indices
+    // staged records in scan order, a segment's padded to a multiple of four
+    // with NaN (which no comparison takes for a record), and their scan indices
+    float rv_s[REC_CAP];
+    int ri_s[REC_CAP];
     unsigned mt[2][624];      // generator state, the next block written beside the last
     float buf[RNG_BUF];       // draws
     float w_top[RP_TEAM][QSK_KMAX];   // per warp: top-K of its part
-    int w_sum[RP_TEAM];       // per warp: records to stage
+    int w_sum[RP_TEAM];       // per warp: records to stage, or ties
     int4 w_fun[RP_TEAM];      // per warp: cpt function and draws of its part
     int w_map[RP_TEAM][QSK_KMAX];     // per warp: slot map of its part
     int stop, staged;         // first thread whose segment did not fit, records staged
@@ -1312,6 +1314,114 @@ __device__ __forceinline__ int replay_trigger(int K, float v, T entry, float (&c
     return 2;
 }
 
+// The position updates of a run: every thread's slot map o, composed in thread
+// order (each warp's to its lane 0, then the warps'), applied to cp.
+template <int KM>
+__device__ __forceinline__ void compose_maps(ReplayShared &w, int tid, int (&o)[KM], unsigned (&cp)[KM]) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = tid & 31, wid = tid >> 5;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        int later[KM];
+#pragma unroll
+        for (int k = 0; k < KM; ++k) later[k] = __shfl_down_sync(FULL, o[k], d);
+        if ((lane & (2 * d - 1)) == 0) {
+            int c[KM];
+#pragma unroll
+            for (int k = 0; k < KM; ++k) c[k] = later[k] < 0 ? later[k] : sel_i<KM>(o, later[k]);
+#pragma unroll
+            for (int k = 0; k < KM; ++k) o[k] = c[k];
+        }
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < KM; ++k) w.w_map[wid][k] = o[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < KM; ++k) o[k] = k;
+    for (int q = 0; q < RP_TEAM; ++q) {
+        int c[KM];
+#pragma unroll
+        for (int k = 0; k < KM; ++k) {
+            const int later = w.w_map[q][k];
+            c[k] = later < 0 ? later : sel_i<KM>(o, later);
+        }
+#pragma unroll
+        for (int k = 0; k < KM; ++k) o[k] = c[k];
+    }
+    unsigned np[KM];
+#pragma unroll
+    for (int k = 0; k < KM; ++k) np[k] = o[k] < 0 ? unsigned(-(o[k] + 1)) : sel_u<KM>(cp, o[k]);
+#pragma unroll
+    for (int k = 0; k < KM; ++k) cp[k] = np[k];
+}
+
+// The staged records [r, n) when none exceeds the K-th value V of a full
+// state: the state's values stay as they are and every record equal to V is a
+// tie (two draws, cpt + 1, a swap inside the xes tail slots that hold V and a
+// possible replacement at K-1).  Thread t takes P consecutive records; ties
+// are ranked by a scan over the team.
+template <int KM>
+__device__ __forceinline__ void team_ties(ReplayShared &w, int tid, int r, int n, int K, const float (&cv)[KM],
+                                          unsigned (&cp)[KM], unsigned &cpt, Rng &g) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = tid & 31, wid = tid >> 5;
+    const float V = sel_f<KM>(cv, K - 1);
+    int xes = 0;
+#pragma unroll
+    for (int q = 0; q < KM; ++q) xes += (q < K && cv[q] == V) ? 1 : 0;
+    // P odd keeps a warp's reads on distinct banks; P <= REC_CAP / RP_THREADS + 1 bits
+    const int P = ((n - r + RP_THREADS - 1) / RP_THREADS) | 1;
+    const int j0 = min(n, r + tid * P), j1 = min(n, j0 + P);
+    unsigned tm = 0u;
+#pragma unroll 1
+    for (int j = j0; j < j1; ++j) tm |= unsigned(w.rv_s[j] == V) << (j - j0);
+    const int mine = __popc(tm);
+    int incl = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(FULL, incl, off);
+        if (lane >= off) incl += y;
+    }
+    if (lane == 31) w.w_sum[wid] = incl;
+    __syncthreads();
+    int before = 0, total = 0;
+#pragma unroll
+    for (int q = 0; q < RP_TEAM; ++q) {
+        const int t = w.w_sum[q];
+        before += q < wid ? t : 0;
+        total += t;
+    }
+    if (total == 0) return;
+    rng_need(w, tid, g, 2 * total);
+    int o[KM];
+#pragma unroll
+    for (int k = 0; k < KM; ++k) o[k] = k;
+    int rank = before + incl - mine;
+    const float fx = (float)xes;
+    while (tm) {
+        const int j = j0 + __ffs(tm) - 1;
+        tm &= tm - 1u;
+        const float u1 = w.buf[g.rp + 2 * rank], u2 = w.buf[g.rp + 2 * rank + 1];
+        int x = K - xes + int(floorf(__fmul_rn(u1, fx)));
+        if (x > K - 1) x = K - 1;
+        const unsigned after = cpt + unsigned(rank) + 1u;
+        const bool write = __fmul_rn(__uint2float_rn(unsigned(xes) + after), u2) < fx;
+        const int ox = sel_i<KM>(o, x), ok1 = sel_i<KM>(o, K - 1);
+        const int wr = -(w.ri_s[j] + 1);
+#pragma unroll
+        for (int k = 0; k < KM; ++k) {
+            if (k == x) o[k] = ok1;
+            if (k == K - 1) o[k] = write ? wr : ox;
+        }
+        ++rank;
+    }
+    compose_maps<KM>(w, tid, o, cp);
+    cpt += unsigned(total);
+    g.rp += 2 * total;
+}
+
 // The scan over the staged records [r, n) by the whole team, thread t taking P
 // consecutive ones.  What a record does follows from prefixes: the K-th best
 // before it (a top-K scan), its draws (a count) and cpt (a composition of
@@ -1334,7 +1444,11 @@ __device__ __forceinline__ void team_scan(ReplayShared &w, int tid, int r, int n
         float st[KM];
 #pragma unroll
         for (int k = 0; k < KM; ++k) st[k] = -CUDART_INF_F;
-        for (int j = j0; j < j1; ++j) topk_insert<KM>(st, w.rv_s[j]);
+#pragma unroll 1
+        for (int j = j0; j < j1; ++j) {
+            const float v = w.rv_s[j];
+            topk_insert<KM>(st, isnan(v) ? -CUDART_INF_F : v);
+        }
         top = st[0];
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
@@ -1381,6 +1495,7 @@ __device__ __forceinline__ void team_scan(ReplayShared &w, int tid, int r, int n
         float st[KM];
 #pragma unroll
         for (int k = 0; k < KM; ++k) st[k] = pre[k];
+#pragma unroll 1
         for (int j = j0; j < j1; ++j) {
             const float v = w.rv_s[j];
             const float kth = sel_f<KM>(st, K - 1);
@@ -1439,48 +1554,14 @@ __device__ __forceinline__ void team_scan(ReplayShared &w, int tid, int r, int n
     for (int k = 0; k < KM; ++k) o[k] = k;
     if (nd > 0) {
         const float *u = w.buf + g.rp + ed;
+#pragma unroll 1
         for (int j = j0; j < j1; ++j) {
             const float v = w.rv_s[j];
             if (!(v >= sel_f<KM>(pre, K - 1))) continue;
             u += replay_trigger<KM, int>(K, v, -(w.ri_s[j] + 1), pre, o, mycpt, u);
         }
     }
-    // composed in thread order: each warp's to its lane 0, then the warps'
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        int later[KM];
-#pragma unroll
-        for (int k = 0; k < KM; ++k) later[k] = __shfl_down_sync(FULL, o[k], d);
-        if ((lane & (2 * d - 1)) == 0) {
-            int c[KM];
-#pragma unroll
-            for (int k = 0; k < KM; ++k) c[k] = later[k] < 0 ? later[k] : sel_i<KM>(o, later[k]);
-#pragma unroll
-            for (int k = 0; k < KM; ++k) o[k] = c[k];
-        }
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < KM; ++k) w.w_map[wid][k] = o[k];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < KM; ++k) o[k] = k;
-    for (int q = 0; q < RP_TEAM; ++q) {
-        int c[KM];
-#pragma unroll
-        for (int k = 0; k < KM; ++k) {
-            const int later = w.w_map[q][k];
-            c[k] = later < 0 ? later : sel_i<KM>(o, later);
-        }
-#pragma unroll
-        for (int k = 0; k < KM; ++k) o[k] = c[k];
-    }
-    unsigned np[KM];
-#pragma unroll
-    for (int k = 0; k < KM; ++k) np[k] = o[k] < 0 ? unsigned(-(o[k] + 1)) : sel_u<KM>(cp, o[k]);
-#pragma unroll
-    for (int k = 0; k < KM; ++k) cp[k] = np[k];
+    compose_maps<KM>(w, tid, o, cp);
     g.rp += total;
 }
 
@@ -1531,10 +1612,6 @@ __device__ __forceinline__ void replay_write(const ReplayArgs &A, const Slot &s,
     }
 }
 
-__device__ __forceinline__ void cp_async4(void *smem_dst, const void *gmem_src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
@@ -1555,10 +1632,12 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // that read each candidate segment on its own and replayed 32 records a step
 // (mean of a level, launch to end): a 200x200 continuous simulation (n = 50)
 // 47 -> 14 us, categorical 101x90 (n = 20) 40 -> 25 us, 250x250 -> 500x500
-// (n = 80) 65 -> 54 us; one slot of 26,000 segments 559 -> 230 us, of which
+// (n = 80) 65 -> 54 us; then with 16-byte staging copies, tie runs of their own
+// (team_ties) and three CTAs of 80 registers per SM the slots of the last two
+// took 54 k -> 35 k and 83 k -> 50 k cycles; one slot of 26,000 segments 559 -> 230 us, of which
 // the generator blocks of its first masked stretch are 210.
 template <int KM>
-__global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayArgs A) {
+__global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 3 : 1) k_replay(ReplayArgs A) {
     __shared__ ReplayShared w;
     constexpr int NT = RP_THREADS;
     const unsigned FULL = 0xffffffffu;
@@ -1601,6 +1680,8 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayAr
     griddep_wait();
     griddep_launch();
     const bool emit_masked = (flags & (SLOT_EMIT_MASKED | SLOT_MISSING)) != 0;
+    long long first_valid = 0;
+    for (int d = 0; d < g.nd; ++d) first_valid += (long long)s.lo[d] * g.sstride[d];
     const float *rv = A.rec_val + (long long)b * g.nseg * QSK_SEG;
     const int *ri = A.rec_idx + (long long)b * g.nseg * QSK_SEG;
     const int *rc = A.rec_cnt + (long long)b * g.nseg;
@@ -1616,18 +1697,23 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayAr
             c[i] = q < g.nseg ? rc[q] : 0;
             m[i] = q < g.nseg ? rm[q] : -CUDART_INF_F;
         }
-#pragma unroll
+        // (one copy of the loop's code; the selects cost less than its fetches)
+#pragma unroll 1
         for (int i = 0; i < SEG_AHEAD; ++i) {
             const int q0 = sg + i * NT;
             if (q0 >= g.nseg) break;
+            int ci = sel_i<SEG_AHEAD>(c, i);
+            const float mx = sel_f<SEG_AHEAD>(m, i);
             for (;;) {   // until the window's segments are staged and scanned
                 const float kth = sel_f<KM>(cv, K - 1);
-                if (!__syncthreads_or(c[i] > 0 && m[i] >= kth)) break;
-                bool fl = c[i] > 0 && m[i] >= kth;
-                if (__syncthreads_or(fl && (m[i] > kth || kth == -CUDART_INF_F))) {
+                if (!__syncthreads_or(ci > 0 && mx >= kth)) break;
+                bool fl = ci > 0 && mx >= kth;
+                // (a state that is not full takes the general scan)
+                const bool above = __syncthreads_or(fl && (mx > kth || kth == -CUDART_INF_F));
+                if (above) {
                     // K-th best of the state and the earlier segments of the window
                     float st[KM], pre[KM];
-                    st[0] = c[i] > 0 ? m[i] : -CUDART_INF_F;
+                    st[0] = ci > 0 ? mx : -CUDART_INF_F;
 #pragma unroll
                     for (int k = 1; k < KM; ++k) st[k] = -CUDART_INF_F;
 #pragma unroll
@@ -1662,9 +1748,9 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayAr
 #pragma unroll
                         for (int k = 0; k < KM; ++k) pre[k] = mrg[k];
                     }
-                    fl = fl && m[i] >= sel_f<KM>(pre, K - 1);
+                    fl = fl && mx >= sel_f<KM>(pre, K - 1);
                 }
-                const int cnt = fl ? c[i] : 0;
+                const int cnt = fl ? (ci + 3) & ~3 : 0;   // padded
                 int incl = cnt;
 #pragma unroll
                 for (int off = 1; off < 32; off <<= 1) {
@@ -1684,19 +1770,24 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayAr
                 const int dst = before + incl - cnt;
                 const bool take = fl && dst + cnt <= REC_CAP;
                 if (fl && !take) atomicMin(&w.stop, tid);
-                // the segments' records, one segment of the warp after the other
+                // the segments' records in 16-byte copies (a segment's start on
+                // 512 bytes), one segment of the warp after the other: the lower
+                // lanes the values, the upper ones the indices
                 unsigned todo = __ballot_sync(FULL, take);
                 while (todo) {
                     const int l = __ffs(todo) - 1;
                     todo &= todo - 1u;
                     const int n = __shfl_sync(FULL, cnt, l), d = __shfl_sync(FULL, dst, l);
                     const long long from = (long long)(q0 + 32 * wid + l) * QSK_SEG;
-                    for (int k = lane; k < n; k += 32) {
-                        cp_async4(&w.rv_s[d + k], rv + from + k);
-                        cp_async4(&w.ri_s[d + k], ri + from + k);
+                    for (int k = 4 * (lane & 15); k < n; k += 64) {
+                        if (lane < 16) cp_async16(&w.rv_s[d + k], rv + from + k);
+                        else cp_async16(&w.ri_s[d + k], ri + from + k);
                     }
                 }
                 cp_async_wait_all();
+                __syncthreads();
+                if (take)
+                    for (int k = ci; k < cnt; ++k) w.rv_s[dst + k] = CUDART_NAN_F;
                 __syncthreads();
                 const int stop = w.stop;
                 int n = all;
@@ -1711,9 +1802,16 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayAr
                 int r = 0;
                 while (!emit_masked && r < n && sel_f<KM>(cv, K - 1) == -CUDART_INF_F) {
                     const float v = w.rv_s[r];
+                    if (isnan(v)) {
+                        ++r;
+                        continue;
+                    }
                     const int mm = w.ri_s[r];
+                    // (the first record is the first valid position as a rule:
+                    // all before it are masked)
                     long long gap = mm - (last + 1);
-                    if (gap > 0) gap -= valid_prefix(g, s.lo, mm) - valid_prefix(g, s.lo, last + 1);
+                    if (gap > 0 && !(last < 0 && mm == first_valid))
+                        gap -= valid_prefix(g, s.lo, mm) - (last < 0 ? 0 : valid_prefix(g, s.lo, last + 1));
                     if (gap > 0) {
                         // the first skip covers the prepared blocks (gap >= the masked
                         // positions before the first valid one, so 2 gap > preskip)
@@ -1726,9 +1824,12 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 4 : 1) k_replay(ReplayAr
                     last = mm;
                     ++r;
                 }
-                if (r < n) team_scan<KM>(w, tid, r, n, K, cv, cp, cpt, rng);
+                if (r < n) {
+                    if (above) team_scan<KM>(w, tid, r, n, K, cv, cp, cpt, rng);
+                    else team_ties<KM>(w, tid, r, n, K, cv, cp, cpt, rng);
+                }
                 if (stop == INT_MAX) break;
-                if (tid < stop) c[i] = 0;   // done; the rest of the window once more
+                if (tid < stop) ci = 0;   // done; the rest of the window once more
             }
         }
         sg += SEG_AHEAD * NT;
