@@ -2997,6 +2997,7 @@ int qsk_jobs_run(qsk_sim *const *sims, int count, int threads, int *status) {
     };
     auto worker = [&]() {
         std::vector<std::pair<int, Scratch *>> mine;   // per device
+        bool clean = true;
         for (int q = next.fetch_add(1); q < count; q = next.fetch_add(1)) {
             const int i = order[size_t(q)];
             qsk_sim *s = sims[i];
@@ -3014,12 +3015,20 @@ int qsk_jobs_run(qsk_sim *const *sims, int count, int threads, int *status) {
                 cudaStreamSynchronize(s->st);   // nothing of the run still reads the scratch
                 swap_scratch(s, *x);
             }
-            if (rc[size_t(i)] != QSK_OK) msg[size_t(i)] = g_err;
+            if (rc[size_t(i)] != QSK_OK) {
+                msg[size_t(i)] = g_err;
+                clean = false;
+            }
         }
+        // the scratch goes to the kept blocks, where the next call finds it,
+        // once every run that used it has ended (a failed run may have left
+        // work behind on its other streams: cudaFree waits for that)
+        g_keep_blocks = clean;
         for (auto &m : mine) {
             DeviceGuard dg(m.first);
             delete m.second;
         }
+        g_keep_blocks = false;
     };
     std::vector<std::thread> pool;
     for (int t = 1; t < T; ++t) pool.emplace_back(worker);
