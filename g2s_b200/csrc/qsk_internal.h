@@ -494,6 +494,29 @@ cudaError_t launch_tc_pattern(const TcPatternArgs &a, float *rowmax, cudaStream_
 #define QSK_TMAX_FEW (1 << 30)   // a node's template maximum: fewer than K positions hold its pattern
 cudaError_t launch_tc_tmax(long long nodes, int n, const int *nb_count, const int *nb_tpl, const int *tpl, const Geom &g,
                            int K, int *tmax, cudaStream_t st);
+// histogram of the automatic prefix: bins[(tmax + 256) / 256] over the nodes
+// with a neighbour (tmax >= 0)
+cudaError_t launch_tc_tmax_bins(long long nodes, const int *tmax, int *bins, int nbins, cudaStream_t st);
+// Order of a run's nodes: within a level by K blocks (nodes beyond the prefix,
+// bucket `buckets` - 1, in a list of their own).  Two passes over a node list:
+// the first counts every level's buckets and lists the audited nodes, the
+// second puts each node where the host's offsets say.
+struct TcPlanArgs {
+    const int *nodes = nullptr;   // level order
+    int count = 0;
+    const int *tmax = nullptr;    // per path node (k_tc_tmax)
+    const int *level = nullptr;   // per path node (null: one level)
+    int first_level = 0;          // of the list
+    int T = 0, L = 0, kbe = 0;    // prefix, layers, elements per K block
+    int buckets = 0;              // K blocks + 1
+    int *bucket = nullptr;        // [level][bucket]: counts, then next positions
+    int *few = nullptr;           // [level]: a node beyond the prefix has fewer than K positions
+    unsigned audit_below = 0;     // nodes whose audit hash lies below are listed
+    int audit_all = 0;
+    int *audit = nullptr, *audit_count = nullptr;
+    int *order = nullptr, *exact = nullptr;   // second pass
+};
+cudaError_t launch_tc_plan(const TcPlanArgs &a, int pass, cudaStream_t st);
 cudaError_t launch_tc_nodes(const TcNodeArgs &a, cudaStream_t st);
 // k_prep_sim and k_tc_nodes of one tensor-core step in one launch (rows of A
 // written, not learned); after_select: the stream's last operation is the

@@ -1070,6 +1070,42 @@ __global__ void k_tc_tmax(long long nodes, int n, const int *__restrict__ nb_cou
     if (lane == 0) tmax[i] = m + (nvalid < K ? QSK_TMAX_FEW : 0);
 }
 
+__global__ void k_tc_tmax_bins(long long nodes, const int *__restrict__ tmax, int *__restrict__ bins, int nbins) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nodes) return;
+    int t = tmax[i];
+    if (t >= QSK_TMAX_FEW - 1) t -= QSK_TMAX_FEW;
+    if (t >= 0) atomicAdd(&bins[min((t + 256) / 256, nbins - 1)], 1);
+}
+
+// The plan of a tensor-core run on the device: a level's nodes in the order
+// of their K blocks (any order within a bucket: a 128-node tile's K is its
+// widest node's).  The host reads the levels' bucket counts and makes the
+// steps; with the nodes' maxima and their order copied to it and sorted
+// there level by level, 9 ms of a 250,000-node simulation went to it.
+// Atomics on a few thousand counters bound it, at microseconds a launch.
+template <bool SCATTER>
+__global__ void k_tc_plan(TcPlanArgs a) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= a.count) return;
+    const int i = a.nodes[q];
+    int t = a.tmax[i];
+    const bool few = t >= QSK_TMAX_FEW - 1;
+    if (few) t -= QSK_TMAX_FEW;
+    const int l = a.level ? a.level[i] - a.first_level : 0;
+    const bool exact = t < 0 || t >= a.T;
+    const int b = exact ? a.buckets - 1 : int((((long long)t + 1) * a.L + a.kbe - 1) / a.kbe) - 1;
+    int *slot = a.bucket + (long long)l * a.buckets + b;
+    const int at = atomicAdd(slot, 1);
+    if (SCATTER) {
+        (exact ? a.exact : a.order)[at] = i;
+        return;
+    }
+    if (exact && few) a.few[l] = 1;
+    // marginal draws have no k best to audit
+    if (t >= 0 && (a.audit_all || tie_hash(0xA5D17u, unsigned(i)) < a.audit_below)) a.audit[atomicAdd(a.audit_count, 1)] = i;
+}
+
 // one warp per tensor slot: the node's row of A (coefficients of its terms at
 // their template columns), its validity box and tie seed
 __global__ void k_tc_nodes(TcNodeArgs A) {
@@ -1594,6 +1630,20 @@ cudaError_t launch_tc_tmax(long long nodes, int n, const int *nb_count, const in
                            int K, int *tmax, cudaStream_t st) {
     if (nodes <= 0) return cudaSuccess;
     k_tc_tmax<<<(unsigned)((nodes * 32 + 255) / 256), 256, 0, st>>>(nodes, n, nb_count, nb_tpl, tpl, g, K, tmax);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tc_tmax_bins(long long nodes, const int *tmax, int *bins, int nbins, cudaStream_t st) {
+    if (nodes <= 0) return cudaSuccess;
+    k_tc_tmax_bins<<<(unsigned)((nodes + 255) / 256), 256, 0, st>>>(nodes, tmax, bins, nbins);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tc_plan(const TcPlanArgs &a, int pass, cudaStream_t st) {
+    if (a.count <= 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)((a.count + 255) / 256);
+    if (pass == 0) k_tc_plan<false><<<blocks, 256, 0, st>>>(a);
+    else k_tc_plan<true><<<blocks, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 

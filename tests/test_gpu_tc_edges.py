@@ -65,3 +65,31 @@ def test_shortlist_edges(g2s, gpu, W, kind, ranges):
             want_p = np.concatenate([np.full(W - len(best), 0xFFFFFFFF, np.uint32), best.astype(np.uint32)])
             assert np.array_equal(keys[b, r], want_k), (b, r)
             assert np.array_equal(pos[b, r], want_p), (b, r)
+
+
+@pytest.mark.parametrize("n,radius,prefix,passes", [(5, 8, 8, 1), (60, 8, 256, 1), (150, 30, 1984, 2)])
+def test_level_plan_does_not_move_draws(g2s, gpu, n, radius, prefix, passes):
+    """The order of a level's nodes, their K blocks (64 elements in BF16, 128
+    in FP8) and the number of passes that plan them leave the draws alone:
+    categorical patterns are exact in both formats, and a shortlist no wider
+    than the kept candidates per range holds the exact k best."""
+    rng = np.random.default_rng(n)
+    ncat = 32
+    ti = rng.integers(0, ncat, (64, 64)).astype(np.float32)   # wide enough for every pattern
+    di = np.full((40, 40), np.nan, np.float32)
+    kernel = np.ones((2 * radius + 1,) * 2, np.float32)
+    got = {}
+    for mode, batch in (("bf16", 0), ("fp8", 0), ("fp8", 128)):
+        sim = g2s.Simulation(ti, di, [1], n=n, k=1.2, seed=7, kernel=kernel)
+        sim.set_tensor(mode, prefix=prefix, width=32, shortlist=32, audit=1.0, batch=batch)
+        sim.run()
+        got[mode, batch] = sim.read()[1], sim.info()
+        sim.close()
+    idx, ref = got["bf16", 0]
+    assert ref["tensor_prefix"] == prefix and ref["tensor_nodes"] + ref["plain_nodes"] == 1600
+    assert (ref["levels"] * (prefix * ncat // 64 + 1) > 1 << 18) == (passes > 1)
+    for out, info in got.values():
+        assert np.array_equal(out, idx)
+        assert info["regret"] == 0 and info["regret_near"] == 0
+        for f in ("levels", "tensor_nodes", "plain_nodes", "audited"):
+            assert info[f] == ref[f], f
