@@ -108,6 +108,121 @@ bool block_keep(void *p, size_t cap) {
 }
 }  // namespace qsk
 
+// Pinned host blocks of the workers' staging.  Page-locking memory takes 0.5
+// to 1.5 ms whatever its size, 20 times a small query, so blocks are lent out
+// and come back: pieces of one allocation up to PINNED_PIECE bytes, larger
+// ones by themselves (at most PINNED_LARGE bytes of them kept).  Freed by
+// qsk_blocks_release, but for allocations with a piece still lent.
+namespace {
+constexpr size_t PINNED_PIECE = 65536, PINNED_LARGE = 64u << 20;
+constexpr int PINNED_PIECES = 8;
+struct PinnedBlocks {
+    std::mutex mu;
+    struct Slab {
+        unsigned char *p;
+        unsigned home;   // bit per piece that is not lent
+    };
+    std::vector<Slab> slabs;
+    std::multimap<size_t, unsigned char *> large;
+    size_t large_bytes = 0;
+};
+constexpr unsigned PINNED_ALL = (1u << PINNED_PIECES) - 1;
+
+PinnedBlocks &pinned() {
+    static PinnedBlocks *b = new PinnedBlocks();   // never destroyed, as above
+    return *b;
+}
+
+int pinned_alloc(size_t bytes, unsigned char **out) {
+    void *q = nullptr;
+    const cudaError_t e = cudaHostAlloc(&q, bytes, cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e != cudaSuccess)
+        return fail(e == cudaErrorMemoryAllocation ? QSK_ERR_NOMEM : QSK_ERR_CUDA, "pinned staging of %zu bytes: %s",
+                    bytes, cudaGetErrorString(e));
+    *out = static_cast<unsigned char *>(q);
+    return QSK_OK;
+}
+
+// at least `bytes` of pinned memory that every device sees at its address
+int pinned_take(size_t bytes, unsigned char **out, size_t *cap) {
+    PinnedBlocks &b = pinned();
+    std::lock_guard<std::mutex> lock(b.mu);
+    if (bytes <= PINNED_PIECE) {
+        size_t i = 0;
+        while (i < b.slabs.size() && b.slabs[i].home == 0) ++i;
+        if (i == b.slabs.size()) {
+            unsigned char *p = nullptr;
+            if (int rc = pinned_alloc(PINNED_PIECE * PINNED_PIECES, &p)) return rc;
+            b.slabs.push_back({p, PINNED_ALL});
+        }
+        int j = 0;
+        while (!(b.slabs[i].home >> j & 1u)) ++j;
+        b.slabs[i].home &= ~(1u << j);
+        *out = b.slabs[i].p + PINNED_PIECE * size_t(j);
+        *cap = PINNED_PIECE;
+        return QSK_OK;
+    }
+    auto it = b.large.lower_bound(bytes);
+    if (it != b.large.end() && it->first <= 4 * bytes) {
+        *out = it->second;
+        *cap = it->first;
+        b.large_bytes -= it->first;
+        b.large.erase(it);
+        return QSK_OK;
+    }
+    if (int rc = pinned_alloc(bytes, out)) return rc;
+    *cap = bytes;
+    return QSK_OK;
+}
+
+// back from its worker, whose stream has ended all work on it
+void pinned_give(unsigned char *p, size_t cap) {
+    if (!p) return;
+    PinnedBlocks &b = pinned();
+    std::lock_guard<std::mutex> lock(b.mu);
+    if (cap != PINNED_PIECE) {
+        if (b.large_bytes + cap > PINNED_LARGE) {
+            cudaFreeHost(p);
+            return;
+        }
+        b.large.emplace(cap, p);
+        b.large_bytes += cap;
+        return;
+    }
+    bool idle = false;   // another allocation with every piece at home
+    for (auto &x : b.slabs) idle |= x.home == PINNED_ALL;
+    for (size_t i = 0; i < b.slabs.size(); ++i) {
+        auto &x = b.slabs[i];
+        if (p < x.p || p >= x.p + PINNED_PIECE * PINNED_PIECES) continue;
+        x.home |= 1u << (size_t(p - x.p) / PINNED_PIECE);
+        if (x.home == PINNED_ALL && idle) {
+            cudaFreeHost(x.p);
+            b.slabs.erase(b.slabs.begin() + long(i));
+        }
+        return;
+    }
+}
+
+int pinned_release() {
+    PinnedBlocks &b = pinned();
+    std::lock_guard<std::mutex> lock(b.mu);
+    cudaError_t e = cudaSuccess;
+    auto drop = [&](unsigned char *p) {
+        const cudaError_t f = cudaFreeHost(p);
+        if (f != cudaSuccess) e = f;
+    };
+    for (auto &x : b.large) drop(x.second);
+    b.large.clear();
+    b.large_bytes = 0;
+    for (size_t i = b.slabs.size(); i-- > 0;) {
+        if (b.slabs[i].home != PINNED_ALL) continue;
+        drop(b.slabs[i].p);
+        b.slabs.erase(b.slabs.begin() + long(i));
+    }
+    return e == cudaSuccess ? QSK_OK : fail(QSK_ERR_CUDA, "cudaFreeHost: %s", cudaGetErrorString(e));
+}
+}  // namespace
+
 int qsk_blocks_set_limit(unsigned long long bytes) {
     KeptBlocks &k = kept();
     std::lock_guard<std::mutex> lock(k.mu);
@@ -127,7 +242,8 @@ int qsk_blocks_release(void) {
         f.second.clear();
         k.bytes[f.first] = 0;
     }
-    return rc;
+    const int prc = pinned_release();
+    return rc != QSK_OK ? rc : prc;
 }
 
 int qsk_blocks_info(int device, unsigned long long *bytes, long long *blocks, long long *hits, long long *misses) {
@@ -233,10 +349,10 @@ struct qsk_worker {
     qsk_ti *ti = nullptr;
     cudaStream_t st = nullptr;
     // a call's slots, terms and exclusion centres, built in pinned memory and
-    // sent in one copy; its results, which the replay writes to pinned memory
-    // that the device sees at the same address
-    unsigned char *h_in = nullptr, *h_out = nullptr;
-    size_t h_in_cap = 0, h_out_cap = 0;
+    // sent in one copy, and behind them its results, which the replay writes
+    // there: the device sees the block at the same address
+    unsigned char *h_io = nullptr;
+    size_t h_cap = 0;
     DBuf<unsigned char> d_in;
     DBuf<float> rec_val;
     DBuf<int> rec_idx;
@@ -244,10 +360,6 @@ struct qsk_worker {
     DBuf<float> rec_max;
     DBuf<unsigned> gen;       // generator states [pattern][624], then the draws they skip
     DBuf<unsigned> xmask;     // [pattern][ceil(N/32)] excluded positions
-    ~qsk_worker() {
-        if (h_in) cudaFreeHost(h_in);
-        if (h_out) cudaFreeHost(h_out);
-    }
 };
 
 namespace {
@@ -332,18 +444,15 @@ int build_pattern_slot(const qsk_ti *ti, int nnb, const int *offsets, int nterms
     return QSK_OK;
 }
 
-// pinned host memory of at least `bytes`, visible to the device
-int pinned_ensure(unsigned char *&p, size_t &cap, size_t bytes) {
-    if (bytes <= cap) return QSK_OK;
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    cap = 0;
-    void *q = nullptr;
-    CK(cudaHostAlloc(&q, bytes, cudaHostAllocMapped));
-    p = static_cast<unsigned char *>(q);
-    cap = bytes;
-    return QSK_OK;
-}
+// ends a worker's queued work when a call fails half-way, so that the next
+// call does not write the staging block under a copy still in flight
+struct DrainOnFailure {
+    cudaStream_t st;
+    bool armed = true;
+    ~DrainOnFailure() {
+        if (armed) cudaStreamSynchronize(st);
+    }
+};
 
 }  // namespace
 
@@ -543,6 +652,11 @@ int qsk_worker_create(qsk_ti *ti, qsk_worker **out) {
         delete w;
         return fail(QSK_ERR_CUDA, "stream: %s", cudaGetErrorString(e));
     }
+    if (int rc = pinned_take(PINNED_PIECE, &w->h_io, &w->h_cap)) {
+        cudaStreamDestroy(w->st);
+        delete w;
+        return rc;
+    }
     *out = w;
     return QSK_OK;
 }
@@ -550,7 +664,11 @@ int qsk_worker_create(qsk_ti *ti, qsk_worker **out) {
 int qsk_worker_destroy(qsk_worker *w) {
     if (!w) return QSK_OK;
     DeviceGuard dgd(w->ti->device);
-    if (w->st) cudaStreamDestroy(w->st);
+    if (w->st) {
+        // after an error the block stays out: work on it may not have ended
+        if (cudaStreamSynchronize(w->st) == cudaSuccess) pinned_give(w->h_io, w->h_cap);
+        cudaStreamDestroy(w->st);
+    }
     delete w;
     return QSK_OK;
 }
@@ -575,11 +693,19 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
     const size_t at_xc = (at_slots + sizeof(Slot) * size_t(B) + 15) / 16 * 16;
     const size_t at_xr = (at_xc + sizeof(int) * size_t(B) + 15) / 16 * 16;
     const size_t in_bytes = at_xr + sizeof(float) * size_t(B);
+    const size_t at_out = (in_bytes + 255) / 256 * 256;
+    const size_t io_bytes = at_out + (sizeof(float) + sizeof(unsigned)) * size_t(B) * k;
     // grown by halves: the number of terms differs from call to call
-    if (in_bytes > w->h_in_cap)
-        if (int rc = pinned_ensure(w->h_in, w->h_in_cap, std::max<size_t>(in_bytes + in_bytes / 2, 16384))) return rc;
-    Term *h_terms = reinterpret_cast<Term *>(w->h_in);
-    Slot *h_slots = reinterpret_cast<Slot *>(w->h_in + at_slots);
+    if (io_bytes > w->h_cap) {
+        unsigned char *p = nullptr;
+        size_t cap = 0;
+        if (int rc = pinned_take(io_bytes + io_bytes / 2, &p, &cap)) return rc;
+        pinned_give(w->h_io, w->h_cap);   // no call of this worker is in flight
+        w->h_io = p;
+        w->h_cap = cap;
+    }
+    Term *h_terms = reinterpret_cast<Term *>(w->h_io);
+    Slot *h_slots = reinterpret_cast<Slot *>(w->h_io + at_slots);
     bool all_match = true;   // unit-weight matches only
     for (int b = 0; b < B; ++b) {
         int nnb = nb_ptr[b + 1] - nb_ptr[b];
@@ -627,16 +753,14 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
         smem_configured_device = ti->device;
     }
     if (any_radius) {
-        std::memcpy(w->h_in + at_xc, xc.data(), sizeof(int) * size_t(B));
-        std::memcpy(w->h_in + at_xr, xr.data(), sizeof(float) * size_t(B));
+        std::memcpy(w->h_io + at_xc, xc.data(), sizeof(int) * size_t(B));
+        std::memcpy(w->h_io + at_xr, xr.data(), sizeof(float) * size_t(B));
     }
-    const size_t out_bytes = (sizeof(float) + sizeof(unsigned)) * size_t(B) * k;
-    if (out_bytes > w->h_out_cap)
-        if (int rc = pinned_ensure(w->h_out, w->h_out_cap, std::max<size_t>(out_bytes, 4096))) return rc;
-    float *const res_val = reinterpret_cast<float *>(w->h_out);
-    unsigned *const res_pos = reinterpret_cast<unsigned *>(w->h_out) + size_t(B) * k;
-    if (in_bytes > w->d_in.n) CK(w->d_in.alloc(w->h_in_cap));
-    CK(cudaMemcpyAsync(w->d_in.p, w->h_in, any_radius ? in_bytes : at_xc, cudaMemcpyHostToDevice, w->st));
+    float *const res_val = reinterpret_cast<float *>(w->h_io + at_out);
+    unsigned *const res_pos = reinterpret_cast<unsigned *>(res_val) + size_t(B) * k;
+    if (in_bytes > w->d_in.n) CK(w->d_in.alloc(std::max<size_t>(in_bytes + in_bytes / 2, 16384)));
+    DrainOnFailure drain{w->st};
+    CK(cudaMemcpyAsync(w->d_in.p, w->h_io, any_radius ? in_bytes : at_xc, cudaMemcpyHostToDevice, w->st));
     const Term *const d_terms = reinterpret_cast<const Term *>(w->d_in.p);
     const Slot *const d_slots = reinterpret_cast<const Slot *>(w->d_in.p + at_slots);
     CK(ensure_records(g, B, w->rec_val, w->rec_idx, w->rec_cnt, w->rec_max));
@@ -704,6 +828,7 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
     ra.mt_pre = gen.pre;
     CK(launch_replay(ra, false, w->st));
     CK(cudaStreamSynchronize(w->st));
+    drain.armed = false;
     std::memcpy(out_score, res_val, sizeof(float) * size_t(B) * k);
     std::memcpy(out_index, res_pos, sizeof(unsigned) * size_t(B) * k);
     // empty patterns keep -inf scores (candidateForPattern returned false)
