@@ -979,7 +979,7 @@ struct qsk_sim {
     DBuf<float> d_tc_nscale, d_tc_bias;
     DBuf<int> d_tc_box, d_tc_tmax, d_tc_kb, d_var_layer0, d_var_ncat;
     DBuf<unsigned> d_tc_seed, d_tc_pos, d_tc_cnt;
-    DBuf<unsigned long long> d_tc_thr;
+    DBuf<unsigned long long> d_tc_thr, d_tc_part;
     DBuf<float> d_var_catv, d_drawn_score, d_drawn_scale;
     DBuf<unsigned long long> d_tc_key, d_tc_counts;
     DBuf<Slot> d_tc_slots;
@@ -1226,6 +1226,9 @@ struct Step {
 int tc_step(qsk_sim *s, const Step &st, bool teacher, bool after_select);
 constexpr int TC_LIST = 1536;   // keys a node's bounded shortlist may hold (ranges x W)
 bool tc_bounded(const qsk_sim *s) { return s->tc_S <= s->tc_W && s->topt.mode != 3; }
+// longer shortlists at W = 32 (FP8): the lists bounded by their 16th best keys
+// (the learned proposal's check reads what each list alone left out)
+bool tc_parts(const qsk_sim *s) { return s->tc_W == 32 && s->tc_S > 32 && s->topt.mode != 3; }
 
 // plain steps, one per slot budget of every level (levels in order)
 std::vector<Step> plain_steps(qsk_sim *s, const std::vector<int> &start) {
@@ -2194,6 +2197,7 @@ int tc_step(qsk_sim *s, const Step &step, bool teacher, bool after_select) {
     na.rows = Bp;
     na.node_thr = s->d_tc_thr.p;
     na.node_count = s->d_tc_cnt.p;
+    na.part = tc_parts(s) ? s->d_tc_part.p : nullptr;
     na.node_scale = s->d_tc_nscale.p;
     na.node_bias = s->d_tc_bias.p;
     na.node_box = s->d_tc_box.p;
@@ -2244,6 +2248,8 @@ int tc_step(qsk_sim *s, const Step &step, bool teacher, bool after_select) {
     // ranges' heaps: enough when the shortlist takes at most W of them
     a.node_thr = bounded ? s->d_tc_thr.p : nullptr;
     a.out_count = bounded ? s->d_tc_cnt.p : nullptr;
+    a.part = na.part;
+    a.part_need = (s->tc_S + 15) / 16;
     a.out_stride = TC_LIST;
     a.out_key = s->d_tc_key.p;
     a.out_pos = s->d_tc_pos.p;
@@ -2329,6 +2335,7 @@ int tc_buffers(qsk_sim *s, size_t n_audit) {
         CK(s->d_tc_key.ensure(slots * 768));
         CK(s->d_tc_pos.ensure(slots * 768));
     }
+    if (tc_parts(s)) CK(s->d_tc_part.ensure(bp * TC_PARTS));
     CK(s->d_tc_slots.ensure(slots));
     CK(s->d_tc_terms.ensure(slots * size_t(s->maxterms)));
     CK(s->d_drawn_score.ensure(size_t(std::max<long long>(s->nodes, 1))));

@@ -364,6 +364,11 @@ struct TcArgs {
     // any range, a lower bound of the row's W-th best key: the ranges filter
     // against it and leave only what it lets through, as a list per row
     unsigned long long *node_thr;
+    // W = 32 without node_thr: null, or [row][TC_PARTS] (zeroed before the
+    // launch) the 16th best key of every list of the row; part_need of them
+    // hold as many keys as the shortlist takes
+    unsigned long long *part;
+    int part_need;
     unsigned *out_count;           // with node_thr: per A row, zeroed before the launch, keys in its list
     // with node_thr: [row][out_stride] the row's out_count keys, in no order;
     // else [row][range][W] ascending, 0 = empty.  A key is
@@ -373,6 +378,7 @@ struct TcArgs {
     int out_stride;                // >= ranges * W
     int *status;
 };
+constexpr int TC_PARTS = 48;       // lists of a row: two per range, at most 768 / 32 ranges
 int tc_supported_width(int w);
 // kind 0: BF16 (kind::f16), 1: FP8 E4M3 (kind::f8f6f4); a_rows % 128 == 0,
 // p_rows % 256 == 0, k_elems * element size % 128 == 0
@@ -443,6 +449,7 @@ struct TcNodeArgs {
     long long rows;
     unsigned long long *node_thr;  // the shortlist's per-node bound and key count, zeroed here (may be null)
     unsigned *node_count;
+    unsigned long long *part = nullptr;   // [slot][TC_PARTS] of the shortlist, zeroed here (may be null)
     float *node_scale;
     float *node_bias;          // sum of the weights of neighbours in a variable's last category
     int *node_box;

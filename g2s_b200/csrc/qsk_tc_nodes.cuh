@@ -66,6 +66,8 @@ __device__ __forceinline__ void tc_nodes_warp(const TcNodeArgs &A, const int war
         A.node_thr[warp] = 0ull;
         A.node_count[warp] = 0u;
     }
+    if (A.part)
+        for (int q = lane; q < TC_PARTS; q += 32) A.part[(long long)warp * TC_PARTS + q] = 0ull;
     float amax = 0.f;
     for (int j = lane; j < cnt; j += 32) {
         const int t = A.nb_tpl[(long long)i * A.n + j];

@@ -93,3 +93,25 @@ def test_level_plan_does_not_move_draws(g2s, gpu, n, radius, prefix, passes):
         assert info["regret"] == 0 and info["regret_near"] == 0
         for f in ("levels", "tensor_nodes", "plain_nodes", "audited"):
             assert info[f] == ref[f], f
+
+
+@pytest.mark.parametrize("shortlist", [33, 48, 64, 128])
+@pytest.mark.parametrize("edge,batch", [(60, 0), (260, 128)])
+def test_long_shortlist_keeps_the_best(g2s, gpu, edge, batch, shortlist):
+    """Shortlists longer than a list's 32 keys, whose lists are bounded by the
+    16th best keys of the others: the k best are exact, so the draws are those
+    of the short list (categorical patterns are exact in both formats, and
+    their many ties are settled by the hash)."""
+    rng = np.random.default_rng(edge)
+    ti = rng.integers(0, 3, (edge, edge)).astype(np.float32)
+    di = np.full((48, 48), np.nan, np.float32)
+    got = []
+    for mode, s in (("bf16", 32), ("fp8", shortlist)):
+        sim = g2s.Simulation(ti, di, [1], n=12, k=2.5, seed=5, kernel=np.ones((21, 21), np.float32))
+        sim.set_tensor(mode, prefix=256, width=32, shortlist=s, batch=batch, audit=1.0)
+        sim.run()
+        got.append((sim.read()[1], sim.info()))
+        sim.close()
+    assert got[0][1]["tensor_nodes"] > 1000 and got[1][1]["tensor_shortlist"] == shortlist
+    assert got[1][1]["regret"] == 0 and got[1][1]["regret_near"] == 0
+    assert np.array_equal(got[0][0], got[1][0])
