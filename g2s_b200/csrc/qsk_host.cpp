@@ -1219,6 +1219,7 @@ struct Step {
     int off, B;
     int kb_off;         // TENSOR: this step's tile K-blocks in d_tc_kb
     int scale = 1;      // TENSOR, learned proposal: the nodes' stencil scale
+    int wide = 0;       // tensor-core form: node tiles at its end that are far wider than the rest
     int level = -1;     // tensor-core form: the dependency level (-1: one stream for all steps)
     bool few = true;    // HASH: a node of the step may have fewer than K positions (it takes the replay)
 };
@@ -1823,6 +1824,12 @@ void tc_level_steps(qsk_sim *s, int level, const int *nodes, int at, const int *
             kb.push_back(b + 1);
             flops += 2.0 * 128 * 256 * double(ntiles_pos) * double(b + 1) * kbe;
         }
+        // tiles whose K is over one and a half times the step's mean: a CTA of
+        // theirs in the second wave would end long after all others
+        const int *k0 = kb.data() + st.kb_off, tiles = int(kb.size()) - st.kb_off;
+        long long sum = 0;
+        for (int q = 0; q < tiles; ++q) sum += k0[q];
+        while (st.wide + 1 < tiles && 2ll * tiles * k0[tiles - 1 - st.wide] > 3 * sum) ++st.wide;
         steps.push_back(st);
     }
 }
@@ -2249,6 +2256,8 @@ int tc_step(qsk_sim *s, const Step &step, bool teacher, bool after_select) {
     a.node_thr = bounded ? s->d_tc_thr.p : nullptr;
     a.out_count = bounded ? s->d_tc_cnt.p : nullptr;
     a.part = na.part;
+    // a bounded shortlist runs in one wave: its order does not matter
+    a.wide = bounded ? 0 : step.wide;
     a.part_need = (s->tc_S + 15) / 16;
     a.out_stride = TC_LIST;
     a.out_key = s->d_tc_key.p;

@@ -349,7 +349,8 @@ struct TcArgs {
     int n_nodes;               // live rows of A
     long long n_pos;           // live rows of P
     long long n_tiles;         // position tiles of 256 rows
-    int ranges;                // position ranges (grid.y)
+    int ranges;                // position ranges
+    int wide;                  // node tiles at the end (< all) that start first, their K being far above the others'
     int tiles_per_range;
     int kblocks;               // K blocks of A and P
     const int *tile_kblocks;   // per 128-row tile of A: K blocks used (null: kblocks)

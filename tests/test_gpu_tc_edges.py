@@ -111,7 +111,11 @@ def test_long_shortlist_keeps_the_best(g2s, gpu, edge, batch, shortlist):
         sim.set_tensor(mode, prefix=256, width=32, shortlist=s, batch=batch, audit=1.0)
         sim.run()
         got.append((sim.read()[1], sim.info()))
+        # all nodes in one step: 18 tiles, the last ones far wider
+        sim.run_teacher(ti[:48, :48])
+        got[-1] += (sim.read()[2],)
         sim.close()
+    assert np.array_equal(got[0][2], got[1][2])
     assert got[0][1]["tensor_nodes"] > 1000 and got[1][1]["tensor_shortlist"] == shortlist
     assert got[1][1]["regret"] == 0 and got[1][1]["regret_near"] == 0
     assert np.array_equal(got[0][0], got[1][0])
