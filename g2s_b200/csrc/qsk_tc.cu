@@ -30,7 +30,9 @@
 //               epilogue bounds the kernel wherever K is short: the 8,000-node
 //               FP8 sample of a 180x150x120 image (W = 32) went 64 -> 44 ms in
 //               this kernel with lists in place of 32-key register insertion
-//               (a chain of 31 compare-and-swaps for the whole warp), the
+//               (a chain of 31 compare-and-swaps for the whole warp) and to
+//               33 with bounds shared by the lists and the widest tiles
+//               first, which leaves it to its widest tile's CTAs; the
 //               BF16 levels of 250x250 -> 500x500 (W = 8) 171 -> 136 us with
 //               the first chunk cut to its own eight best and keys alone
 //
