@@ -228,7 +228,7 @@ __device__ __forceinline__ void order_desc(float &a, float &b) {
     b = fminf(a, b);
     a = hi;
 }
-// eight values in descending order (Batcher's odd-even merge sort, 19 steps)
+// eight values, none of them NaN, in descending order (Batcher's odd-even merge sort, 19 steps)
 __device__ __forceinline__ void sort8(float (&x)[8]) {
     constexpr int A[19] = {0, 2, 4, 6, 0, 1, 4, 5, 1, 5, 0, 1, 2, 3, 2, 3, 1, 3, 5};
     constexpr int B[19] = {1, 3, 5, 7, 2, 3, 6, 7, 2, 6, 4, 5, 6, 7, 4, 5, 2, 4, 6};
@@ -538,13 +538,16 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                 if constexpr (W == 8) {
                     // fewer than eight keys so far: no more than the chunk's own
                     // eight best can enter (their ties too), which a sorting
-                    // network finds without one insertion
+                    // network finds without one insertion.  A NaN score (an
+                    // infinite layer value times a zero) is no candidate and
+                    // stands as -inf: an exchange of it by fmaxf / fminf would
+                    // leave its partner twice
                     if (__any_sync(0xffffffffu, root == 0ull && vmask != 0u)) {
                         float best[8], more[8];
 #pragma unroll
                         for (int o = 0; o < 32; o += 8) {
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) more[j] = ((vmask >> (o + j)) & 1u) ? v[o + j] : -INFINITY;
+                            for (int j = 0; j < 8; ++j) more[j] = ((vmask >> (o + j)) & 1u) ? fmaxf(v[o + j], -INFINITY) : -INFINITY;
                             sort8(more);
                             if (o == 0) {
 #pragma unroll

@@ -119,3 +119,36 @@ def test_long_shortlist_keeps_the_best(g2s, gpu, edge, batch, shortlist):
     assert got[0][1]["tensor_nodes"] > 1000 and got[1][1]["tensor_shortlist"] == shortlist
     assert got[1][1]["regret"] == 0 and got[1][1]["regret_near"] == 0
     assert np.array_equal(got[0][0], got[1][0])
+
+
+@pytest.mark.parametrize("W", [8, 16, 32])
+@pytest.mark.parametrize("fmt,share", [(0, 0.03), (0, 0.6), (0, 0.97), (1, 0.6)])
+def test_nan_scores_are_no_candidates(g2s, gpu, fmt, share, W):
+    """Positions whose score is NaN (a NaN layer value, or an infinite one
+    times a zero coefficient) leave the other positions' shortlist alone."""
+    rng = np.random.default_rng(int(100 * share) + W)
+    X, Y, B, K = 50, 41, 130, 64
+    N = X * Y
+    rows = rng.integers(-2, 3, (N, K)).astype(np.float32)
+    q = rng.integers(-1, 2, (B, K)).astype(np.float32)
+    q[:, 0] = 0.0
+    bad = rng.random(N) < share
+    rows[bad, 0] = np.nan if fmt else np.where(rng.random(bad.sum()) < 0.5, np.nan, np.inf)
+    fp8 = {0.0: 0x00, 1.0: 0x38, 2.0: 0x40, -1.0: 0xb8, -2.0: 0xc0}   # E4M3; NaN 0x7f
+    bits = bf16_bits if fmt == 0 else np.vectorize(lambda x: fp8.get(float(x), 0x7f), otypes=[np.uint8])
+    box = np.tile(np.array([1, X - 2, 0, Y - 1, 0, 1], np.int32), (B, 1))
+    seeds = rng.integers(0, 2**32, B, dtype=np.uint32)
+    keys, pos = g2s.tc_topk(bits(q), bits(rows), fmt, X, Y, box, W=W, q_seed=seeds)
+    rows[bad, 0] = 0.0
+    score = (q @ rows.T).astype(np.float32)
+    ordered = score.view(np.uint32).astype(np.uint64)
+    ordered = np.where(score < 0, ~ordered & np.uint64(0xFFFFFFFF), ordered | np.uint64(0x80000000))
+    p = np.arange(N)
+    x, y = p % X, p // X
+    at = p[~bad & (x >= 1) & (x < X - 2) & (y < Y - 1)]
+    for b in range(B):
+        full = (ordered[b, at] << np.uint64(32)) | tie_hash(seeds[b], at)
+        best = np.argsort(full)[-W:]
+        pad = W - len(best)
+        assert np.array_equal(keys[b, 0], np.concatenate([np.zeros(pad, np.uint64), full[best]])), b
+        assert np.array_equal(pos[b, 0], np.concatenate([np.full(pad, 0xFFFFFFFF), at[best]]).astype(np.uint32)), b
