@@ -44,6 +44,41 @@ struct Geom {
     int nseg;                // ceil(N / QSK_SEG)
 };
 
+// number of valid scan positions < x (x in [0, N])
+__host__ __device__ inline long long valid_prefix(const Geom &g, const int *lo, long long x) {
+    long long vd[QSK_MAXD];
+    long long acc = 1;
+    for (int d = 0; d < g.nd; ++d) {
+        vd[d] = acc;
+        long long w = g.fft[d] - lo[d];
+        acc *= (w > 0 ? w : 0);
+    }
+    if (x >= g.N) return acc;
+    // scan indices are below 2^31 (int record indices): 32-bit digits
+    long long count = 0;
+    const unsigned ux = (unsigned)x;
+    for (int d = g.nd - 1; d >= 0; --d) {
+        const int digit = int((ux / (unsigned)g.sstride[d]) % (unsigned)g.fft[d]);
+        const int t = digit - lo[d];
+        if (t > 0) count += (long long)t * vd[d];
+        if (digit < lo[d]) break;
+    }
+    return count;
+}
+
+// Generator blocks (624 draws each) that the first skip of a slot's replay
+// regenerates without output (see k_mt_prep), and the draws that so many
+// blocks stand for.  A scan of nearly 2^31 positions skips nearly 2^32 draws:
+// the count of blocks fits the int that is kept of them, the draws do not.
+__host__ __device__ inline long long skipped_blocks(const Geom &g, const int *lo, long long nvalid, int K) {
+    if (nvalid < K || nvalid <= 0) return 0;
+    long long m0 = 0;
+    for (int d = 0; d < g.nd; ++d) m0 += (long long)lo[d] * g.sstride[d];
+    const long long n = 2 * (m0 - valid_prefix(g, lo, m0));
+    return n > 624 ? (n - 1) / 624 : 0;
+}
+__host__ __device__ inline long long skipped_draws(int blocks) { return 624LL * blocks; }
+
 // Per node (batch slot) description written by the prep step.
 struct Slot {
     int node;                // path index (simulation) or pattern id
@@ -147,7 +182,7 @@ inline FastDiv make_fast_div(unsigned d) {
     return {unsigned(((1ull << (31 + l)) + d - 1) / d), l - 1};
 }
 
-// Generator states of explicit patterns (state rows and skipped draws as
+// Generator states of explicit patterns (state rows and skipped blocks as
 // k_mt_prep writes them): one more CTA per slot of a map launch makes them
 // while the others run the map; null: none
 struct GenArgs {
@@ -230,8 +265,8 @@ struct ReplayArgs {
     unsigned *id_image;   // per grid cell (-fs: per cell value)
     unsigned *node_cell;  // per path index: chosen TI cell
     int full;             // -fs: write the slot's variable only
-    // generator states from k_mt_prep ([slot][624]) and the draws their
-    // skipped blocks stand for; null: each slot is seeded in the replay
+    // generator states from k_mt_prep ([slot][624]) and the blocks they have
+    // skipped (skipped_draws); null: each slot is seeded in the replay
     const unsigned *mt_state;
     const int *mt_pre;
     // replay only the slots flagged SLOT_EMIT_MASKED (the hash select takes

@@ -68,28 +68,6 @@ __device__ __forceinline__ void topk_insert(float (&st)[KF], float x) {
     }
 }
 
-// number of valid scan positions < x (x in [0, N])
-__device__ long long valid_prefix(const Geom &g, const int *lo, long long x) {
-    long long vd[QSK_MAXD];
-    long long acc = 1;
-    for (int d = 0; d < g.nd; ++d) {
-        vd[d] = acc;
-        long long w = g.fft[d] - lo[d];
-        acc *= (w > 0 ? w : 0);
-    }
-    if (x >= g.N) return acc;
-    // scan indices are below 2^31 (int record indices): 32-bit digits
-    long long count = 0;
-    const unsigned ux = (unsigned)x;
-    for (int d = g.nd - 1; d >= 0; --d) {
-        const int digit = int((ux / (unsigned)g.sstride[d]) % (unsigned)g.fft[d]);
-        const int t = digit - lo[d];
-        if (t > 0) count += (long long)t * vd[d];
-        if (digit < lo[d]) break;
-    }
-    return count;
-}
-
 // ---------------------------------------------------------------------------
 // layers: flipped copy of each TI variable (DataImage.hpp:538-599)
 // continuous: value with NaN -> 0 ; categorical: value kept as the category
@@ -746,22 +724,12 @@ __device__ void mt_roll(unsigned *mt, long long blocks, int lane) {
     __syncwarp();
 }
 
-// blocks that the first skip of a slot's replay regenerates without output:
-// see k_mt_prep
-__device__ long long skipped_blocks(const Geom &g, const int *lo, long long nvalid, int K) {
-    if (nvalid < K || nvalid <= 0) return 0;
-    long long m0 = 0;
-    for (int d = 0; d < g.nd; ++d) m0 += (long long)lo[d] * g.sstride[d];
-    const long long n = 2 * (m0 - valid_prefix(g, lo, m0));
-    return n > 624 ? (n - 1) / 624 : 0;
-}
-
-// the state mt[624] (shared memory) and its skipped draws to row b, one warp
+// the state mt[624] (shared memory) and the blocks it skipped to row b, one warp
 __device__ void store_generator(const unsigned *mt, long long blocks, int b, unsigned *state, int *pre, int lane) {
     // a state row is 624 words, a multiple of 16 bytes
     uint4 *row = reinterpret_cast<uint4 *>(state + (long long)b * 624);
     for (int i = lane; i < 156; i += 32) row[i] = *reinterpret_cast<const uint4 *>(&mt[4 * i]);
-    if (lane == 0) pre[b] = int(624 * blocks);
+    if (lane == 0) pre[b] = int(blocks);
 }
 
 // GenArgs: slot b's generator state by the first warp of a CTA
@@ -1667,7 +1635,7 @@ __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 3 : 1) k_replay(ReplayAr
         // 156 16-byte copies (state rows and w.mt are 16-byte aligned), awaited
         // with the first records
         for (int q = tid; q < 156; q += NT) cp_async16(&w.mt[0][4 * q], A.mt_state + (long long)b * 624 + 4 * q);
-        preskip = A.mt_pre[b];
+        preskip = skipped_draws(A.mt_pre[b]);
     } else if (tid == 0) {
         mt_seed(w.mt[0], s.seed);
     }
