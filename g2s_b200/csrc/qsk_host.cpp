@@ -972,6 +972,7 @@ struct qsk_sim {
     int tc_T_auto = 0;                  // automatic prefix, chosen at the first tensor run
     long long tc_Kp = 0, tc_rows = 0;
     bool tc_ready = false;              // pattern matrix built for (tc_T, tc_fmt)
+    bool tc_finite = true;              // ... and every element of it finite
     std::vector<int> var_layer0;
     DBuf<unsigned char> d_tc_P;         // tc_rows x tc_Kp
     DBuf<float> d_tc_pscale;
@@ -984,7 +985,7 @@ struct qsk_sim {
     DBuf<unsigned long long> d_tc_key, d_tc_counts;
     DBuf<Slot> d_tc_slots;
     DBuf<Term> d_tc_terms;
-    DBuf<int> d_audit_nodes, d_exact_nodes, d_tc_order, d_tc_bins;
+    DBuf<int> d_audit_nodes, d_exact_nodes, d_tc_order, d_tc_bins, d_tc_flag;
     DBuf<float> d_audit_val;
     DBuf<unsigned> d_audit_pos, d_err_max;
     DBuf<double> d_err_sum;
@@ -1719,12 +1720,19 @@ int tc_configure(qsk_sim *s, int T_auto) {
     pa.fmt = fmt;
     pa.P = s->d_tc_P.p;
     pa.pos_scale = s->d_tc_pscale.p;
+    CK(s->d_tc_flag.ensure(1));
+    pa.nonfinite = s->d_tc_flag.p;
+    CK(cudaMemsetAsync(pa.nonfinite, 0, sizeof(int), s->st));
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     CK(cudaEventRecord(e0, s->st));
     CK(launch_tc_pattern(pa, rowmax.p, s->st));
     CK(cudaEventRecord(e1, s->st));
+    int nonfinite = 0;
+    CK(cudaMemcpyAsync(&nonfinite, pa.nonfinite, sizeof(int), cudaMemcpyDeviceToHost, s->st));
+    CK(cudaStreamSynchronize(s->st));
+    s->tc_finite = nonfinite == 0;
     CK(cudaEventSynchronize(e1));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
@@ -1834,8 +1842,8 @@ void tc_level_steps(qsk_sim *s, int level, const int *nodes, int at, const int *
     }
 }
 
-// Tensor steps of a run, planned on the device (the learned proposal's:
-// tc_plan): steps, K blocks per tile, and the audited nodes in d_audit_nodes
+// Tensor steps of a run, planned on the device (the learned proposal's, and
+// those over a pattern matrix with infinities: tc_plan): steps, K blocks per tile, and the audited nodes in d_audit_nodes
 // (their number in *n_audit).  Sorting the levels on the host instead: a
 // simulation of 250,000 nodes 84.1 ms (now 75.5), of 40,000 36.4 (now 35.0).
 int tc_plan_device(qsk_sim *s, const std::vector<int> &start, bool teacher, std::vector<Step> &steps, int *n_audit) {
@@ -1914,9 +1922,13 @@ int tc_plan_device(qsk_sim *s, const std::vector<int> &start, bool teacher, std:
     return QSK_OK;
 }
 
-// The learned proposal's steps: one stencil scale per step, the rest as above
-// but for the K blocks (one), planned on the host.  Rewrites the level node
-// list in that order.
+// The same planned on the host, for the learned proposal (one stencil scale per
+// step, one K block a tile) and for a pattern matrix that is not finite: there
+// a node's scores follow from the K blocks of its whole tile (a zero
+// coefficient times an infinity is NaN), and the device's order, free within a
+// bucket, would let its neighbours in the tile change from call to call.  Here
+// a level's nodes keep their order among equal template maxima.  Rewrites the
+// level node list in that order.
 int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &tmax, std::vector<Step> &steps,
             std::vector<int> &audit_nodes) {
     const long long nodes = s->nodes;
@@ -1927,6 +1939,7 @@ int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &t
     CK(cudaMemcpyAsync(order.data(), s->d_level_nodes.p, sizeof(int) * nodes, cudaMemcpyDeviceToHost, s->st));
     CK(cudaStreamSynchronize(s->st));
     const int kbe = s->tc_fmt == 0 ? 64 : 128;
+    const bool learned = s->topt.mode == 3;
     std::vector<int> kb;   // K blocks of every 128-node tile of every tensor step
     steps.clear();
     audit_nodes.clear();
@@ -1936,7 +1949,7 @@ int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &t
     const unsigned athr = s->topt.audit >= 1.f ? 0xFFFFFFFFu : unsigned(double(s->topt.audit) * 4294967296.0);
     // learned proposal: every node's stencil scale (per position of the level order)
     std::vector<int> lscale;
-    if (!start.empty() && start.back() > 0) {
+    if (learned && !start.empty() && start.back() > 0) {
         const long long tot = start.back();
         CK(s->d_lscale.ensure(size_t(tot)));
         int rc = node_scales(s, s->enc, s->d_level_nodes.p, tot, s->d_lscale.p);
@@ -1952,11 +1965,12 @@ int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &t
         esc.clear();
         for (int q = start[l]; q < start[l + 1]; ++q) {
             const int i = order[size_t(q)];
-            const bool tc = tmax[size_t(i)] >= 0;
+            const bool tc = tmax[size_t(i)] >= 0 && (learned || tmax[size_t(i)] < s->tc_T);
             (tc ? el : pl).push_back(i);
-            if (tc) esc.push_back(lscale[size_t(q)]);
+            if (tc) esc.push_back(learned ? lscale[size_t(q)] : tmax[size_t(i)]);
         }
-        // one stencil scale per step: the level's nodes grouped by scale
+        // one stencil scale per step: the level's nodes grouped by scale (else
+        // ordered by their template maximum)
         idx.resize(el.size());
         for (size_t j = 0; j < idx.size(); ++j) idx[j] = int(j);
         std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) { return esc[size_t(a)] < esc[size_t(b)]; });
@@ -1971,16 +1985,17 @@ int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &t
         for (int i : el) order[size_t(q++)] = i;
         for (int i : pl) order[size_t(q++)] = i;
         for (int g0 = 0; g0 < int(el.size());) {
-            int g1 = g0 + 1;
+            int g1 = learned ? g0 + 1 : int(el.size());
             while (g1 < int(el.size()) && esc[size_t(g1)] == esc[size_t(g0)]) ++g1;
             for (int off = g0; off < g1; off += s->max_tc_slots) {
                 const int B = std::min(s->max_tc_slots, g1 - off);
                 Step st{STEP_TENSOR, s->d_level_nodes.p, start[l] + off, B, int(kb.size())};
-                st.scale = esc[size_t(off)];
+                st.scale = learned ? esc[size_t(off)] : 1;
                 st.level = int(l);
                 for (int t0 = 0; t0 < B; t0 += 128) {
-                    kb.push_back(1);
-                    flops += 2.0 * 128 * 256 * double(ntiles_pos) * kbe;
+                    const long long last = esc[size_t(off + std::min(B, t0 + 128) - 1)];
+                    kb.push_back(learned ? 1 : int(((last + 1) * s->tc_L + kbe - 1) / kbe));
+                    flops += 2.0 * 128 * 256 * double(ntiles_pos) * double(kb.back()) * kbe;
                 }
                 steps.push_back(st);
             }
@@ -1991,7 +2006,7 @@ int tc_plan(qsk_sim *s, const std::vector<int> &start, const std::vector<int> &t
                     std::min(s->max_slots, int(pl.size()) - off), 0};
             // the learned proposal's fallback uses the exact map's buffers
             // inside its tensor steps: its levels stay on one stream
-            st.level = -1;
+            st.level = learned ? -1 : int(l);
             st.few = false;
             for (int q = off; q < off + st.B; ++q) st.few |= s->few[size_t(pl[size_t(q)])] != 0;
             steps.push_back(st);
@@ -2378,11 +2393,11 @@ int tc_run(qsk_sim *s, const std::vector<int> &start, bool teacher) {
     if (rc) return rc;
     if (s->tc_T_auto == 0 && (rc = tc_auto_prefix(s, &s->tc_T_auto)) != QSK_OK) return rc;
     if ((rc = tc_configure(s, s->tc_T_auto)) != QSK_OK) return rc;
-    const bool learned = s->topt.mode == 3;
+    const bool learned = s->topt.mode == 3, host_plan = learned || !s->tc_finite;
     std::vector<Step> steps;
-    std::vector<int> audit;   // the learned proposal's
+    std::vector<int> audit;   // the host plan's
     int n_audit = 0;
-    if (learned) {
+    if (host_plan) {
         if ((rc = tc_tmax(s)) != QSK_OK) return rc;
         if ((rc = tc_plan(s, start, s->tmax, steps, audit)) != QSK_OK) return rc;
         n_audit = int(audit.size());
@@ -2401,7 +2416,7 @@ int tc_run(qsk_sim *s, const std::vector<int> &start, bool teacher) {
     // audit: the plain path, teacher-forced on the final grid (every node's
     // neighbours hold the values they had at its turn), k best per node
     if (n_audit > 0) {
-        if (learned)
+        if (host_plan)
             CK(cudaMemcpyAsync(s->d_audit_nodes.p, audit.data(), sizeof(int) * audit.size(), cudaMemcpyHostToDevice,
                                s->st));
         std::vector<Step> as;

@@ -1081,6 +1081,9 @@ __global__ void k_tc_pattern(TcPatternArgs A, int pass, float *__restrict__ rowm
                 }
                 if (in) v = layer_value(A.ti, A.nvar, q, A.layer[l]) * inv;
             }
+            // (BF16 rounds to infinity from half a step above its largest value
+            // on; FP8 saturates, and keeps a NaN)
+            if (A.fmt == 0 ? !(fabsf(v) < 0x1.ffp127f) : isnan(v)) *A.nonfinite = 1;
             store_elem(A.P, p * A.Kp + k, v, A.fmt);
         }
     }

@@ -152,3 +152,27 @@ def test_nan_scores_are_no_candidates(g2s, gpu, fmt, share, W):
         pad = W - len(best)
         assert np.array_equal(keys[b, 0], np.concatenate([np.zeros(pad, np.uint64), full[best]])), b
         assert np.array_equal(pos[b, 0], np.concatenate([np.full(pad, 0xFFFFFFFF), at[best]]).astype(np.uint32)), b
+
+
+@pytest.mark.parametrize("mode", ["bf16", "fp8"])
+@pytest.mark.parametrize("edge,n", [(60, 20), (100, 40)])
+def test_infinite_layers_leave_the_draws_repeatable(g2s, gpu, edge, n, mode):
+    """Where the training image holds infinities, a node's scores follow from
+    the K blocks of its whole tile; the tiles of a level are the same in every
+    call, and so are the draws."""
+    rng = np.random.default_rng(edge)
+    ti = rng.standard_normal((edge, edge)).astype(np.float32)
+    ti[5, 7], ti[edge - 9, edge // 2] = np.inf, -np.inf
+    done = rng.standard_normal((40, 40)).astype(np.float32)
+    sim = g2s.Simulation(ti, np.full((40, 40), np.nan, np.float32), [0], n=n, k=2.5, seed=5)
+    sim.set_tensor(mode, audit=0.1)
+    nodes = np.arange(50, 1600, dtype=np.int32)
+    got = []
+    for _ in range(8):
+        sim.run_teacher_nodes(done, nodes)
+        info = sim.info()
+        got.append((sim.read()[2][nodes], [info[f] for f in ("tensor_nodes", "plain_nodes", "audited", "regret")]))
+    sim.close()
+    assert got[0][1][0] > 1000 and got[0][1][2] > 0
+    for cells, counts in got[1:]:
+        assert np.array_equal(cells, got[0][0]) and counts == got[0][1]
