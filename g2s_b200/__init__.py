@@ -203,13 +203,16 @@ _pack_term = struct.Struct("=iiiff").pack
 def _terms(terms):
     """QskTerm array of rows (neighbour, layer, op, a, b)."""
     n = len(terms)
-    try:
-        raw = b"".join(itertools.starmap(_pack_term, terms))
-    except (struct.error, TypeError, OverflowError):
-        # rows of other number types, or longer ones
-        return (QskTerm * max(n, 1))(*[QskTerm(int(t[0]), int(t[1]), int(t[2]), float(t[3]), float(t[4]))
-                                       for t in terms])
-    return (QskTerm * max(n, 1)).from_buffer_copy(raw or bytes(ctypes.sizeof(QskTerm)))
+    # tuples and lists are packed in one pass; any other row is asked for its
+    # fields one by one (iterating over it may give something else: a mapping
+    # its keys, a set its elements in some order)
+    if all(issubclass(t, (tuple, list)) for t in set(map(type, terms))):
+        try:
+            raw = b"".join(itertools.starmap(_pack_term, terms))
+            return (QskTerm * max(n, 1)).from_buffer_copy(raw or bytes(ctypes.sizeof(QskTerm)))
+        except (struct.error, TypeError, OverflowError):
+            pass   # fields of other number types, or longer rows
+    return (QskTerm * max(n, 1))(*[QskTerm(int(t[0]), int(t[1]), int(t[2]), float(t[3]), float(t[4])) for t in terms])
 
 
 def device_count() -> int:

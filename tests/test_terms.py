@@ -38,3 +38,23 @@ def test_rows_that_were_refused():
         with pytest.raises((TypeError, ValueError, IndexError)):
             g._terms(rows)
     assert ctypes.sizeof(g.QskTerm) == 20
+
+
+@pytest.mark.parametrize("row", [
+    {0: 3, 1: 1, 2: 2, 3: 0.5, 4: -0.25},                       # fields by key, not the keys
+    np.array([3, 1, 2, 4, 5]),
+    np.array([(3, 1, 2, 0.5, -0.25)], "i4,i4,i4,f4,f4")[0],
+], ids=["mapping", "integer array", "record"])
+def test_rows_by_index(row):
+    rows = [(0, 1, 2, -1.0, 0.25), row]
+    assert bytes(g._terms(rows)) == bytes(by_field(rows))
+    assert bytes(g._terms([row])) == bytes(by_field([row]))
+
+
+@pytest.mark.parametrize("make", [lambda: {3, 1, 2, 0, 4}, lambda: iter((0, 1, 2, 3, 4)),
+                                  lambda: (x for x in (0, 1, 2, 3, 4)), lambda: {0: 1, 1: 1, 2: 1, 3: 1, 5: 1}],
+                         ids=["set", "iterator", "generator", "mapping without a field"])
+def test_rows_without_an_index_are_refused(make):
+    for f in (by_field, g._terms):
+        with pytest.raises((TypeError, KeyError)):
+            f([make()])
