@@ -2718,13 +2718,11 @@ int qsk_sim_create(int device, const qsk_qs_params *p, const float *di_init, qsk
     }
     if (s->full && s->ti->missing)
         return bail(fail(QSK_ERR_UNSUPPORTED, "-fs with missing training-image values is not implemented"));
-    // the generator states come a group ahead: their blocks give way to the
-    // level chain's, which wait for an SM the least
-    int prio_low = 0, prio_high = 0;
-    cudaError_t e = cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
-    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->st, cudaStreamNonBlocking, prio_high);
-    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->st_rng, cudaStreamNonBlocking, prio_low);
-    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->st2, cudaStreamNonBlocking, prio_high);
+    // normal priority for all three: a higher one for the level chain would set
+    // a simulation before the calling program's own streams on this GPU
+    cudaError_t e = cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->st_rng, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->st2, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_level, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->ev_side, cudaEventDisableTiming);
     for (int p = 0; p < 2 && e == cudaSuccess; ++p) {

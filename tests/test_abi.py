@@ -29,6 +29,14 @@ def test_library_exports_every_declared_symbol(g2s):
     assert set(names) <= exported
 
 
+def test_library_asks_for_no_stream_priority(g2s):
+    """A simulation's streams run at the normal priority: a calling program's
+    own streams on the same GPU are not set behind them."""
+    out = subprocess.run(["nm", "-D", "--undefined-only", g2s.LIB_PATH], capture_output=True, text=True).stdout
+    used = set(re.findall(r"\b(cudaStreamCreate\w*|cudaLaunchKernel\w*)", out))
+    assert "cudaStreamCreateWithFlags" in used and "cudaStreamCreateWithPriority" not in used
+
+
 def test_library_is_sm100a():
     out = subprocess.run(["/usr/local/cuda/bin/cuobjdump", "--list-elf", os.path.join(ROOT, "g2s_b200", "libg2s_b200.so")],
                          capture_output=True, text=True).stdout
