@@ -2860,9 +2860,14 @@ int qsk_sim_create(int device, const qsk_qs_params *p, const float *di_init, qsk
     ms = std::max<long long>(1, std::min<long long>(ms, std::max<long long>(s->nodes, 1)));
     ms = std::min<long long>(ms, 65535);
     s->max_slots = int(ms);
-    // a group of batches prepares up to 4,096 nodes' generator states (2.5 KB
-    // each) in one launch, or one batch where that is more
-    s->rng_slots = int(std::max<long long>(ms, std::min<long long>(4096, std::max<long long>(s->nodes, 1))));
+    // a group of batches prepares its nodes' generator states (2.5 KB each, and
+    // the slots and static terms of the bit-sliced map) in one launch: as many
+    // as 4 MiB hold, so that the two buffers are small beside the records (a
+    // group of 256 or of 4,096 nodes makes no difference that can be measured),
+    // or one batch where that is more
+    const size_t rng_slot = 625 * sizeof(unsigned) + (s->use_bits ? sizeof(StaticTerm) * s->maxterms + sizeof(Slot) : 0);
+    s->rng_slots = int(std::max<long long>(
+        ms, std::min<long long>((long long)((size_t(4) << 20) / rng_slot), std::max<long long>(s->nodes, 1))));
     if ((e = s->d_slots.alloc(size_t(s->max_slots))) != cudaSuccess ||
         (e = s->d_mt_state.alloc(size_t(2) * s->rng_slots * 624)) != cudaSuccess ||
         (e = s->d_mt_pre.alloc(size_t(2) * s->rng_slots)) != cudaSuccess ||

@@ -60,3 +60,24 @@ def test_limit_zero_keeps_nothing(g2s, gpu):
     assert g2s.blocks_info(0)["bytes"] > 0
     g2s.blocks_release()
     assert g2s.blocks_info(0)["bytes"] == 0
+
+
+@pytest.mark.parametrize("categorical", [False, True])
+def test_prepared_nodes_take_little_beside_the_records(g2s, gpu, categorical):
+    """On a large image a batch is a few dozen nodes; the generator states
+    prepared ahead of the batches are bounded by their bytes, not by the nodes
+    of the grid: from a grid of 216 nodes to one of 8,000 a simulation that
+    has not run grows by its per-node lists (under 2 MB) and at most two
+    buffers of 4 MiB."""
+    rng = np.random.default_rng(1)
+    ti = rng.standard_normal((100, 128, 128)).astype(np.float32)
+    if categorical:
+        ti = (ti > 0).astype(np.float32)
+    kept = []
+    for edge in (6, 20):
+        g2s.blocks_release()
+        sim = g2s.Simulation(ti, np.full((edge,) * 3, np.nan, np.float32), [int(categorical)], n=10, k=1.2, seed=1)
+        sim.close()
+        kept.append(g2s.blocks_info(0)["bytes"])
+    g2s.blocks_release()
+    assert kept[1] - kept[0] <= (8 << 20) + 2_000_000
