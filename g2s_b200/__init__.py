@@ -689,12 +689,14 @@ def blocks_info(device: int = 0) -> dict:
 
 
 def blocks_release() -> None:
-    """Free every kept device block (qsk_blocks_release)."""
+    """Free every kept device block, and the page-locked host memory that no
+    worker holds (qsk_blocks_release)."""
     _check(lib().qsk_blocks_release(), "qsk_blocks_release")
 
 
 def blocks_set_limit(nbytes: int) -> None:
-    """Bytes kept per device from ended simulations (0: keep none)."""
+    """Bytes kept per device from ended simulations (0: keep none; no
+    page-locked host memory of destroyed workers then either)."""
     _check(lib().qsk_blocks_set_limit(int(nbytes)), "qsk_blocks_set_limit")
 
 

@@ -96,6 +96,12 @@ void *block_take(size_t bytes, size_t *cap) {
     return p;
 }
 
+unsigned long long kept_limit() {
+    KeptBlocks &k = kept();
+    std::lock_guard<std::mutex> lock(k.mu);
+    return k.limit;
+}
+
 bool block_keep(void *p, size_t cap) {
     int dev = -1;
     if (!p || cap == 0 || cudaGetDevice(&dev) != cudaSuccess) return false;
@@ -111,7 +117,9 @@ bool block_keep(void *p, size_t cap) {
 // Pinned host blocks of the workers' staging.  Page-locking memory takes 0.5
 // to 1.5 ms whatever its size, 20 times a small query, so blocks are lent out
 // and come back: pieces of one allocation up to PINNED_PIECE bytes, larger
-// ones by themselves (at most PINNED_LARGE bytes of them kept).  Freed by
+// ones by themselves.  Without a worker at most one allocation of pieces and
+// PINNED_LARGE bytes of larger blocks stay, and no more than the limit of the
+// kept device blocks of either (qsk_blocks_set_limit).  Freed by
 // qsk_blocks_release, but for allocations with a piece still lent.
 namespace {
 constexpr size_t PINNED_PIECE = 65536, PINNED_LARGE = 64u << 20;
@@ -178,10 +186,11 @@ int pinned_take(size_t bytes, unsigned char **out, size_t *cap) {
 // back from its worker, whose stream has ended all work on it
 void pinned_give(unsigned char *p, size_t cap) {
     if (!p) return;
+    const unsigned long long limit = kept_limit();
     PinnedBlocks &b = pinned();
     std::lock_guard<std::mutex> lock(b.mu);
     if (cap != PINNED_PIECE) {
-        if (b.large_bytes + cap > PINNED_LARGE) {
+        if (b.large_bytes + cap > std::min<unsigned long long>(PINNED_LARGE, limit)) {
             cudaFreeHost(p);
             return;
         }
@@ -189,7 +198,7 @@ void pinned_give(unsigned char *p, size_t cap) {
         b.large_bytes += cap;
         return;
     }
-    bool idle = false;   // another allocation with every piece at home
+    bool idle = PINNED_PIECE * PINNED_PIECES > limit;   // not to be kept, or another with every piece at home
     for (auto &x : b.slabs) idle |= x.home == PINNED_ALL;
     for (size_t i = 0; i < b.slabs.size(); ++i) {
         auto &x = b.slabs[i];

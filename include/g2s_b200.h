@@ -73,6 +73,11 @@ int qsk_ti_destroy(qsk_ti *ti);
 /* ------------------------------------------------------------------------
  * Per-thread worker: stream + scratch for pattern queries (one per G2S path
  * thread, like one NvidiaGPUAcceleratorDevice per thread, src/qs.cpp:1577-1588).
+ * A worker's calls go through page-locked host memory, lent to it from blocks
+ * shared by all workers of the process: 64 KB from its creation on (eight
+ * workers share one allocation; QSK_ERR_NOMEM if none can be had), a block of
+ * the call's size once a call needs more.  See qsk_blocks_set_limit for what
+ * stays after the workers have gone.
  * ---------------------------------------------------------------------- */
 typedef struct qsk_worker qsk_worker;
 int qsk_worker_create(qsk_ti *ti, qsk_worker **out);
@@ -423,9 +428,15 @@ int qsk_sim_destroy(qsk_sim *s);
 /* Kept blocks: the limit per device (0: keep none), freeing every kept block
  * of every device (nothing reads them), and the kept bytes and blocks of one
  * device with the process-wide count of allocations served from them (hits)
- * or not (misses).  Kept blocks belong to the device's primary context: call
+ * or not (misses).  qsk_jobs_run leaves its threads' batch scratch there too,
+ * if their jobs all ended well.  Page-locked host memory of destroyed workers
+ * is kept beside them for the next ones: at most 512 KB of small pieces and
+ * 64 MB of larger blocks, and neither beyond the limit (0: none stays);
+ * qsk_blocks_release frees what no worker holds, qsk_blocks_info does not
+ * count it.  Kept blocks belong to the device's primary context (the host
+ * memory to that of the device whose worker needed it first): call
  * qsk_blocks_release before a cudaDeviceReset (or any reset of that context),
- * after which they would no longer be valid device memory. */
+ * after which they would no longer be valid memory. */
 int qsk_blocks_set_limit(unsigned long long bytes);
 int qsk_blocks_release(void);
 int qsk_blocks_info(int device, unsigned long long *bytes, long long *blocks, long long *hits, long long *misses);
