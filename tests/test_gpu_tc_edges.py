@@ -176,3 +176,35 @@ def test_infinite_layers_leave_the_draws_repeatable(g2s, gpu, edge, n, mode):
     assert got[0][1][0] > 1000 and got[0][1][2] > 0
     for cells, counts in got[1:]:
         assert np.array_equal(cells, got[0][0]) and counts == got[0][1]
+
+
+@pytest.mark.parametrize("k", [1.0, 2.5])
+def test_compact_list_beyond_the_staged_keys(g2s, gpu, k):
+    """A bounded shortlist's list may hold more keys than the select stages
+    (768): patterns 195 columns wide on a 200-column image leave five valid
+    columns, too few in any position range for a bound, so nearly all of their
+    900 positions reach the list.  The draws are those of the longer shortlist,
+    whose lists are not bounded."""
+    X, Y, W = 200, 180, 8
+    rng = np.random.default_rng(int(2 * k))
+    ti = rng.integers(0, 3, (Y, X)).astype(np.float32)
+    p = np.arange(X * Y)
+    valid = np.bincount(p[(p % X >= 100) & (p % X < 105)] // 256, minlength=(X * Y + 255) // 256)
+    assert len(valid) <= 148 and np.minimum(valid, W).sum() > 768   # one tile a range
+    di = np.full((30, X), np.nan, np.float32)
+    di[:, 2], di[:, 197] = rng.integers(0, 3, (2, 30))
+    done = rng.integers(0, 3, di.shape).astype(np.float32)
+    done[:, [2, 197]] = di[:, [2, 197]]
+    got = []
+    for shortlist in (W, 32):
+        sim = g2s.Simulation(ti, di, [1], n=50, k=k, seed=3, kernel=np.ones((1, 399), np.float32))
+        sim.set_tensor("bf16", prefix=512, width=W, shortlist=shortlist, audit=1.0)
+        order, _, begin = sim.path()
+        at = np.array([i for i in range(400) if 2 < order[begin + i] % X < 197][:100], np.int32)
+        sim.run_teacher_nodes(done, at)
+        info = sim.info()
+        assert info["tensor_nodes"] == 100 and info["tensor_shortlist"] == shortlist and info["tensor_width"] == W
+        assert info["audited"] == 100 and info["regret"] == 0 and info["regret_near"] == 0
+        got.append(sim.read()[2][at])
+        sim.close()
+    assert np.array_equal(got[0], got[1])
