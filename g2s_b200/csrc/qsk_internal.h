@@ -459,7 +459,7 @@ struct TcPatternArgs {
     int fmt;                   // 0 BF16, 1 FP8 E4M3
     void *P;
     float *pos_scale;          // FP8: per tile of 256 rows
-    int *nonfinite;            // set where an element of P is infinite or NaN (zeroed before the launch)
+    int *nonfinite;            // set where a layer value is beyond BF16 (zeroed before the launch)
 };
 struct TcNodeArgs {
     int nd, nvar;

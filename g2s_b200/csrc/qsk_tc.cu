@@ -1065,6 +1065,11 @@ __global__ void k_tc_pattern(TcPatternArgs A, int pass, float *__restrict__ rowm
             if (lane == 0) rowmax[p] = mx;
             continue;
         }
+        // the row's own cell stands for all its copies (BF16 rounds to infinity
+        // from half a step above its largest value on)
+        if (live)
+            for (int l = lane; l < A.L; l += 32)
+                if (!(fabsf(layer_value(A.ti, A.nvar, p, A.layer[l])) < 0x1.ffp127f)) *A.nonfinite = 1;
         if (A.fmt == 1) scale = A.pos_scale[p >> 8];
         const float inv = 1.f / scale;
         for (long long k = lane; k < A.Kp; k += 32) {
@@ -1081,9 +1086,6 @@ __global__ void k_tc_pattern(TcPatternArgs A, int pass, float *__restrict__ rowm
                 }
                 if (in) v = layer_value(A.ti, A.nvar, q, A.layer[l]) * inv;
             }
-            // (BF16 rounds to infinity from half a step above its largest value
-            // on; FP8 saturates, and keeps a NaN)
-            if (A.fmt == 0 ? !(fabsf(v) < 0x1.ffp127f) : isnan(v)) *A.nonfinite = 1;
             store_elem(A.P, p * A.Kp + k, v, A.fmt);
         }
     }
