@@ -47,6 +47,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 
 #include "qsk_internal.h"
 #include "qsk_pdl.cuh"
@@ -417,6 +418,7 @@ __global__ void __launch_bounds__(threads_for(W), 1)
             for (int l = 0; l < 32; ++l) lists[l * LIST_STRIDE + lane] = 0ull;
             __syncwarp();
         }
+        int fill = 0;   // LISTS: keys in this lane's list
         float *scratch = reinterpret_cast<float *>(epi) + e * 32 + lane;   // !LISTS: score j at [j * 32 * EPI_WARPS]
         u64 root = 0ull;    // this group's W-th best key
         u64 kb = 0ull;      // the bound to pass: root, or the best W-th of any range seen
@@ -590,9 +592,17 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                         thr = kb ? unordered((unsigned)(kb >> 32)) : thr;
                     }
                 } else {
-                    // the lanes' next candidates, one list after the other: the key
-                    // takes the place of the list's smallest, whose successor two
-                    // warp-wide minima find
+                    // the lanes' next candidates.  A list that is not full takes its
+                    // own lane's key behind its last, all lanes at once; in a full
+                    // one the key takes the place of the smallest, whose successor
+                    // two warp-wide minima find, list after list.  That chain of
+                    // shared-memory reads and reductions is long where every lane
+                    // has candidates, so four lists go through it together.  One
+                    // list at a time, empty ones too, was slower than keys in
+                    // registers wherever lists are filled again and again: levels
+                    // of a 100x100 GRF (207, FP8) 60 -> 70 ms, now 44; of a
+                    // 200x200 one 209 -> 201, now 141; 100 nodes against 2,400
+                    // positions in one range 1.23 -> 1.68 ms a call, now 1.23.
                     while (__any_sync(0xffffffffu, cand != 0u)) {
                         u64 key = 0ull;
                         if (cand) {
@@ -610,25 +620,59 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                             for (int u = 0; u < 2; ++u) t2[u] = (j & 8) ? t4[2 * u + 1] : t4[2 * u];
                             key = (u64)ordered((j & 16) ? t2[1] : t2[0]) << 32 | tie_hash(nseed, (unsigned)(pc + j));
                             if (key <= kb) key = 0ull;
+                            if (key && fill < 32) {
+                                u64 *mine = lists + lane * LIST_STRIDE;
+                                mine[fill++] = key;
+                                key = 0ull;
+                                if (fill == 32) {
+                                    root = mine[0];
+                                    for (int l = 1; l < 32; ++l) root = min(root, mine[l]);
+                                    kb = max(kb, root);
+                                    thr = unordered((unsigned)(kb >> 32));
+                                }
+                            }
                         }
+                        __syncwarp();
                         unsigned act = __ballot_sync(0xffffffffu, key != 0ull);
-                        while (act) {
-                            const int l = __ffs(act) - 1;
-                            act &= act - 1u;
-                            const u64 kl = shfl_u64(key, l), rl = shfl_u64(root, l);
-                            u64 k = lists[l * LIST_STRIDE + lane];
-                            const int slot = __ffs(__ballot_sync(0xffffffffu, k == rl)) - 1;
-                            if (lane == slot) {
-                                k = kl;
-                                lists[l * LIST_STRIDE + lane] = kl;
+                        const auto insert = [&](auto lists_at_once) {
+                            constexpr int U = decltype(lists_at_once)::value;
+                            int l[U], slot[U];
+                            u64 kl[U], rl[U], k[U];
+                            unsigned hi[U], lo[U];
+#pragma unroll
+                            for (int u = 0; u < U; ++u) {
+                                l[u] = __ffs(act) - 1;
+                                act &= act - 1u;
                             }
-                            const unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32));
-                            const unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : ~0u);
-                            if (lane == l) {
-                                root = (u64)hi << 32 | lo;
-                                kb = max(kb, root);
-                                thr = kb ? unordered((unsigned)(kb >> 32)) : thr;
+#pragma unroll
+                            for (int u = 0; u < U; ++u) {
+                                kl[u] = shfl_u64(key, l[u]);
+                                rl[u] = shfl_u64(root, l[u]);
+                                k[u] = lists[l[u] * LIST_STRIDE + lane];
                             }
+#pragma unroll
+                            for (int u = 0; u < U; ++u) {
+                                slot[u] = __ffs(__ballot_sync(0xffffffffu, k[u] == rl[u])) - 1;
+                                if (lane == slot[u]) {
+                                    k[u] = kl[u];
+                                    lists[l[u] * LIST_STRIDE + lane] = kl[u];
+                                }
+                            }
+#pragma unroll
+                            for (int u = 0; u < U; ++u) hi[u] = __reduce_min_sync(0xffffffffu, (unsigned)(k[u] >> 32));
+#pragma unroll
+                            for (int u = 0; u < U; ++u)
+                                lo[u] = __reduce_min_sync(0xffffffffu, (unsigned)(k[u] >> 32) == hi[u] ? (unsigned)k[u] : ~0u);
+#pragma unroll
+                            for (int u = 0; u < U; ++u)
+                                if (lane == l[u]) root = (u64)hi[u] << 32 | lo[u];
+                        };
+                        const bool changed = key != 0ull;
+                        while (__popc(act) >= 4) insert(std::integral_constant<int, 4>{});
+                        while (act) insert(std::integral_constant<int, 1>{});
+                        if (changed) {
+                            kb = max(kb, root);
+                            thr = kb ? unordered((unsigned)(kb >> 32)) : thr;
                         }
                     }
                 }
