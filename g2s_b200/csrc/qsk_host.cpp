@@ -806,7 +806,7 @@ static int pattern_batch_impl(qsk_worker *w, int B, const int *nb_ptr, const int
         ma.terms = d_terms;
         ma.gen = gen;
         ma.maxterms = maxterms;
-        ma.segs_per_cta = map_segs_per_cta(g, B);
+        ma.segs_per_cta = map_segs_per_cta(g, B, int(k));
         ma.rec_val = w->rec_val.p;
         ma.rec_idx = w->rec_idx.p;
         ma.rec_cnt = w->rec_cnt.p;
@@ -1451,7 +1451,7 @@ int sim_batches(qsk_sim *s, const std::vector<Step> &steps, bool teacher) {
                 ma.slots = s->d_slots.p;
                 ma.terms = s->d_terms.p;
                 ma.maxterms = s->maxterms;
-                ma.segs_per_cta = map_segs_per_cta(g, B);
+                ma.segs_per_cta = map_segs_per_cta(g, B, s->K);
                 ma.rec_val = s->d_rec_val.p;
                 ma.rec_idx = s->d_rec_idx.p;
                 ma.rec_cnt = s->d_rec_cnt.p;
@@ -2094,7 +2094,7 @@ int exact_nodes(qsk_sim *s, const int *nodes, int count, bool teacher) {
         ma.slots = s->d_slots.p;
         ma.terms = s->d_terms.p;
         ma.maxterms = s->maxterms;
-        ma.segs_per_cta = map_segs_per_cta(g, B);
+        ma.segs_per_cta = map_segs_per_cta(g, B, s->K);
         ma.rec_val = s->d_rec_val.p;
         ma.rec_idx = s->d_rec_idx.p;
         ma.rec_cnt = s->d_rec_cnt.p;
@@ -2516,7 +2516,7 @@ int sim_batches_multi(qsk_sim *s, const std::vector<Step> &steps) {
             ma.slots = s->d_slots.p;
             ma.terms = s->d_terms.p;
             ma.maxterms = s->maxterms;
-            ma.segs_per_cta = map_segs_per_cta(T->g, B);
+            ma.segs_per_cta = map_segs_per_cta(T->g, B, s->K);
             ma.rec_val = s->d_rec_val.p;
             ma.rec_idx = s->d_rec_idx.p;
             ma.rec_cnt = s->d_rec_cnt.p;
@@ -3601,7 +3601,7 @@ int qsk_pattern_kbest_noalloc(const qsk_ti *ti, void *stream, int n_neighbours, 
         ma.slots = d_slot;
         ma.terms = d_terms;
         ma.maxterms = maxterms;
-        ma.segs_per_cta = map_segs_per_cta(g, 1);
+        ma.segs_per_cta = map_segs_per_cta(g, 1, int(k));
         ma.rec_val = rec_val;
         ma.rec_idx = rec_idx;
         ma.rec_cnt = rec_cnt;

@@ -356,7 +356,7 @@ cudaError_t launch_levels(const LevelArgs &a, cudaStream_t st);
 // this one in its level's chain (replay or select -> preparation -> map ->
 // replay or hash select), behind which it may begin launching
 cudaError_t launch_prep_sim(const SimPrepArgs &a, bool chained, cudaStream_t st);
-int map_segs_per_cta(const Geom &g, int nslots);
+int map_segs_per_cta(const Geom &g, int nslots, int K);
 cudaError_t launch_map_records(const MapArgs &a, int nslots, int K, int maxterms_in_batch, bool chained,
                                cudaStream_t st);
 cudaError_t set_map_smem_limit(int bytes);

@@ -2822,13 +2822,18 @@ cudaError_t launch_prep_sim(const SimPrepArgs &a, bool chained, cudaStream_t st)
     return launch_chain(chained, k_prep_sim, dim3((unsigned)blocks), dim3(threads), 0, st, a);
 }
 
-int map_segs_per_cta(const Geom &g, int nslots) {
+int map_segs_per_cta(const Geom &g, int nslots, int K) {
     // a CTA takes 8 warps x MR_SEGS segments a turn; more turns (up to 8)
     // tighten the filter and share the set-up while the grid still fills the
-    // GPU's 4 resident CTAs per SM three times
+    // GPU's 4 resident CTAs per SM three times.  Beyond K = 4 (2 resident
+    // CTAs) a warp's first turns, which hold no bound yet, cost the most, and
+    // one wave of CTAs is best: 80x70x60 continuous (n = 25), K = 15, map and
+    // replay of all levels 205 ms by the rule for K <= 4 (196 with a prefix per
+    // segment), 183 with three waves of two CTAs, 178 with two, 175 with one;
+    // K = 8 51, 51, 50, 51
     const long long turn = 8 * MR_SEGS;
     const long long turns = (g.nseg + turn - 1) / turn * nslots;
-    long long per = turns / (148LL * 4 * 3);
+    long long per = turns / (K <= 4 ? 148LL * 4 * 3 : 148LL * 2);
     per = per < 1 ? 1 : (per > 8 ? 8 : per);
     return (int)(per * turn);
 }
