@@ -10,13 +10,14 @@ namespace qsk {
 
 // Device blocks kept across simulations, per device (qsk_host.cpp).  A
 // simulation's buffers are handed here by qsk_sim_destroy after a device
-// synchronisation, so no work in flight reads them; DBuf::alloc takes the
+// synchronisation, and a job thread's scratch by qsk_jobs_run once its runs
+// have ended, so no work in flight reads them; DBuf::alloc takes the
 // smallest kept block of the current device that holds the request (and at
 // most twice it, plus 2 MiB) before it calls cudaMalloc.  Blocks are not
 // cleared: every buffer is written before it is read, as with cudaMalloc.
 void *block_take(size_t bytes, size_t *cap);
 bool block_keep(void *p, size_t cap);   // false: over the limit, the caller frees
-extern thread_local bool g_keep_blocks; // set while qsk_sim_destroy releases
+extern thread_local bool g_keep_blocks; // set while qsk_sim_destroy or qsk_jobs_run releases
 
 // device buffer owned by the host object that holds it
 template <typename T>

@@ -667,9 +667,10 @@ __device__ __forceinline__ void mt_seed(unsigned *mt, float sd) {
 // The blocks roll through registers: a step makes the next 224 words, seven
 // consecutive ones per lane (the recurrence reaches back 227 words at the
 // least, so a step depends on earlier steps only), from the three steps
-// before it: eleven shuffles, no shared memory and no barrier.  In shared
-// memory, three phases a block, the 600 blocks of a 128^3 image's first
-// masked plane took 265 us for 102 slots, now 391 us for one of 396.
+// before it: eleven shuffles, no shared memory and no barrier.  512 slots of a
+// 128^3 image (up to 600 blocks each): in shared memory, three phases a block,
+// five launches of 126 slots or fewer took 107 to 634 us, 1.30 ms in all; now
+// two, of 126 and 386 slots, take 405 and 367.
 __device__ __forceinline__ void mt_step(unsigned (&n)[7], const unsigned (&a)[7], const unsigned (&b)[7],
                                         const unsigned (&c)[7], int lane) {
     // word t = 7 lane + i of the step needs words t - 3 of the last step (a),
@@ -1602,8 +1603,9 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // 47 -> 14 us, categorical 101x90 (n = 20) 40 -> 25 us, 250x250 -> 500x500
 // (n = 80) 65 -> 54 us; then with 16-byte staging copies, tie runs of their own
 // (team_ties) and three CTAs of 80 registers per SM the slots of the last two
-// took 54 k -> 35 k and 83 k -> 50 k cycles; one slot of 26,000 segments 559 -> 230 us, of which
-// the generator blocks of its first masked stretch are 210.
+// took 54 k -> 35 k and 83 k -> 50 k cycles.  One slot of 26,000 segments takes
+// 64 us; 559 in the old form, most of them the generator blocks of its first
+// masked stretch, which now run beside the map (GenArgs).
 template <int KM>
 __global__ void __launch_bounds__(RP_THREADS, KM <= 4 ? 3 : 1) k_replay(ReplayArgs A) {
     __shared__ ReplayShared w;
@@ -2592,7 +2594,8 @@ __global__ void __launch_bounds__(256, KF <= 4 ? 4 : 1) k_map_bits(BitArgs A) {
 
 // The slot of path node i and its terms without their values (bit-sliced
 // simulations: unit weights, categorical variables, complete TI): everything
-// k_prep_sim derives from the neighbour lists, computed one batch ahead.
+// k_prep_sim derives from the neighbour lists, computed a group of batches
+// ahead.
 // The map reads the values (and derives the -nV exclusion) when it runs.
 __device__ void write_static_slot(const SimPrepArgs &A, int b, int i, unsigned pv, unsigned cell, const NodeGeom &ng,
                                   int lane) {
@@ -2673,8 +2676,8 @@ __device__ void write_static_slot(const SimPrepArgs &A, int b, int i, unsigned p
 }
 
 // MT19937 state of each slot ahead of its replay (one warp per slot; the
-// host runs it for the next batch while the current one is simulated, as it
-// reads the neighbour lists only): the seeding and, with masked positions
+// host runs it for the next group of batches while the current one is
+// simulated, as it reads the neighbour lists only): the seeding and, with masked positions
 // not emitted as records, the state-only blocks of the replay's first
 // skip.  That skip covers the c
 // masked positions before the first record (two draws each); c is at least
@@ -2822,6 +2825,7 @@ cudaError_t launch_prep_sim(const SimPrepArgs &a, bool chained, cudaStream_t st)
     return launch_chain(chained, k_prep_sim, dim3((unsigned)blocks), dim3(threads), 0, st, a);
 }
 
+// (148: the SMs of a B200, here and below)
 int map_segs_per_cta(const Geom &g, int nslots, int K) {
     // a CTA takes 8 warps x MR_SEGS segments a turn; more turns (up to 8)
     // tighten the filter and share the set-up while the grid still fills the

@@ -459,7 +459,7 @@ cudaError_t launch_sgemm(int M, int N, int K, const float *A, int lda, int ta, c
                          int ldc, float alpha, float beta, const float *bias, cudaStream_t st) {
     if (M <= 0 || N <= 0) return cudaSuccess;
     auto tiles = [&](int tm, int tn) { return dim3((unsigned)((N + tn - 1) / tn), (unsigned)((M + tm - 1) / tm)); };
-    const dim3 big = tiles(64, 64);
+    const dim3 big = tiles(64, 64);   // (148: the SMs of a B200)
     if ((long long)big.x * big.y >= 148)
         k_sgemm<64, 64, 16, 4, 4><<<big, 256, 0, st>>>(M, N, K, A, lda, ta, B, ldb, tb, C, ldc, alpha, beta, bias);
     else

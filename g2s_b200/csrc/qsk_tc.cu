@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(threads_for(W), 1)
         // scanned grow by an eighth: the bound falls behind by no more.
         // 8,000 draws of the 180x150x120 GRF, 4,096-node launches: the one of
         // shorter patterns 14 -> 10 ms (6 without any insertion), the one of
-        // longer ones 30 -> 29 (27, the pattern matrix's reads); 59.0 -> 55.4 in all.
+        // longer ones 30 -> 29 (27; its widest tile's time); 59.0 -> 55.4 in all.
         int exchange = 0;
         const auto publish = [&]() {
             const int node0 = tile_m * BM + q * 32;
@@ -540,7 +540,8 @@ __global__ void __launch_bounds__(threads_for(W), 1)
                 if constexpr (W == 8) {
                     // fewer than eight keys so far: no more than the chunk's own
                     // eight best can enter (their ties too), which a sorting
-                    // network finds without one insertion.  A NaN score (an
+                    // network finds without one insertion (W = 16 inserts; a
+                    // network for its sixteen best was not tried).  A NaN score (an
                     // infinite layer value times a zero) is no candidate and
                     // stands as -inf: an exchange of it by fmaxf / fminf would
                     // leave its partner twice
@@ -1029,7 +1030,7 @@ cudaError_t launch_gemm_bn(const CUtensorMap &ma, const CUtensorMap &mb, const T
 // product of few tiles is bound by the latency of its chain of K blocks, and
 // a narrow tile's are shorter: the 14 products of a 1,024-pair gradient took
 // 368 us in tiles of 256, 171 in tiles of 64).  The products of an element run
-// in the same order in every tile.
+// in the same order in every tile.  148: the SMs of a B200.
 int tc_gemm_bn(int M, int N) {
     const long long tm = (M + tc::BM - 1) / tc::BM;
     if (N > 128 && tm * ((N + 255) / 256) >= 148) return 256;
