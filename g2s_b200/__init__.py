@@ -198,6 +198,7 @@ def _p(a, t):
 
 
 _pack_term = struct.Struct("=iiiff").pack
+_ROW_TYPES = {tuple, list}
 
 
 def _terms(terms):
@@ -206,7 +207,8 @@ def _terms(terms):
     # tuples and lists are packed in one pass; any other row is asked for its
     # fields one by one (iterating over it may give something else: a mapping
     # its keys, a set its elements in some order)
-    if all(issubclass(t, (tuple, list)) for t in set(map(type, terms))):
+    kinds = set(map(type, terms))
+    if kinds <= _ROW_TYPES or all(issubclass(t, (tuple, list)) for t in kinds):
         try:
             raw = b"".join(itertools.starmap(_pack_term, terms))
             return (QskTerm * max(n, 1)).from_buffer_copy(raw or bytes(ctypes.sizeof(QskTerm)))
